@@ -25,7 +25,7 @@ struct KernelConfig {
     uint64_t allbits = 0;      // enumeration bit j quantifier is All
     bool data = false;         // items from a buffer (reduction tests)
     // TABLE
-    uint32_t fmt = 0;          // 0 u32, 1 u64, 2 u64 + distance
+    uint32_t fmt = 0;          // 0 u32, 1 u64
     uint32_t nout = 1;
 
     uint32_t threads() const { return 32u << wb; }

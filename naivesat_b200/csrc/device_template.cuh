@@ -384,22 +384,17 @@ nsat_table(u64 nwords, u64 w0, void* __restrict__ table, LaunchOut* __restrict__
         transpose32(o);
         if (NSAT_NOUT > 32) transpose32(o + 32);
         u64* t64 = reinterpret_cast<u64*>(table) + (w << 5);
-#if NSAT_FMT == 2
-        const u64 hi_or = 1ull << 32;   // distance 1 per entry
-#else
-        const u64 hi_or = 0ull;
-#endif
         if (lanes == 32) {
             ulonglong2* dst = reinterpret_cast<ulonglong2*>(t64);
 #pragma unroll
             for (int q = 0; q < 16; q++) {
                 ulonglong2 v;
-                v.x = (u64)o[2 * q] | ((u64)o[32 + 2 * q] << 32) | hi_or;
-                v.y = (u64)o[2 * q + 1] | ((u64)o[32 + 2 * q + 1] << 32) | hi_or;
+                v.x = (u64)o[2 * q] | ((u64)o[32 + 2 * q] << 32);
+                v.y = (u64)o[2 * q + 1] | ((u64)o[32 + 2 * q + 1] << 32);
                 __stcs(dst + q, v);
             }
         } else {
-            for (int l = 0; l < lanes; l++) t64[l] = (u64)o[l] | ((u64)o[32 + l] << 32) | hi_or;
+            for (int l = 0; l < lanes; l++) t64[l] = (u64)o[l] | ((u64)o[32 + l] << 32);
         }
 #endif
     }

@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include "circuit.h"
+#include "stop_kernels.h"
 
 namespace nsat {
 
@@ -31,6 +32,9 @@ int ctx_fail(nsat_ctx* ctx, int code, const std::string& msg);
 // allocation.
 cudaError_t ctx_alloc(nsat_ctx* ctx, void** p, size_t bytes);
 void ctx_free(nsat_ctx* ctx, void* p);
+// The context's device state of a SATOSTOP solve and its pinned host copy.
+void ctx_stop_state(nsat_ctx* ctx, NsatStopState** dev, NsatStopState** host);
+cudaEvent_t ctx_stop_event(nsat_ctx* ctx);
 // Returns the pool's unused memory to the device (after the context's
 // stream finishes), for a caller about to size a buffer by free memory.
 void ctx_trim(nsat_ctx* ctx);

@@ -26,6 +26,7 @@
 #include "qreducer.h"
 #include "internal.h"
 #include "static_kernels.h"
+#include "stop_join.h"
 
 using namespace nsat;
 typedef unsigned __int128 u128;
@@ -67,6 +68,8 @@ struct nsat_ctx {
     size_t data_bytes = 0;
     NsatJoinState* d_join = nullptr;
     NsatJoinState* h_join = nullptr;
+    NsatStopState* d_stop = nullptr;
+    NsatStopState* h_stop = nullptr;
     // loaded kernels by everything their generated source depends on (the
     // kernel configuration, the entry point and the LUT net, compared
     // whole): a fresh circuit handle whose cover and launch configuration
@@ -107,9 +110,12 @@ struct nsat_circuit {
 
 struct nsat_table {
     nsat_ctx* ctx = nullptr;
-    uint32_t n = 0, fmt = 0;
+    uint32_t n = 0;
+    bool steps = false;   // distances wanted: 64-bit entries (with them) once solved
     uint64_t N = 0;
-    size_t entry_bytes = 0;
+    size_t entry_bytes = 0;   // of a buffer's entries; `narrow` tables use half of 8
+    bool narrow = false;  // the current table has 32-bit entries (a table with steps
+                          // starts so: every distance is 1 until it is solved)
     void* buf[2] = {nullptr, nullptr};
     int cur = 0;          // buffer holding the current table
     bool any_stop = false;
@@ -489,7 +495,7 @@ int plan_table(const Circuit& circ, bool steps, KernelConfig* kc, std::string* e
     uint32_t fmt;
     if (steps) {
         if (n > 31) { *err = "steps need n <= 31"; return NSAT_EUNSUPPORTED; }
-        fmt = 2;
+        fmt = 0;
     } else {
         fmt = (n <= 31 && !chunked) ? 0 : 1;
     }
@@ -560,6 +566,8 @@ extern "C" int nsat_create(int device, const nsat_opts* opts, nsat_ctx** out) {
     CK(cudaMallocHost(&ctx->h_init, sizeof(LaunchOut)));
     CK(cudaMalloc(&ctx->d_join, sizeof(NsatJoinState)));
     CK(cudaMallocHost(&ctx->h_join, sizeof(NsatJoinState)));
+    CK(cudaMalloc(&ctx->d_stop, sizeof(NsatStopState)));
+    CK(cudaMallocHost(&ctx->h_stop, sizeof(NsatStopState)));
     memset(ctx->h_init, 0, sizeof(LaunchOut));
     ctx->h_init->min_idx = ~0ull;
     for (int i = 0; i < kRing; i++) {
@@ -589,6 +597,8 @@ extern "C" void nsat_destroy(nsat_ctx* ctx) {
     cudaFree(ctx->d_data);
     cudaFree(ctx->d_join);
     cudaFreeHost(ctx->h_join);
+    cudaFree(ctx->d_stop);
+    cudaFreeHost(ctx->h_stop);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     delete ctx;
@@ -956,6 +966,11 @@ cudaError_t nsat::ctx_alloc(nsat_ctx* ctx, void** p, size_t bytes) {
 void nsat::ctx_free(nsat_ctx* ctx, void* p) {
     if (p) cudaFreeAsync(p, ctx->stream);
 }
+void nsat::ctx_stop_state(nsat_ctx* ctx, NsatStopState** dev, NsatStopState** host) {
+    *dev = ctx->d_stop;
+    *host = ctx->h_stop;
+}
+cudaEvent_t nsat::ctx_stop_event(nsat_ctx* ctx) { return ctx->evd[0]; }
 void nsat::ctx_trim(nsat_ctx* ctx) {
     cudaStreamSynchronize(ctx->stream);
     cudaMemPoolTrimTo(ctx->pool, 0);
@@ -1002,9 +1017,10 @@ extern "C" int nsat_stop_table_build(nsat_ctx* ctx, nsat_circuit* c, const nsat_
     std::unique_ptr<nsat_table> t(new nsat_table());
     t->ctx = ctx;
     t->n = n;
-    t->fmt = kc.fmt;
+    t->steps = opts && opts->want_steps;
     t->N = 1ull << n;
-    t->entry_bytes = kc.fmt == 0 ? 4 : 8;
+    t->entry_bytes = kc.fmt == 0 && !t->steps ? 4 : 8;
+    t->narrow = kc.fmt == 0;
     const size_t bytes = std::max<size_t>(t->N * t->entry_bytes, 256);
     for (int i = 0; i < 2; i++) {
         cudaError_t e = ctx_alloc(ctx, &t->buf[i], bytes);
@@ -1092,8 +1108,8 @@ extern "C" int nsat_table_read(nsat_table* t, uint64_t first, uint64_t count, ui
     if (!t || !out || first > t->N || count > t->N - first) return NSAT_EINVAL;
     nsat_ctx* ctx = t->ctx;
     if (int rc = set_device(ctx)) return rc;
-    const uint64_t mask = (t->fmt == 2) ? 0xffffffffull : ~0ull;
-    if (t->entry_bytes == 4) {
+    const uint64_t mask = t->steps ? 0xffffffffull : ~0ull;
+    if (t->narrow) {
         std::vector<uint32_t> tmp(count);
         CK(cudaMemcpy(tmp.data(), (uint32_t*)t->buf[t->cur] + first, count * 4, cudaMemcpyDeviceToHost));
         for (uint64_t i = 0; i < count; i++) out[i] = tmp[i];
@@ -1112,15 +1128,58 @@ extern "C" int nsat_stop_solve(nsat_ctx* ctx, nsat_table* t, const nsat_stop_opt
     if (int rc = set_device(ctx)) return rc;
     res->build_ms = t->build_ms;
     if (!t->any_stop) return NSAT_OK;   // check_stop: no state ever stops
+    const uint32_t n = t->n;
+    float ms = 0;
+    if (t->narrow) {
+        StopRun x;
+        x.n = n;
+        x.unknowns = opts->unknowns;
+        x.mode = opts->mode;
+        x.steps = t->steps;
+        x.done = ctx->ev1[0];
+        if (t->steps) {       // both 32-bit tables share buffer 0; buffer 1 takes the 64-bit result
+            x.a = (uint32_t*)t->buf[0];
+            x.b = x.a + t->N;
+            x.out64 = (uint64_t*)t->buf[1];
+        } else {
+            x.a = (uint32_t*)t->buf[t->cur];
+            x.b = (uint32_t*)t->buf[t->cur ^ 1];
+        }
+        CK(cudaEventRecord(ctx->ev0[0], ctx->stream));
+        const int rc = stop_run(ctx, &x);
+        if (rc == NSAT_OK) {
+            CK(cudaEventElapsedTime(&ms, ctx->ev0[0], ctx->ev1[0]));
+            res->join_ms = ms;
+            res->rounds = x.rounds;
+            if (t->steps) {
+                t->narrow = false;
+                t->cur = 1;
+            } else {
+                t->cur = x.table == (uint32_t*)t->buf[0] ? 0 : 1;
+            }
+            if (x.found) {
+                res->found = 1;
+                res->start = x.start;
+                res->end = x.entry & ((1ull << n) - 1);
+                res->steps = t->steps ? x.steps_of : 0;
+            }
+            return NSAT_OK;
+        }
+        if (rc != NSAT_ENOMEM) return rc;
+        // no room for the distances: 64-bit entries from here on
+        if (nsat_stop_widen(x.a, nullptr, t->N, n, 0, x.out64, ctx->sm_count, ctx->stream))
+            return fail(ctx, NSAT_ECUDA, "join launch failed");
+        t->narrow = false;
+        t->cur = 1;
+    }
     NsatJoinState* h = ctx->h_join;
     memset(h, 0, sizeof(*h));
     for (int i = 0; i < 72; i++) h->best[i] = ~0ull;
     CK(cudaMemcpyAsync(ctx->d_join, h, sizeof(*h), cudaMemcpyHostToDevice, ctx->stream));
-    const uint32_t n = t->n;
     CK(cudaEventRecord(ctx->ev0[0], ctx->stream));
     int src = t->cur;
     for (uint32_t r = 1; r <= n; r++) {
-        int rc = nsat_launch_join_round((int)t->fmt, t->buf[src], t->buf[src ^ 1], t->N, n, opts->unknowns, r,
+        int rc = nsat_launch_join_round(t->steps ? 2 : 1, t->buf[src], t->buf[src ^ 1], t->N, n, opts->unknowns, r,
                                         opts->mode, ctx->d_join, ctx->sm_count, ctx->stream);
         if (rc) return fail(ctx, NSAT_ECUDA, "join launch failed");
         src ^= 1;
@@ -1128,7 +1187,6 @@ extern "C" int nsat_stop_solve(nsat_ctx* ctx, nsat_table* t, const nsat_stop_opt
     CK(cudaEventRecord(ctx->ev1[0], ctx->stream));
     CK(cudaMemcpyAsync(h, ctx->d_join, sizeof(*h), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    float ms = 0;
     CK(cudaEventElapsedTime(&ms, ctx->ev0[0], ctx->ev1[0]));
     res->join_ms = ms;
     const uint32_t fr = h->final_round ? h->final_round : n;
@@ -1139,17 +1197,11 @@ extern "C" int nsat_stop_solve(nsat_ctx* ctx, nsat_table* t, const nsat_stop_opt
     t->cur = buf;
     if (best != ~0ull) {
         uint64_t e = 0;
-        if (t->entry_bytes == 4) {
-            uint32_t v;
-            CK(cudaMemcpy(&v, (uint32_t*)t->buf[buf] + best, 4, cudaMemcpyDeviceToHost));
-            e = v;
-        } else {
-            CK(cudaMemcpy(&e, (uint64_t*)t->buf[buf] + best, 8, cudaMemcpyDeviceToHost));
-        }
+        CK(cudaMemcpy(&e, (uint64_t*)t->buf[buf] + best, 8, cudaMemcpyDeviceToHost));
         res->found = 1;
         res->start = best;
         res->end = e & ((1ull << n) - 1);
-        res->steps = t->fmt == 2 ? (e >> 32) : 0;
+        res->steps = t->steps ? (e >> 32) : 0;
     }
     return NSAT_OK;
 }

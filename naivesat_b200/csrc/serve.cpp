@@ -38,7 +38,7 @@
 #include "qreducer.h"
 #include "serve_common.h"
 #include "serve_kernels.h"
-#include "static_kernels.h"
+#include "stop_join.h"
 
 using namespace nsat;
 
@@ -297,8 +297,6 @@ struct nsat_server {
     SrvState* d_state = nullptr;     // kMaxActive persistent job states (cursor, results)
     SrvState* h_state_init = nullptr;
     std::vector<uint32_t> free_slots;
-    NsatJoinState* d_join = nullptr;
-    NsatJoinState* h_join = nullptr;
     uint64_t epochs = 0, launches = 0;
     uint64_t launched = 0;   // epochs launched (the sequence number of the last one)
     uint32_t shape = 0;      // interpreter shape (index into kSrvShapes)
@@ -365,8 +363,6 @@ struct nsat_server {
         cudaFree(arena.base);
         cudaFree(d_state);
         cudaFreeHost(h_state_init);
-        cudaFree(d_join);
-        cudaFreeHost(h_join);
     }
 };
 
@@ -427,6 +423,7 @@ void finish(nsat_server* s, Job* j) {
 
 size_t prog_bytes(const Job* j) { return j->prog.ins.size() * sizeof(SrvIns) + sizeof(SrvIns); }
 size_t outs_bytes(const Job* j) { return j->prog.outs.size() * 2 + 2; }
+// SATOSTOP: two areas of 2^n 8-byte entries (the first holds the 32-bit table)
 size_t table_bytes(const Job* j) { return j->kind == SRV_TABLE ? ((size_t)8 << j->n) : 0; }
 
 int admit(nsat_server* s, Job* j) {
@@ -459,7 +456,7 @@ int admit(nsat_server* s, Job* j) {
     r.outs = (const uint16_t*)(s->arena.base + j->outs_off);
     r.st = s->d_state + j->slot;
     r.flags = j->find_all ? SRV_JOB_FIND_ALL : 0u;
-    r.table = tbytes ? (srv_u64*)(s->arena.base + j->table_off) : nullptr;
+    r.table = tbytes ? (uint32_t*)(s->arena.base + j->table_off) : nullptr;
     r.ngroups = (uint32_t)(j->prog.ins.size() / kSrvShapes[s->shape].group);
     r.nslots = j->prog.nslots;
     r.kind = j->kind;
@@ -501,35 +498,26 @@ void release(nsat_server* s, Job* j) {
 // Synchronous doubling on a finished table (naivesatostop: lowest stopping
 // start, with steps).
 int run_joins(nsat_server* s, Job* j) {
-    cudaStream_t st = ctx_stream(s->ctx);
     j->res.found = 0;
     if (!j->any_stop) return NSAT_OK;
-    NsatJoinState* h = s->h_join;
-    memset(h, 0, sizeof(*h));
-    for (int i = 0; i < 72; i++) h->best[i] = ~0ull;
-    SCK(cudaMemcpyAsync(s->d_join, h, sizeof(*h), cudaMemcpyHostToDevice, st));
-    s->h2d_bytes += sizeof(*h);
-    s->d2h_bytes += sizeof(*h) + 8;
-    void* buf[2] = {s->arena.base + j->table_off, s->arena.base + j->table2_off};
-    int src = 0;
-    for (uint32_t r = 1; r <= j->n; r++) {
-        if (nsat_launch_join_round(2, buf[src], buf[src ^ 1], 1ull << j->n, j->n, j->unknowns, r, 1, s->d_join,
-                                   ctx_sm_count(s->ctx), st))
-            return ctx_fail(s->ctx, NSAT_ECUDA, "join launch failed");
-        s->launches++;
-        src ^= 1;
-    }
-    SCK(cudaMemcpyAsync(h, s->d_join, sizeof(*h), cudaMemcpyDeviceToHost, st));
-    SCK(cudaStreamSynchronize(st));
-    const uint32_t fr = h->final_round ? h->final_round : j->n;
-    const uint64_t best = h->best[fr];
-    if (best != ~0ull) {
-        uint64_t e = 0;
-        SCK(cudaMemcpy(&e, (uint64_t*)buf[fr & 1] + best, 8, cudaMemcpyDeviceToHost));
+    StopRun x;
+    x.n = j->n;
+    x.unknowns = j->unknowns;
+    x.mode = 1;
+    x.steps = true;
+    // the second area holds the other 32-bit table and the distances
+    x.a = (uint32_t*)(s->arena.base + j->table_off);
+    x.b = (uint32_t*)(s->arena.base + j->table2_off);
+    x.dist = x.b + (1ull << j->n);
+    if (int rc = stop_run(s->ctx, &x)) return rc;
+    s->launches += x.launches;
+    s->h2d_bytes += sizeof(NsatStopState);
+    s->d2h_bytes += sizeof(NsatStopState) + 8;
+    if (x.found) {
         j->res.found = 1;
-        j->res.start = best;
-        j->res.end = e & ((1ull << j->n) - 1);
-        j->res.steps = e >> 32;
+        j->res.start = x.start;
+        j->res.end = x.entry & ((1ull << j->n) - 1);
+        j->res.steps = x.steps_of;
     }
     return NSAT_OK;
 }
@@ -773,8 +761,6 @@ extern "C" int nsat_server_create(nsat_ctx* ctx, const nsat_server_opts* opts, n
     memset(s->h_state_init, 0, sizeof(SrvState));
     s->h_state_init->min_idx = ~0ull;
     for (uint32_t k = kMaxActive; k-- > 0;) s->free_slots.push_back(k);
-    SCK(cudaMalloc(&s->d_join, sizeof(NsatJoinState)));
-    SCK(cudaMallocHost(&s->h_join, sizeof(NsatJoinState)));
     // defaults measured on the 10,000-request mixed serving trace: 30 ms and
     // 8 workers took its first 3000 requests from 366 to 609 solves/s; on all
     // of it, 12 workers (the compiles are the limit) reach 517 solves/s

@@ -82,7 +82,7 @@ struct SrvJob {
     const SrvIns* prog;          // ngroups * G instructions (G: the server shape's group size)
     SrvState* st;                // the job's persistent cursor and results
     const uint16_t* outs;        // output slots (bit 15 = negated), nout of them
-    srv_u64* table;             // TABLE: 2^np u64 entries (next|STOP<<n | 1<<32)
+    uint32_t* table;             // TABLE: 2^n u32 entries (next | STOP<<n)
     uint32_t ngroups;
     uint32_t nslots;
     uint32_t kind;               // SRV_SAT / SRV_QSAT / SRV_TABLE

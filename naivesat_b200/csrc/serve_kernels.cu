@@ -339,8 +339,16 @@ __device__ __forceinline__ void do_tile(SrvJob* J, u64 tile, char* __restrict__ 
                 transpose32(o);
                 const u64 word = (tile_base >> 5) + ((u64)(it * W + w) << 5) + lane;   // word index
                 if ((word << 5) < states) {
-                    srv_u64* dst = J->table + (word << 5);
-                    for (u32 l = 0; l < lanes; l++) dst[l] = (srv_u64)o[l] | (1ull << 32);
+                    u32* dst = J->table + (word << 5);
+                    if (lanes == 32u) {
+#pragma unroll
+                        for (int q = 0; q < 8; q++)
+                            reinterpret_cast<uint4*>(dst)[q] = make_uint4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
+                    } else {
+#pragma unroll
+                        for (int l = 0; l < 16; l++)
+                            if ((u32)l < lanes) dst[l] = o[l];
+                    }
                 }
             }
             if (__any_sync(0xffffffffu, stop_any != 0u) && lane == 0) atomicOr(&J->st->any, 1u);

@@ -11,15 +11,12 @@ typedef unsigned long long u64;
 
 namespace {
 
-// Entry formats of the next-state table.
-//   FMT 0: u32  next | STOP << n            (n <= 31)
+// Entry formats of the next-state tables of 64-bit entries (tables of 32-bit
+// entries: stop_kernels.cu).
 //   FMT 1: u64  next | STOP << n            (n <= 63)
 //   FMT 2: u64  (next | STOP << n) | dist << 32   (n <= 31)
-template <int FMT> struct EntryT { typedef u64 type; };
-template <> struct EntryT<0> { typedef u32 type; };
-
-template <int FMT, typename E>
-__device__ __forceinline__ E combine(E v, E w) {
+template <int FMT>
+__device__ __forceinline__ u64 combine(u64 v, u64 w) {
     if constexpr (FMT == 2) {
         return (w & 0xffffffffull) | (((v >> 32) + (w >> 32)) << 32);
     } else {
@@ -42,11 +39,11 @@ __device__ __forceinline__ u64 warp_min(u64 v) {
 // with find_solution (greedysatostop.rs:883-895): the lowest start whose entry
 // now has STOP is min-reduced into st->best[r].
 template <int FMT>
-__global__ void __launch_bounds__(256) join_round(const typename EntryT<FMT>::type* __restrict__ src,
-                                                  typename EntryT<FMT>::type* __restrict__ dst,
+__global__ void __launch_bounds__(256) join_round(const u64* __restrict__ src,
+                                                  u64* __restrict__ dst,
                                                   u64 N, u32 n, u32 u, u32 r, u32 mode,
                                                   NsatJoinState* __restrict__ st) {
-    typedef typename EntryT<FMT>::type E;
+    typedef u64 E;
     if (r > 1) {
         const u64 pb = *(volatile u64*)&st->best[r - 1];
         if (pb != ~0ull && (mode == 0 || pb == 0)) {
@@ -157,9 +154,6 @@ extern "C" int nsat_launch_join_round(int fmt, const void* src, void* dst, uint6
     unsigned blocks = (unsigned)(want < cap ? want : cap);
     if (blocks == 0) blocks = 1;
     switch (fmt) {
-    case 0:
-        join_round<0><<<blocks, threads, 0, stream>>>((const u32*)src, (u32*)dst, N, n, u, r, mode, st);
-        break;
     case 1:
         join_round<1><<<blocks, threads, 0, stream>>>((const u64*)src, (u64*)dst, N, n, u, r, mode, st);
         break;
