@@ -67,3 +67,35 @@ def test_rounds_match_plain_doubling(ctx, n, kind, unknowns, mode, steps):
             assert r["steps"] == (int(dist[best]) if steps else 0)
         np.testing.assert_array_equal(t.read(), table.astype(np.uint64))
     t.close()
+
+
+@pytest.mark.parametrize("n,stop_bits,unknowns,partitions", [
+    (11, 3, 11, 2), (11, 8, 4, 32), (12, 12, 12, 64), (13, 10, 7, 16), (16, 2, 16, 1024), (18, 13, 3, 4),
+    (19, 19, 19, 8), (21, 12, 0, 2),
+])
+def test_device_table_steps_match_host_image(ctx, n, stop_bits, unknowns, partitions):
+    """The two-kernel steps over a device table against one kernel per join
+    over a host image, up to the smallest partitions (64 entries)."""
+    h = ctx.circuit(machine(n + stop_bits, n, stop_bits))
+    a = h.greedy_partitioned(unknowns, partitions)
+    b = h.greedy_partitioned(unknowns, partitions, device_bytes=1)
+    assert (a["storage"], b["storage"]) == (0, 1)
+    keys = ("found", "start", "end", "stage", "partition", "joins", "load_bits")
+    assert {k: a[k] for k in keys} == {k: b[k] for k in keys}
+
+
+@pytest.mark.parametrize("n", [5, 9, 10, 11, 15, 17, 20])
+def test_table_words(ctx, n):
+    """Tables below and above the staged size."""
+    c = machine(n, n, 3)
+    t = ctx.circuit(c).stop_table()
+    got = t.read()
+    t.close()
+    s = np.arange(1 << n, dtype=np.uint32)
+    w = [((s >> np.uint32(i)) & 1).astype(bool) for i in range(n)]
+    for f, a, b in c.gates.tolist():
+        w.append([w[a] & w[b], ~(w[a] | w[b]), w[a] & ~w[b], w[a] ^ w[b]][f])
+    exp = np.zeros(1 << n, dtype=np.uint64)
+    for k, (o, neg) in enumerate(c.outputs.tolist()):
+        exp |= (w[o] ^ bool(neg)).astype(np.uint64) << np.uint64(k)
+    np.testing.assert_array_equal(got, exp)
