@@ -17,8 +17,11 @@
 //   this stage), or, for j == i, a copy of dest as it is at that point; then
 //   the lowest unknown start of dest with STOP is the answer, else dest is
 //   written back.
-// dest is unpacked to u64 entries for the race-free in-place join; the other
-// partitions are read packed by the join's gathers.
+// Where a table of 32-bit entries fits the device (n <= 31) the image is not
+// packed: it is built in one launch and a step is two kernels over it
+// (nsat_greedy_step).  Otherwise dest is unpacked to u64 entries for the
+// race-free in-place join, and the other partitions are read packed by the
+// join's gathers, one kernel per join.
 #include <cuda_runtime.h>
 #include <fcntl.h>
 #include <unistd.h>
@@ -82,6 +85,9 @@ struct Work {
     uint64_t* stage[2] = {nullptr, nullptr};   // HOST/FILEIMG: packed partitions on the device
     uint64_t* chunk = nullptr;        // first pass: u64 entries of one chunk
     uint64_t* best = nullptr;
+    uint32_t* table32 = nullptr;      // DEVICE: 32-bit entries instead of the packed image
+    uint32_t* snap32 = nullptr;
+    NsatGreedyState* state = nullptr;
     cudaStream_t copy = nullptr;
     cudaEvent_t ready[2] = {nullptr, nullptr}, used[2] = {nullptr, nullptr};
     cudaEvent_t wb = nullptr;
@@ -91,7 +97,7 @@ struct Work {
         if (copy) cudaStreamSynchronize(copy);   // the copy stream's uses end before the frees
         if (ctx) {
             for (void* p : {(void*)dev_image, (void*)dest, (void*)snap, (void*)stage[0], (void*)stage[1],
-                            (void*)chunk, (void*)best})
+                            (void*)chunk, (void*)best, (void*)table32, (void*)snap32, (void*)state})
                 ctx_free(ctx, p);
         }
         if (host_image) cudaFreeHost(host_image);
@@ -142,10 +148,19 @@ int setup(nsat_ctx* ctx, Work& w, uint32_t n, uint64_t L, uint64_t chunk, const 
     w.bytes = packed_bytes(1ull << n, bits);
     const uint64_t pbytes = packed_bytes(L, bits), cbytes = packed_bytes(chunk, bits);
     const uint64_t work_dev = (joins ? 2 * L * 8 : 0) + chunk * 8 + 64;
+    const uint64_t table32 = ((1ull << n) + L) * 4 + sizeof(NsatGreedyState);
+    uint64_t budget = 0;
     if (o->file_prefix) {
         w.storage = FILEIMG;
     } else {
-        uint64_t budget = o->device_bytes;
+        budget = o->device_bytes;
+        const uint64_t take = n <= 31 && joins ? table32 : w.bytes + work_dev;   // what is allocated below
+        if (!budget && take <= ctx_pool_unused(ctx)) {
+            // buffers that an earlier call gave back to the pool are enough: no
+            // need to ask the driver for the free memory (70 us, and on a host
+            // shared with other jobs now and then tens of milliseconds)
+            budget = std::max(table32, w.bytes + work_dev);
+        }
         if (!budget) {
             // free device memory less 1 GiB; if the image does not fit, what
             // the context's pool keeps for reuse is returned and counted too
@@ -161,6 +176,12 @@ int setup(nsat_ctx* ctx, Work& w, uint32_t n, uint64_t L, uint64_t chunk, const 
         w.storage = (w.bytes + work_dev <= budget) ? DEVICE : HOST;
     }
     if (w.storage == DEVICE) {
+        if (n <= 31 && joins && table32 <= budget) {       // everything runs on the context's stream
+            GCK(ctx_alloc(ctx, (void**)&w.table32, 4ull << n));
+            GCK(ctx_alloc(ctx, (void**)&w.snap32, L * 4));
+            GCK(ctx_alloc(ctx, (void**)&w.state, sizeof(NsatGreedyState)));
+            return NSAT_OK;
+        }
         GCK(ctx_alloc(ctx, (void**)&w.dev_image, w.bytes));
     } else {
         for (int k = 0; k < 2; k++) GCK(ctx_alloc(ctx, (void**)&w.stage[k], std::max(pbytes, cbytes)));
@@ -241,10 +262,18 @@ int build_image(nsat_ctx* ctx, nsat_circuit* c, Work& w, uint32_t lb, bool* any_
     cudaStream_t st = ctx_stream(ctx);
     const int sms = ctx_sm_count(ctx);
     *any_stop = false;
+    if (w.table32) {       // the whole table at once
+        uint32_t stop = 0;
+        float ms = 0;
+        if (int rc = table_chunk(ctx, c, 0, 1ull << n, false, w.table32, &stop, &ms)) return rc;
+        r->build_ms = ms;
+        *any_stop = stop != 0;
+        return NSAT_OK;
+    }
     for (uint64_t a = 0; a < (1ull << lb); a++) {
         uint32_t stop = 0;
         float ms = 0;
-        if (int rc = table_chunk_u64(ctx, c, a * chunk, chunk, w.chunk, &stop, &ms)) return rc;
+        if (int rc = table_chunk(ctx, c, a * chunk, chunk, true, w.chunk, &stop, &ms)) return rc;
         r->build_ms += ms;
         *any_stop |= stop != 0;
         if (w.storage == DEVICE) {
@@ -332,6 +361,46 @@ int join_partition(nsat_ctx* ctx, Work& w, uint32_t n, uint32_t P, uint64_t L, u
     return NSAT_OK;
 }
 
+// The stages over a device table of 32-bit entries.  Steps are queued without
+// waiting (a step behind the answer does nothing); the host looks after each
+// stage, or every kStepsQueued steps of one.
+int run_table32(nsat_ctx* ctx, Work& w, uint32_t n, uint32_t P, uint32_t pbits, uint32_t unknowns,
+              nsat_greedy_result* r) {
+    constexpr uint32_t kStepsQueued = 32;
+    cudaStream_t st = ctx_stream(ctx);
+    const int sms = ctx_sm_count(ctx);
+    cudaEvent_t e0, e1;
+    ctx_timing_events(ctx, &e0, &e1);
+    NsatGreedyState h{~0ull, 0u, 0u};
+    GCK(cudaMemcpyAsync(w.state, &h, sizeof(h), cudaMemcpyHostToDevice, st));
+    uint64_t step = 0;                       // n * P < 2^32: P <= 2^(n-6), n <= 31
+    for (const uint64_t steps = (uint64_t)n * P; step < steps;) {
+        const uint64_t until = std::min<uint64_t>(steps, step + std::min(P, kStepsQueued));
+        GCK(cudaEventRecord(e0, st));
+        for (uint64_t s = step; s < until; s++)
+            KCK(nsat_greedy_step(w.table32, w.snap32, (uint32_t)(s & (P - 1)), n - pbits, n, unknowns, (uint32_t)s,
+                                 w.state, sms, st));
+        GCK(cudaEventRecord(e1, st));
+        GCK(cudaMemcpyAsync(&h, w.state, sizeof(h), cudaMemcpyDeviceToHost, st));
+        GCK(cudaStreamSynchronize(st));
+        float ms = 0;
+        GCK(cudaEventElapsedTime(&ms, e0, e1));
+        r->join_ms += ms;
+        if (h.key != ~0ull) {
+            r->found = 1;
+            r->start = h.key >> 32;
+            r->end = h.key & ((1ull << n) - 1);
+            r->stage = h.step / P;
+            r->partition = h.step & (P - 1);
+            r->joins = ((uint64_t)h.step + 1) * P;
+            return NSAT_OK;
+        }
+        step = until;
+        r->joins = step * P;
+    }
+    return NSAT_OK;
+}
+
 }  // namespace
 
 extern "C" int nsat_greedy_solve(nsat_ctx* ctx, nsat_circuit* c, const nsat_greedy_opts* o, nsat_greedy_result* r) {
@@ -358,6 +427,11 @@ extern "C" int nsat_greedy_solve(nsat_ctx* ctx, nsat_circuit* c, const nsat_gree
     if (!any_stop) {
         r->wall_ms = now_ms() - t0;
         return NSAT_OK;
+    }
+    if (w.table32) {
+        const int rc = run_table32(ctx, w, n, P, pbits, o->unknowns, r);
+        r->wall_ms = now_ms() - t0;
+        return rc;
     }
     cudaStream_t st = ctx_stream(ctx);
     const int sms = ctx_sm_count(ctx);

@@ -102,6 +102,96 @@ __global__ void find_kernel(const u64* __restrict__ dest, u64 start, u64 count, 
     }
 }
 
+// Partition steps of a device table of 32-bit entries (n <= 31).
+//
+// A step joins partition i with every partition j in order.  An entry's joins
+// are independent of its neighbours' except for j == i, which gathers from
+// partition i as it is after the joins with j < i.  So a step is two kernels:
+// chase_before follows each entry through the partitions below i (it jumps
+// whenever its next state lies in a partition that is still to come) into a
+// snapshot; chase_after goes on through the snapshot and the partitions above
+// i, takes the lowest unknown start with STOP and writes the partition back.
+// That is two reads and two writes of 4 bytes per entry besides the gathers,
+// which bound it (the L1 tag stage: one random word per SM clock).  A kernel
+// per join reads and writes 8-byte entries P times, gathers from packed
+// entries (a second word for 40 % of them) and unpacks, copies, searches and
+// packs in passes of their own: 2^26 states in 4 partitions take 340 us a step
+// that way and 140 us in two kernels.
+//
+// A thread follows four neighbouring entries: one 16-byte access each way and
+// four gathers in flight.
+
+// Follows the entries through the partitions of the state range [lo, hi) in
+// order: an entry jumps while its next state lies at or above the end of the
+// partition it jumped to last; one with STOP lies above every range.  States
+// below own_end are read from snap.
+__device__ __forceinline__ void chase(u32 (&v)[4], const u32* table, const u32* snap, u32 own_end, u32 lo, u32 hi,
+                                      u32 imask) {
+    u32 from[4] = {lo, lo, lo, lo};
+    for (;;) {
+        bool on[4], any = false;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            on[k] = v[k] >= from[k] && v[k] < hi;
+            any |= on[k];
+        }
+        if (!any) return;
+        u32 w[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (on[k]) w[k] = v[k] < own_end ? snap[v[k] & imask] : table[v[k]];
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (on[k]) {
+                from[k] = (v[k] | imask) + 1u;
+                v[k] = w[k];
+            }
+    }
+}
+
+__global__ void __launch_bounds__(256) chase_before(const u32* __restrict__ table, u32 i, u32 lp,
+                                                    u32* __restrict__ snap, NsatGreedyState* st) {
+    // only chase_after writes the key: here it is that of an earlier step
+    if (*(volatile const u64*)&st->key != ~0ull) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) st->done = 1u;
+        return;
+    }
+    const u32 quads = 1u << (lp - 2), first = i << lp;
+    const uint4* in = reinterpret_cast<const uint4*>(table + first);
+    for (u32 q = blockIdx.x * blockDim.x + threadIdx.x; q < quads; q += gridDim.x * blockDim.x) {
+        const uint4 t = in[q];
+        u32 v[4] = {t.x, t.y, t.z, t.w};
+        chase(v, table, nullptr, 0u, 0u, first, (1u << lp) - 1u);
+        reinterpret_cast<uint4*>(snap)[q] = make_uint4(v[0], v[1], v[2], v[3]);
+    }
+}
+
+__global__ void __launch_bounds__(256) chase_after(u32* table, const u32* __restrict__ snap, u32 i, u32 lp, u32 n,
+                                                   u32 unknowns, u32 step, NsatGreedyState* st) {
+    if (*(volatile const u32*)&st->done) return;
+    const u32 stop = 1u << n, before = (u32)((1ull << (n - unknowns)) - 1ull);
+    const u32 quads = 1u << (lp - 2), first = i << lp;
+    u64 best = ~0ull;
+    for (u32 q = blockIdx.x * blockDim.x + threadIdx.x; q < quads; q += gridDim.x * blockDim.x) {
+        const uint4 t = reinterpret_cast<const uint4*>(snap)[q];
+        u32 v[4] = {t.x, t.y, t.z, t.w};
+        chase(v, table, snap, first + (1u << lp), first, stop, (1u << lp) - 1u);
+        reinterpret_cast<uint4*>(table + first)[q] = make_uint4(v[0], v[1], v[2], v[3]);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const u32 s = first + 4u * q + k;
+            if ((v[k] & stop) && (s & before) == 0u) {
+                const u64 key = ((u64)s << 32) | v[k];
+                best = key < best ? key : best;
+            }
+        }
+    }
+    if (best != ~0ull) {
+        st->step = step;
+        atomicMin(&st->key, best);
+    }
+}
+
 unsigned grid_for(u64 items, int sms) {
     const u64 want = (items + 255) / 256;
     const u64 cap = (u64)sms * 8;
@@ -139,5 +229,13 @@ extern "C" int nsat_greedy_join_packed(uint64_t* dest, uint64_t count, const uin
 extern "C" int nsat_greedy_find(const uint64_t* dest, uint64_t start, uint64_t count, uint32_t n, uint32_t unknowns,
                                 uint64_t* best, int sms, cudaStream_t st) {
     find_kernel<<<grid_for(count, sms), 256, 0, st>>>((const u64*)dest, start, count, n, unknowns, (u64*)best);
+    return cudaGetLastError() == cudaSuccess ? 0 : -4;
+}
+
+extern "C" int nsat_greedy_step(uint32_t* table, uint32_t* snap, uint32_t i, uint32_t lp, uint32_t n,
+                                uint32_t unknowns, uint32_t step, NsatGreedyState* state, int sms, cudaStream_t st) {
+    const unsigned g = grid_for((u64)1 << (lp - 2), sms);
+    chase_before<<<g, 256, 0, st>>>(table, i, lp, snap, state);
+    chase_after<<<g, 256, 0, st>>>(table, snap, i, lp, n, unknowns, step, state);
     return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }

@@ -4,7 +4,19 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+// Device state of a solve over a device table (nsat_greedy_step).
+typedef struct {
+    unsigned long long key;    // start << 32 | entry of the lowest start found (~0 = none)
+    uint32_t step;             // the step that found it
+    uint32_t done;             // an earlier step has the answer
+} NsatGreedyState;
+
 extern "C" {
+// Step `step`: partition i (2^lp entries, lp >= 6) of the table of 32-bit
+// entries (n <= 31) joined with every partition in order and searched; does
+// nothing once an earlier step has an answer.  snap: 2^lp words.
+int nsat_greedy_step(uint32_t* table, uint32_t* snap, uint32_t i, uint32_t lp, uint32_t n, uint32_t unknowns,
+                     uint32_t step, NsatGreedyState* state, int sms, cudaStream_t st);
 // packed (bits-wide) entries -> u64 entries; count entries
 int nsat_greedy_unpack(const uint64_t* packed, uint64_t count, uint32_t bits, uint64_t* out, int sms,
                        cudaStream_t st);

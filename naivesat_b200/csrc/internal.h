@@ -35,6 +35,10 @@ void ctx_free(nsat_ctx* ctx, void* p);
 // The context's device state of a SATOSTOP solve and its pinned host copy.
 void ctx_stop_state(nsat_ctx* ctx, NsatStopState** dev, NsatStopState** host);
 cudaEvent_t ctx_stop_event(nsat_ctx* ctx);
+// A pair of timing events of the context, for one interval at a time.
+void ctx_timing_events(nsat_ctx* ctx, cudaEvent_t* begin, cudaEvent_t* end);
+// Bytes that the pool holds and no buffer uses.
+uint64_t ctx_pool_unused(nsat_ctx* ctx);
 // Returns the pool's unused memory to the device (after the context's
 // stream finishes), for a caller about to size a buffer by free memory.
 void ctx_trim(nsat_ctx* ctx);
@@ -57,11 +61,12 @@ int qsat_solve_blocks(nsat_ctx* ctx, nsat_circuit* c, const uint8_t* quants, uin
                       uint64_t first, uint64_t count,
                       const std::function<bool(uint64_t, const nsat_qsat_result&)>& on_block);
 
-// Next-state entries (next | STOP << n, u64) of states first_state ..
-// first_state+count-1 (both multiples of 32) into device memory dev_out, on
-// the context's stream (synchronous); any_stop reports a STOP among them.
-int table_chunk_u64(nsat_ctx* ctx, nsat_circuit* c, uint64_t first_state, uint64_t count, uint64_t* dev_out,
-                    uint32_t* any_stop, float* ms);
+// Next-state entries (next | STOP << n) of states first_state ..
+// first_state+count-1 (both multiples of 1024, n >= 10) into device memory
+// dev_out, as u64 (wide) or, for n <= 31, u32, on the context's stream
+// (synchronous); any_stop reports a STOP among them.
+int table_chunk(nsat_ctx* ctx, nsat_circuit* c, uint64_t first_state, uint64_t count, bool wide, void* dev_out,
+                uint32_t* any_stop, float* ms);
 
 const Circuit& circuit_of(const nsat_circuit* c);
 

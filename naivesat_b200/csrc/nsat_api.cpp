@@ -971,6 +971,20 @@ void nsat::ctx_stop_state(nsat_ctx* ctx, NsatStopState** dev, NsatStopState** ho
     *host = ctx->h_stop;
 }
 cudaEvent_t nsat::ctx_stop_event(nsat_ctx* ctx) { return ctx->evd[0]; }
+void nsat::ctx_timing_events(nsat_ctx* ctx, cudaEvent_t* begin, cudaEvent_t* end) {
+    *begin = ctx->ev0[0];
+    *end = ctx->ev1[0];
+}
+uint64_t nsat::ctx_pool_unused(nsat_ctx* ctx) {
+    uint64_t reserved = 0, used = 0;
+    cudaStreamSynchronize(ctx->stream);      // frees take effect in stream order
+    if (cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+        cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return reserved > used ? reserved - used : 0;
+}
 void nsat::ctx_trim(nsat_ctx* ctx) {
     cudaStreamSynchronize(ctx->stream);
     cudaMemPoolTrimTo(ctx->pool, 0);
@@ -1061,15 +1075,16 @@ extern "C" int nsat_stop_table_build(nsat_ctx* ctx, nsat_circuit* c, const nsat_
 
 namespace nsat {
 
-int table_chunk_u64(nsat_ctx* ctx, nsat_circuit* c, uint64_t first_state, uint64_t count, uint64_t* dev_out,
-                    uint32_t* any_stop, float* ms) {
+int table_chunk(nsat_ctx* ctx, nsat_circuit* c, uint64_t first_state, uint64_t count, bool wide, void* dev_out,
+                uint32_t* any_stop, float* ms) {
     if (int rc = set_device(ctx)) return rc;
     KernelConfig kc;
     std::string perr;
     if (int rc = plan_table(c->circ, false, &kc, &perr, true)) return fail(ctx, rc, perr);
     const uint32_t n = c->circ.n;
-    if (n < 5 || (first_state & 31) || (count & 31) || count == 0)
-        return fail(ctx, NSAT_EINVAL, "table chunks are whole 32-state words");
+    if (n < 10 || (first_state & 1023) || (count & 1023) || count == 0 || (!wide && n > 31))
+        return fail(ctx, NSAT_EINVAL, "table chunks are whole 1024-state tiles");
+    kc.fmt = wide ? 1 : 0;
     std::vector<uint32_t> which;
     for (uint32_t j = 0; j <= n; j++) which.push_back(j);
     const LutNet& net = get_net(c, which);
