@@ -127,11 +127,13 @@ __global__ void __launch_bounds__(kSmallThreads) small_solve(const u32* __restri
                                                              u32* __restrict__ out32, u64* __restrict__ out64,
                                                              NsatStopState* __restrict__ st) {
     extern __shared__ u32 sm[];
-    __shared__ u32 s_best[2];
+    __shared__ u32 s_best;        // lowest start that has stopped so far
     const u32 N = 1u << n, stop = N, smask = (1u << (n - u)) - 1u;
     u32* table = sm;
     u32* dist = sm + N;
     const u32 tid = threadIdx.x;
+    if (tid == 0) s_best = kNone;
+    __syncthreads();
     u32 v[E];
 #pragma unroll
     for (int k = 0; k < E; k++) {
@@ -140,40 +142,34 @@ __global__ void __launch_bounds__(kSmallThreads) small_solve(const u32* __restri
         if (i < N) {
             table[i] = v[k];
             if constexpr (STEPS) dist[i] = 1u;
+            if ((v[k] & stop) && (i & smask) == 0u) atomicMin(&s_best, i);
         }
     }
-    if (tid < 2) s_best[tid] = kNone;
     __syncthreads();
     u32 r = 1, best = kNone;
     for (;; r++) {
-        u32 b = kNone;
         u32 w[E];
 #pragma unroll
         for (int k = 0; k < E; k++) w[k] = (v[k] & stop) ? v[k] : table[v[k]];
 #pragma unroll
-        for (int k = E - 1; k >= 0; k--) {
-            const u32 i = tid + k * kSmallThreads;
-            if (i < N && (w[k] & stop)) {
+        for (int k = 0; k < E; k++) {
+            if ((w[k] & ~v[k]) & stop) {             // stops in this round: once per entry
+                const u32 i = tid + k * kSmallThreads;
                 // dist[v] belongs to an entry that stopped before this round:
                 // nobody writes it now
-                if constexpr (STEPS) if (!(v[k] & stop)) dist[i] = (1u << (r - 1)) + dist[v[k]];
-                if ((i & smask) == 0u) b = i;
+                if constexpr (STEPS) dist[i] = (1u << (r - 1)) + dist[v[k]];
+                if ((i & smask) == 0u) atomicMin(&s_best, i);
             }
         }
-        b = __reduce_min_sync(0xffffffffu, b);
-        if ((tid & 31u) == 0 && b != kNone) atomicMin(&s_best[r & 1u], b);
         __syncthreads();
-        best = s_best[r & 1u];
-        if (tid == 0) s_best[(r & 1u) ^ 1u] = kNone;     // read by all before the last barrier
-        const bool end = r == n || (best != kNone && (mode == 0 || best == 0));
+        best = s_best;
 #pragma unroll
         for (int k = 0; k < E; k++) {
-            const u32 i = tid + k * kSmallThreads;
-            if (i < N && !(v[k] & stop)) table[i] = w[k];
+            if (!(v[k] & stop)) table[tid + k * kSmallThreads] = w[k];
             v[k] = w[k];
         }
         __syncthreads();
-        if (end) break;
+        if (r == n || (best != kNone && (mode == 0 || best == 0))) break;
     }
 #pragma unroll
     for (int k = 0; k < E; k++) {
