@@ -236,9 +236,13 @@ class NsatError(RuntimeError):
     pass
 
 
+# byte -> 1 for A and a (All), 0 otherwise
+_IS_ALL = bytes(1 if chr(b) in "Aa" else 0 for b in range(256))
+
+
 def _quants_array(quants, n):
     if isinstance(quants, str):
-        q = np.array([1 if ch in "Aa" else 0 for ch in quants], dtype=np.uint8)
+        q = np.frombuffer(quants.encode("latin-1", "replace").translate(_IS_ALL), dtype=np.uint8)
     else:
         q = np.ascontiguousarray(np.asarray(quants, dtype=np.uint8))
     if len(q) != n:

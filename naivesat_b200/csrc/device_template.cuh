@@ -32,10 +32,36 @@ struct LaunchOut {
     u64 min_idx;   // SAT: lowest satisfying launch-relative index; QSAT: lowest decisive unit
     u64 count;     // SAT: solutions in this launch
     u32 tree;      // QSAT: tree value of the launch when no unit boundary is inside it
-    u32 ticket;    // CTAs finished (last-CTA tail), reset by the last CTA
+    u32 ticket;    // CTAs finished
     u32 any;       // table build: some STOP output seen
-    u32 err;
+    u32 values;    // QSAT: CTAs that have written their value (last-CTA tail)
 };
+
+// Ends a CTA, all threads together, after its last update of *out.  The last
+// CTA of the launch copies the result to pinned host memory and puts the slot
+// back as the next launch expects it: a solve is a kernel between two events,
+// where a copy that set the slot and one that read it back took 6 us of a
+// small solve.
+__device__ __forceinline__ void nsat_finish(LaunchOut* out, LaunchOut* host) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&out->ticket, 1u) == gridDim.x - 1u) {
+            __threadfence();
+            volatile LaunchOut* o = out;
+            volatile LaunchOut* h = host;
+            h->min_idx = o->min_idx;
+            h->count = o->count;
+            h->tree = o->tree;
+            h->any = o->any;
+            o->min_idx = ~0ull;
+            o->count = 0ull;
+            o->tree = 0u;
+            o->ticket = 0u;
+            o->any = 0u;
+        }
+    }
+}
 
 __device__ __forceinline__ u64 warp_min_u64(u64 v) {
 #pragma unroll
@@ -50,7 +76,7 @@ __device__ __forceinline__ u64 warp_min_u64(u64 v) {
 // --------------------------------------------------------------------------
 // SAT: count every satisfying assignment and find the lowest one.
 extern "C" __global__ void NSAT_BOUNDS
-nsat_sat(u64 launch, LaunchOut* __restrict__ out) {
+nsat_sat(u64 launch, LaunchOut* out, LaunchOut* host) {
     const u32 lane = threadIdx.x & 31u;
     const u32 warp = threadIdx.x >> 5;
     const u32 cta = blockIdx.x;
@@ -97,6 +123,7 @@ nsat_sat(u64 launch, LaunchOut* __restrict__ out) {
             }
         }
     }
+    nsat_finish(out, host);
 }
 #endif
 
@@ -146,7 +173,7 @@ __device__ constexpr int low_run(u64 allbits) {
 }
 
 extern "C" __global__ void NSAT_BOUNDS
-nsat_qsat(u64 launch, LaunchOut* __restrict__ out, unsigned char* __restrict__ scratch,
+nsat_qsat(u64 launch, LaunchOut* out, LaunchOut* host, unsigned char* __restrict__ scratch,
           const u32* __restrict__ data) {
     constexpr int M = NSAT_M;
     // Folding.  When levels 0..9 (the word and the warp tile) and the lowest
@@ -283,7 +310,7 @@ nsat_qsat(u64 launch, LaunchOut* __restrict__ out, unsigned char* __restrict__ s
                 if (threadIdx.x == 0) {
                     scratch[cta] = (unsigned char)cres;
                     __threadfence();
-                    const u32 t = atomicAdd(&out->ticket, 1u);
+                    const u32 t = atomicAdd(&out->values, 1u);
                     s_last = (t == (1u << NSAT_CB) - 1u) ? 1u : 0u;
                 }
                 __syncthreads();
@@ -325,11 +352,12 @@ nsat_qsat(u64 launch, LaunchOut* __restrict__ out, unsigned char* __restrict__ s
                             done = true;
                         }
                     }
-                    if (threadIdx.x == 0) out->ticket = 0u;
+                    if (threadIdx.x == 0) out->values = 0u;
                 }
             }
         }
     }
+    nsat_finish(out, host);
 }
 #endif
 
@@ -364,7 +392,7 @@ __device__ __forceinline__ void transpose32(u32* a) {
 constexpr bool NSAT_STAGED = NSAT_FMT == 0 && NSAT_NB >= 10;
 
 extern "C" __global__ void NSAT_BOUNDS
-nsat_table(u64 nwords, u64 w0, void* __restrict__ table, LaunchOut* __restrict__ out) {
+nsat_table(u64 nwords, u64 w0, void* __restrict__ table, LaunchOut* out, LaunchOut* host) {
     // entries of words w0 .. w0+nwords-1 (32 states each), stored from table[0]
     const u64 stride = (u64)gridDim.x * NSAT_NT;
     u32 anystop = 0;
@@ -413,5 +441,6 @@ nsat_table(u64 nwords, u64 w0, void* __restrict__ table, LaunchOut* __restrict__
 #endif
     }
     if (__any_sync(0xffffffffu, anystop != 0u) && (threadIdx.x & 31u) == 0) atomicOr(&out->any, 1u);
+    nsat_finish(out, host);
 }
 #endif

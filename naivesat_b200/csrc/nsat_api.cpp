@@ -40,10 +40,11 @@ struct LaunchOut {
     uint32_t tree;
     uint32_t ticket;
     uint32_t any;
-    uint32_t err;
+    uint32_t values;
 };
 static_assert(sizeof(LaunchOut) == 32, "LaunchOut layout");
 
+constexpr uint64_t kReadStage = 64 * 1024;
 constexpr int kRing = 4;   // launches in flight before the host reads results
 
 double now_ms() {
@@ -58,10 +59,11 @@ struct nsat_ctx {
     cudaStream_t stream = nullptr;
     int sm_count = 0;
     std::string last_err;
-    LaunchOut* d_out = nullptr;       // kRing slots
-    LaunchOut* h_out = nullptr;       // pinned mirror
-    LaunchOut* h_init = nullptr;      // pinned init template
-    cudaEvent_t ev0[kRing]{}, ev1[kRing]{}, evd[kRing]{};
+    char* d_fixed = nullptr;          // the device allocation behind d_out, d_join and d_stop
+    char* h_fixed = nullptr;          // the pinned one behind h_out, h_join, h_stop and h_read
+    LaunchOut* d_out = nullptr;       // kRing slots, put back to their first state by each launch
+    LaunchOut* h_out = nullptr;       // pinned: a launch's last CTA writes its result here
+    cudaEvent_t ev0[kRing]{}, ev1[kRing]{}, evd = nullptr;
     unsigned char* d_scratch = nullptr;
     size_t scratch_bytes = 0;
     uint32_t* d_data = nullptr;
@@ -70,6 +72,7 @@ struct nsat_ctx {
     NsatJoinState* h_join = nullptr;
     NsatStopState* d_stop = nullptr;
     NsatStopState* h_stop = nullptr;
+    void* h_read = nullptr;           // pinned, kReadStage bytes (nsat_table_read)
     // loaded kernels by everything their generated source depends on (the
     // kernel configuration, the entry point and the LUT net, compared
     // whole): a fresh circuit handle whose cover and launch configuration
@@ -89,12 +92,59 @@ constexpr uint64_t kPoolKeepBytes = 8ull << 30;
 struct Shape {
     uint32_t block_threads = 0, min_blocks = 0, cb_max = 0;
     uint32_t sync_every = 0;     // 0 = default (kDefaultSync); kNoSync = no barriers
+    bool operator==(const Shape& o) const {
+        return block_threads == o.block_threads && min_blocks == o.min_blocks && cb_max == o.cb_max &&
+               sync_every == o.sync_every;
+    }
 };
 
 constexpr uint32_t kDefaultSync = 64;
 constexpr uint32_t kNoSync = 0xffffffffu;
 
 uint32_t sync_of(const Shape& sh) { return sh.sync_every == kNoSync ? 0 : (sh.sync_every ? sh.sync_every : kDefaultSync); }
+
+// kernel plans (shared by the solvers and nsat_jit_check)
+struct SatPlan {
+    KernelConfig kc;
+    uint32_t d = 0, C = 0;
+    u128 bp = 0, ep = 0;   // range in the padded index space
+};
+
+struct QsatPlan {
+    KernelConfig kc;
+    std::vector<uint8_t> q;   // padded quantifiers
+    uint32_t n = 0, d = 0, np = 0, C = 0, A = 0;
+    uint32_t s = 0;           // fixed prefix bits (inputs 0..s-1)
+    uint32_t fsub = 0;        // first quantifier block of the problem below the prefix
+    uint32_t m = 0;           // unit level: np - (s + fsub)
+};
+
+// The last solve's plan and kernel of one kind, with everything they follow
+// from besides the circuit: a repeated call skips planning and the kernel
+// maps' string keys (10 us of a 35 us solve).
+struct SatMemo {
+    bool set = false;
+    uint32_t chunk_bits = 0;
+    u128 begin = 0, end = 0;
+    Shape shape;
+    SatPlan plan;
+    CUfunction fn = nullptr;
+    std::shared_ptr<JitModule> mod;
+};
+struct QsatMemo {
+    bool set = false;
+    uint32_t chunk_bits = 0, prefix_bits = 0;
+    std::vector<uint8_t> quants;
+    Shape shape;
+    QsatPlan plan;
+    CUfunction fn = nullptr;
+    std::shared_ptr<JitModule> mod;
+};
+struct TableMemo {
+    CUfunction fn = nullptr;
+    unsigned threads = 0;
+    std::shared_ptr<JitModule> mod;
+};
 
 struct nsat_circuit {
     nsat_ctx* ctx = nullptr;
@@ -106,6 +156,9 @@ struct nsat_circuit {
     std::map<std::string, std::pair<CUfunction, std::shared_ptr<JitModule>>> kernels;
     Shape tuned;                 // set by nsat_autotune (per kind)
     Shape tuned_qsat;
+    SatMemo sat_memo;
+    QsatMemo qsat_memo;
+    TableMemo table_memo[2];     // by entry format
 };
 
 struct nsat_table {
@@ -359,8 +412,6 @@ int run_ring(nsat_ctx* ctx, uint64_t total, Issue issue, Consume consume, double
         }
         if (!stop && issued < total && issued - done < (uint64_t)kRing) {
             const int slot = (int)(issued % kRing);
-            CK(cudaMemcpyAsync(ctx->d_out + slot, ctx->h_init, sizeof(LaunchOut), cudaMemcpyHostToDevice,
-                               ctx->stream));
             CK(cudaEventRecord(ctx->ev0[slot], ctx->stream));
             int rc = issue(issued, slot);
             if (rc) {
@@ -370,14 +421,11 @@ int run_ring(nsat_ctx* ctx, uint64_t total, Issue issue, Consume consume, double
                 return rc;
             }
             CK(cudaEventRecord(ctx->ev1[slot], ctx->stream));
-            CK(cudaMemcpyAsync(ctx->h_out + slot, ctx->d_out + slot, sizeof(LaunchOut), cudaMemcpyDeviceToHost,
-                               ctx->stream));
-            CK(cudaEventRecord(ctx->evd[slot], ctx->stream));
             issued++;
             continue;
         }
         const int slot = (int)(done % kRing);
-        CK(cudaEventSynchronize(ctx->evd[slot]));
+        CK(cudaEventSynchronize(ctx->ev1[slot]));
         float ms = 0;
         CK(cudaEventElapsedTime(&ms, ctx->ev0[slot], ctx->ev1[slot]));
         *dev_ms += ms;
@@ -392,13 +440,7 @@ int run_ring(nsat_ctx* ctx, uint64_t total, Issue issue, Consume consume, double
 
 
 // ---------------------------------------------------------------------------
-// kernel plans (shared by the solvers and nsat_jit_check)
-
-struct SatPlan {
-    KernelConfig kc;
-    uint32_t d = 0, C = 0;
-    u128 bp = 0, ep = 0;   // range in the padded index space
-};
+// kernel plans
 
 int plan_sat(uint32_t n, const nsat_sat_opts& o, const Shape& sh, SatPlan* pl, std::string* err, uint32_t lop3 = 0) {
     const uint32_t block_threads = sh.block_threads, min_blocks = sh.min_blocks;
@@ -429,15 +471,6 @@ int plan_sat(uint32_t n, const nsat_sat_opts& o, const Shape& sh, SatPlan* pl, s
     pl->d = d; pl->C = C; pl->bp = bp; pl->ep = ep;
     return NSAT_OK;
 }
-
-struct QsatPlan {
-    KernelConfig kc;
-    std::vector<uint8_t> q;   // padded quantifiers
-    uint32_t n = 0, d = 0, np = 0, C = 0, A = 0;
-    uint32_t s = 0;           // fixed prefix bits (inputs 0..s-1)
-    uint32_t fsub = 0;        // first quantifier block of the problem below the prefix
-    uint32_t m = 0;           // unit level: np - (s + fsub)
-};
 
 int plan_qsat(uint32_t n, const std::vector<uint8_t>& quants_in, bool data, uint32_t chunk_bits,
               const Shape& sh, uint32_t prefix_bits, QsatPlan* pl, std::string* err, uint32_t lop3 = 0) {
@@ -510,6 +543,20 @@ int plan_table(const Circuit& circ, bool steps, KernelConfig* kc, std::string* e
     return NSAT_OK;
 }
 
+// The next-state table kernel of format kc.fmt, kept on the circuit.
+int table_kernel(nsat_ctx* ctx, nsat_circuit* c, const KernelConfig& kc) {
+    TableMemo& memo = c->table_memo[kc.fmt];
+    if (memo.fn) return NSAT_OK;
+    std::vector<uint32_t> which;
+    for (uint32_t j = 0; j < kc.nout; j++) which.push_back(j);
+    const LutNet& net = get_net(c, which);
+    TableMemo m;
+    if (int rc = get_circuit_kernel(ctx, c, which, kc, net, "nsat_table", &m.fn, &m.mod)) return rc;
+    m.threads = kc.threads();
+    memo = std::move(m);
+    return NSAT_OK;
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -561,20 +608,29 @@ extern "C" int nsat_create(int device, const nsat_opts* opts, nsat_ctx** out) {
     CK(cudaMemPoolCreate(&ctx->pool, &pp));
     uint64_t keep = kPoolKeepBytes;
     CK(cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep));
-    CK(cudaMalloc(&ctx->d_out, sizeof(LaunchOut) * kRing));
-    CK(cudaMallocHost(&ctx->h_out, sizeof(LaunchOut) * kRing));
-    CK(cudaMallocHost(&ctx->h_init, sizeof(LaunchOut)));
-    CK(cudaMalloc(&ctx->d_join, sizeof(NsatJoinState)));
-    CK(cudaMallocHost(&ctx->h_join, sizeof(NsatJoinState)));
-    CK(cudaMalloc(&ctx->d_stop, sizeof(NsatStopState)));
-    CK(cudaMallocHost(&ctx->h_stop, sizeof(NsatStopState)));
-    memset(ctx->h_init, 0, sizeof(LaunchOut));
-    ctx->h_init->min_idx = ~0ull;
+    // the small fixed buffers in one allocation each: page-locking is the
+    // slowest part of creating a context, and a server creates a dozen
+    constexpr size_t kOut = 256, kJoin = 1024, kStop = 512;
+    static_assert(sizeof(LaunchOut) * kRing <= kOut && sizeof(NsatJoinState) <= kJoin && sizeof(NsatStopState) <= kStop,
+                  "fixed buffer sizes");
+    CK(cudaMalloc(&ctx->d_fixed, kOut + kJoin + kStop));
+    CK(cudaMallocHost(&ctx->h_fixed, kOut + kJoin + kStop + kReadStage));
+    ctx->d_out = (LaunchOut*)ctx->d_fixed;
+    ctx->d_join = (NsatJoinState*)(ctx->d_fixed + kOut);
+    ctx->d_stop = (NsatStopState*)(ctx->d_fixed + kOut + kJoin);
+    ctx->h_out = (LaunchOut*)ctx->h_fixed;
+    ctx->h_join = (NsatJoinState*)(ctx->h_fixed + kOut);
+    ctx->h_stop = (NsatStopState*)(ctx->h_fixed + kOut + kJoin);
+    ctx->h_read = ctx->h_fixed + kOut + kJoin + kStop;
+    memset(ctx->h_out, 0, sizeof(LaunchOut) * kRing);
     for (int i = 0; i < kRing; i++) {
+        ctx->h_out[i].min_idx = ~0ull;
         CK(cudaEventCreate(&ctx->ev0[i]));
         CK(cudaEventCreate(&ctx->ev1[i]));
-        CK(cudaEventCreateWithFlags(&ctx->evd[i], cudaEventDisableTiming));
     }
+    CK(cudaEventCreateWithFlags(&ctx->evd, cudaEventDisableTiming));
+    // in order before every launch, whose results are the next writes of h_out
+    CK(cudaMemcpyAsync(ctx->d_out, ctx->h_out, sizeof(LaunchOut) * kRing, cudaMemcpyHostToDevice, ctx->stream));
     std::string err;
     if (!driver_api(&err)) return NSAT_ECUDA;
     *out = c.release();
@@ -588,17 +644,12 @@ extern "C" void nsat_destroy(nsat_ctx* ctx) {
     for (int i = 0; i < kRing; i++) {
         if (ctx->ev0[i]) cudaEventDestroy(ctx->ev0[i]);
         if (ctx->ev1[i]) cudaEventDestroy(ctx->ev1[i]);
-        if (ctx->evd[i]) cudaEventDestroy(ctx->evd[i]);
     }
-    cudaFree(ctx->d_out);
-    cudaFreeHost(ctx->h_out);
-    cudaFreeHost(ctx->h_init);
+    if (ctx->evd) cudaEventDestroy(ctx->evd);
+    cudaFree(ctx->d_fixed);
+    cudaFreeHost(ctx->h_fixed);
     cudaFree(ctx->d_scratch);
     cudaFree(ctx->d_data);
-    cudaFree(ctx->d_join);
-    cudaFreeHost(ctx->h_join);
-    cudaFree(ctx->d_stop);
-    cudaFreeHost(ctx->h_stop);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     delete ctx;
@@ -702,18 +753,29 @@ extern "C" int nsat_sat_solve(nsat_ctx* ctx, nsat_circuit* c, const nsat_sat_opt
     if (int rc = set_device(ctx)) return rc;
     nsat_sat_opts o{};
     if (opts) o = *opts;
-    SatPlan plan;
-    std::string perr;
-    const std::vector<uint32_t> out0{0};
-    const LutNet& net = get_net(c, out0);
-    if (int rc = plan_sat(c->circ.n, o, effective_shape(ctx, c->tuned), &plan, &perr, (uint32_t)net.luts.size()))
-        return fail(ctx, rc, perr);
+    SatMemo& memo = c->sat_memo;
+    const Shape shape = effective_shape(ctx, c->tuned);
+    const u128 o_begin = ((u128)o.begin_hi << 64) | o.begin_lo, o_end = ((u128)o.end_hi << 64) | o.end_lo;
+    if (!memo.set || memo.chunk_bits != o.chunk_bits || memo.begin != o_begin || memo.end != o_end ||
+        !(memo.shape == shape)) {
+        memo = SatMemo();
+        std::string perr;
+        const std::vector<uint32_t> out0{0};
+        const LutNet& net = get_net(c, out0);
+        if (int rc = plan_sat(c->circ.n, o, shape, &memo.plan, &perr, (uint32_t)net.luts.size()))
+            return fail(ctx, rc, perr);
+        if (int rc = get_circuit_kernel(ctx, c, out0, memo.plan.kc, net, "nsat_sat", &memo.fn, &memo.mod)) return rc;
+        memo.chunk_bits = o.chunk_bits;
+        memo.begin = o_begin;
+        memo.end = o_end;
+        memo.shape = shape;
+        memo.set = true;
+    }
+    const SatPlan& plan = memo.plan;
     const KernelConfig& kc = plan.kc;
     const uint32_t d = plan.d, C = plan.C;
     const u128 bp = plan.bp, ep = plan.ep;
-    CUfunction fn;
-    std::shared_ptr<JitModule> mod;
-    if (int rc = get_circuit_kernel(ctx, c, out0, kc, net, "nsat_sat", &fn, &mod)) return rc;
+    const CUfunction fn = memo.fn;
     const uint64_t L0 = (uint64_t)(bp >> C);
     const uint64_t nl = (uint64_t)((ep - bp) >> C);
     const unsigned grid = 1u << kc.cb, threads = kc.threads();
@@ -725,14 +787,13 @@ extern "C" int nsat_sat_solve(nsat_ctx* ctx, nsat_circuit* c, const nsat_sat_opt
     uint32_t launches = 0;
     uint64_t launch_idx_buf[kRing];
     uint64_t chunk_of_slot[kRing];
-    LaunchOut* d_out = ctx->d_out;
     nsat_sat_share* share = o.find_all ? nullptr : o.share;
     int rc = run_ring(
         ctx, nl,
         [&](uint64_t k, int slot) {
             launch_idx_buf[slot] = L0 + (share ? chunk_of_slot[slot] : k);
-            LaunchOut* po = d_out + slot;
-            void* params[] = {&launch_idx_buf[slot], &po};
+            LaunchOut *po = ctx->d_out + slot, *ph = ctx->h_out + slot;
+            void* params[] = {&launch_idx_buf[slot], &po, &ph};
             return launch(ctx, fn, grid, threads, params);
         },
         [&](uint64_t k, const LaunchOut& r) {
@@ -802,15 +863,22 @@ int qsat_common(nsat_ctx* ctx, nsat_circuit* c, const std::vector<uint8_t>& quan
     if (int rc = set_device(ctx)) return rc;
     const bool data = data_words != nullptr;
     const uint32_t n = data ? n_items_bits : c->circ.n;
-    QsatPlan plan;
-    std::string perr;
-    LutNet empty;
-    const std::vector<uint32_t> out0{0};
-    const LutNet& net = data ? empty : get_net(c, out0);
     const Shape sh = data ? effective_shape(ctx, Shape()) : effective_shape(ctx, c->tuned_qsat);
-    if (int rc = plan_qsat(n, quants_in, data, chunk_bits, sh, prefix_bits, &plan, &perr,
-                           data ? 0u : (uint32_t)net.luts.size()))
-        return fail(ctx, rc, perr);
+    QsatMemo one;                       // a data reduction has no circuit to keep its plan on
+    QsatMemo& memo = data ? one : c->qsat_memo;
+    const bool planned = memo.set && memo.chunk_bits == chunk_bits && memo.prefix_bits == prefix_bits &&
+                         memo.quants == quants_in && memo.shape == sh;
+    const std::vector<uint32_t> out0{0};
+    LutNet empty;
+    const LutNet* net = planned || data ? &empty : &get_net(c, out0);
+    if (!planned) {
+        memo = QsatMemo();
+        std::string perr;
+        if (int rc = plan_qsat(n, quants_in, data, chunk_bits, sh, prefix_bits, &memo.plan, &perr,
+                               (uint32_t)net->luts.size()))
+            return fail(ctx, rc, perr);
+    }
+    const QsatPlan& plan = memo.plan;
     if (prefix_bits < 64 && (prefix >> prefix_bits) != 0) return fail(ctx, NSAT_EINVAL, "prefix wider than prefix_bits");
     const KernelConfig& kc = plan.kc;
     // a launch the fixed area cannot hold is refused before any kernel is compiled or loaded
@@ -825,11 +893,17 @@ int qsat_common(nsat_ctx* ctx, nsat_circuit* c, const std::vector<uint8_t>& quan
     const uint32_t d = plan.d, np = plan.np, m = plan.m, C = plan.C, s = plan.s, f = plan.fsub;
     const uint32_t A = plan.A - s;
     const uint64_t L0 = s ? (prefix << A) : 0;
-    CUfunction fn;
-    std::shared_ptr<JitModule> mod;
-    if (int rc = data ? get_kernel(ctx, kc, net, "nsat_qsat", &fn, &mod)
-                      : get_circuit_kernel(ctx, c, out0, kc, net, "nsat_qsat", &fn, &mod))
-        return rc;
+    if (!planned) {
+        if (int rc = data ? get_kernel(ctx, kc, *net, "nsat_qsat", &memo.fn, &memo.mod)
+                          : get_circuit_kernel(ctx, c, out0, kc, *net, "nsat_qsat", &memo.fn, &memo.mod))
+            return rc;
+        memo.chunk_bits = chunk_bits;
+        memo.prefix_bits = prefix_bits;
+        memo.quants = quants_in;
+        memo.shape = sh;
+        memo.set = true;
+    }
+    const CUfunction fn = memo.fn;
     if (!fixed_scratch) {
         if (int rc = ensure_scratch(ctx, (size_t)2 << kc.cb)) return rc;
     }
@@ -862,7 +936,6 @@ int qsat_common(nsat_ctx* ctx, nsat_circuit* c, const std::vector<uint8_t>& quan
     uint64_t nl = prefix_count > 1 ? prefix_count : (A == 64 ? ~0ull : (1ull << A));
     const unsigned grid = 1u << kc.cb, threads = kc.threads();
     uint64_t launch_idx_buf[kRing];
-    LaunchOut* d_out = ctx->d_out;
     unsigned char* scratch = fixed_scratch ? fixed_scratch : ctx->d_scratch;
     const uint32_t* dd = ctx->d_data;
     double dev_ms = 0;
@@ -871,8 +944,8 @@ int qsat_common(nsat_ctx* ctx, nsat_circuit* c, const std::vector<uint8_t>& quan
         ctx, nl,
         [&](uint64_t k, int slot) {
             launch_idx_buf[slot] = L0 + k;
-            LaunchOut* po = d_out + slot;
-            void* params[] = {&launch_idx_buf[slot], &po, &scratch, &dd};
+            LaunchOut *po = ctx->d_out + slot, *ph = ctx->h_out + slot;
+            void* params[] = {&launch_idx_buf[slot], &po, &ph, &scratch, &dd};
             return launch(ctx, fn, grid, threads, params);
         },
         [&](uint64_t k, const LaunchOut& r) {
@@ -970,7 +1043,7 @@ void nsat::ctx_stop_state(nsat_ctx* ctx, NsatStopState** dev, NsatStopState** ho
     *dev = ctx->d_stop;
     *host = ctx->h_stop;
 }
-cudaEvent_t nsat::ctx_stop_event(nsat_ctx* ctx) { return ctx->evd[0]; }
+cudaEvent_t nsat::ctx_stop_event(nsat_ctx* ctx) { return ctx->evd; }
 void nsat::ctx_timing_events(nsat_ctx* ctx, cudaEvent_t* begin, cudaEvent_t* end) {
     *begin = ctx->ev0[0];
     *end = ctx->ev1[0];
@@ -1044,25 +1117,19 @@ extern "C" int nsat_stop_table_build(nsat_ctx* ctx, nsat_circuit* c, const nsat_
             return fail(ctx, NSAT_ENOMEM, "table allocation failed");
         }
     }
-    std::vector<uint32_t> which;
-    for (uint32_t j = 0; j <= n; j++) which.push_back(j);
-    const LutNet& net = get_net(c, which);
-    CUfunction fn;
-    std::shared_ptr<JitModule> mod;
-    if (int rc = get_circuit_kernel(ctx, c, which, kc, net, "nsat_table", &fn, &mod)) return rc;
+    if (int rc = table_kernel(ctx, c, kc)) return rc;
+    const TableMemo& memo = c->table_memo[kc.fmt];
     uint64_t nwords = n >= 5 ? (t->N >> 5) : 1;
-    const unsigned threads = kc.threads();
+    const unsigned threads = memo.threads;
     uint64_t want = (nwords + threads - 1) / threads;
     unsigned grid = (unsigned)std::min<uint64_t>(want, (uint64_t)ctx->sm_count * 16);
-    LaunchOut* po = ctx->d_out;
+    LaunchOut *po = ctx->d_out, *ph = ctx->h_out;
     void* tb = t->buf[0];
     uint64_t w0 = 0;
-    void* params[] = {&nwords, &w0, &tb, &po};
-    CK(cudaMemcpyAsync(ctx->d_out, ctx->h_init, sizeof(LaunchOut), cudaMemcpyHostToDevice, ctx->stream));
+    void* params[] = {&nwords, &w0, &tb, &po, &ph};
     CK(cudaEventRecord(ctx->ev0[0], ctx->stream));
-    if (int rc = launch(ctx, fn, grid, threads, params)) return rc;
+    if (int rc = launch(ctx, memo.fn, grid, threads, params)) return rc;
     CK(cudaEventRecord(ctx->ev1[0], ctx->stream));
-    CK(cudaMemcpyAsync(ctx->h_out, ctx->d_out, sizeof(LaunchOut), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     float ms = 0;
     CK(cudaEventElapsedTime(&ms, ctx->ev0[0], ctx->ev1[0]));
@@ -1085,24 +1152,18 @@ int table_chunk(nsat_ctx* ctx, nsat_circuit* c, uint64_t first_state, uint64_t c
     if (n < 10 || (first_state & 1023) || (count & 1023) || count == 0 || (!wide && n > 31))
         return fail(ctx, NSAT_EINVAL, "table chunks are whole 1024-state tiles");
     kc.fmt = wide ? 1 : 0;
-    std::vector<uint32_t> which;
-    for (uint32_t j = 0; j <= n; j++) which.push_back(j);
-    const LutNet& net = get_net(c, which);
-    CUfunction fn;
-    std::shared_ptr<JitModule> mod;
-    if (int rc = get_circuit_kernel(ctx, c, which, kc, net, "nsat_table", &fn, &mod)) return rc;
+    if (int rc = table_kernel(ctx, c, kc)) return rc;
+    const TableMemo& memo = c->table_memo[kc.fmt];
     uint64_t nwords = count >> 5, w0 = first_state >> 5;
-    const unsigned threads = kc.threads();
+    const unsigned threads = memo.threads;
     const uint64_t want = (nwords + threads - 1) / threads;
     const unsigned grid = (unsigned)std::min<uint64_t>(want, (uint64_t)ctx->sm_count * 16);
-    LaunchOut* po = ctx->d_out;
+    LaunchOut *po = ctx->d_out, *ph = ctx->h_out;
     void* tb = dev_out;
-    void* params[] = {&nwords, &w0, &tb, &po};
-    CK(cudaMemcpyAsync(ctx->d_out, ctx->h_init, sizeof(LaunchOut), cudaMemcpyHostToDevice, ctx->stream));
+    void* params[] = {&nwords, &w0, &tb, &po, &ph};
     CK(cudaEventRecord(ctx->ev0[0], ctx->stream));
-    if (int rc = launch(ctx, fn, grid, threads, params)) return rc;
+    if (int rc = launch(ctx, memo.fn, grid, threads, params)) return rc;
     CK(cudaEventRecord(ctx->ev1[0], ctx->stream));
-    CK(cudaMemcpyAsync(ctx->h_out, ctx->d_out, sizeof(LaunchOut), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     if (ms) CK(cudaEventElapsedTime(ms, ctx->ev0[0], ctx->ev1[0]));
     if (any_stop) *any_stop = ctx->h_out[0].any != 0;
@@ -1124,12 +1185,19 @@ extern "C" int nsat_table_read(nsat_table* t, uint64_t first, uint64_t count, ui
     nsat_ctx* ctx = t->ctx;
     if (int rc = set_device(ctx)) return rc;
     const uint64_t mask = t->steps ? 0xffffffffull : ~0ull;
-    if (t->narrow) {
+    const uint64_t entry = t->narrow ? 4 : 8;
+    const char* src = (const char*)t->buf[t->cur] + first * entry;
+    if (count * entry <= kReadStage) {       // through pinned memory: 8 us instead of 17 for 16 KB
+        CK(cudaMemcpyAsync(ctx->h_read, src, count * entry, cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        for (uint64_t i = 0; i < count; i++)
+            out[i] = t->narrow ? ((const uint32_t*)ctx->h_read)[i] : ((const uint64_t*)ctx->h_read)[i] & mask;
+    } else if (t->narrow) {
         std::vector<uint32_t> tmp(count);
-        CK(cudaMemcpy(tmp.data(), (uint32_t*)t->buf[t->cur] + first, count * 4, cudaMemcpyDeviceToHost));
+        CK(cudaMemcpy(tmp.data(), src, count * 4, cudaMemcpyDeviceToHost));
         for (uint64_t i = 0; i < count; i++) out[i] = tmp[i];
     } else {
-        CK(cudaMemcpy(out, (uint64_t*)t->buf[t->cur] + first, count * 8, cudaMemcpyDeviceToHost));
+        CK(cudaMemcpy(out, src, count * 8, cudaMemcpyDeviceToHost));
         for (uint64_t i = 0; i < count; i++) out[i] &= mask;
     }
     return NSAT_OK;
