@@ -170,7 +170,8 @@ typedef struct {
     uint64_t solution_lo, solution_hi;  /* bit k = input k of the first block */
     uint32_t launches;
     uint32_t chunk_bits;       /* log2 assignments per launch actually used */
-    uint64_t scanned;          /* assignments evaluated (launches x 2^chunk_bits) */
+    uint64_t scanned;          /* assignments of the launches run (launches x 2^chunk_bits);
+                                  what is decided already is not evaluated */
     double device_ms;
     double wall_ms;
 } nsat_qsat_result;
@@ -183,7 +184,7 @@ int nsat_qsat_solve(nsat_ctx* ctx, nsat_circuit* c, const uint8_t* quants,
  * budget, where cudaMalloc/cudaFree would synchronize the device or break the
  * budget mid-request.  No counterpart in the reference (its OpenCL reducer
  * allocates its buffers per solver, qsat.rs:1046-1064).
- * The last-CTA scratch comes from a static device array of
+ * The chunk tree's scratch comes from a static device array of
  * NSAT_NOALLOC_SCRATCH_BYTES (64 KiB) inside libnsat.so instead of the
  * context's lazily allocated buffer; every GPU that loads the library holds it
  * until exit.  A solve whose launches need more scratch (2 << CB bytes, CB =

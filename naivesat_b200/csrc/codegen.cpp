@@ -91,6 +91,12 @@ std::string generate_source(const KernelConfig& kc, const LutNet& net) {
     s << "constexpr int NSAT_Q0ALL = " << (kc.q0all ? 1 : 0) << ";\n";
     s << "constexpr u64 NSAT_ALLBITS = " << kc.allbits << "ull;\n";
 
+    // few iterations of a large evaluation are not unrolled: four copies of 665
+    // LUTs doubled the compile time and gained nothing; the loop of a 38-LUT
+    // adder is (244 us against 351 us)
+    s << "#define NSAT_ONE " << (kc.cb <= kResidentBits ? 1 : 0) << "\n";
+    s << "#define NSAT_UNROLL " << (net.luts.size() > 64 ? "_Pragma(\"unroll 1\")" : "") << "\n";
+
     // enumeration: which circuit input each bit drives
     const uint32_t it_lo = 10, wb_lo = 10 + kc.it, cb_lo = wb_lo + kc.wb, c_lo = cb_lo + kc.cb;
     std::ostringstream fixed, iter, word;

@@ -10,6 +10,9 @@ namespace nsat {
 
 enum class Mode { SAT = 1, QSAT = 2, TABLE = 3 };
 
+// A launch of up to 2^7 CTAs has them all resident (148 SMs).
+constexpr uint32_t kResidentBits = 7;
+
 struct KernelConfig {
     Mode mode = Mode::SAT;
     uint32_t nin = 0;          // circuit inputs, padding included

@@ -3,7 +3,9 @@
 // The host generator (codegen.cpp) prepends a prelude that defines:
 //   constexpr ints NSAT_NIN, NSAT_NOUT, NSAT_NB (enumeration bits), NSAT_NT
 //   (threads per CTA), NSAT_IT / NSAT_WB / NSAT_CB (log2 of iterations per
-//   warp, warps per CTA and CTAs per launch), NSAT_BOUNDS (the kernels'
+//   warp, warps per CTA and CTAs per launch; QSAT: chunks per launch),
+//   NSAT_ONE (QSAT: a CTA per chunk), NSAT_UNROLL (a pragma for the loop over
+//   iterations), NSAT_BOUNDS (the kernels'
 //   __launch_bounds__), NSAT_C (= 10+IT+WB+CB, log2 of
 //   assignments per launch), NSAT_M (QSAT unit level), NSAT_Q0ALL,
 //   NSAT_ALLBITS (bit j = quantifier of enumeration bit j is All),
@@ -34,31 +36,35 @@ struct LaunchOut {
     u32 tree;      // QSAT: tree value of the launch when no unit boundary is inside it
     u32 ticket;    // CTAs finished
     u32 any;       // table build: some STOP output seen
-    u32 values;    // QSAT: CTAs that have written their value (last-CTA tail)
+    u32 values;    // QSAT: chunks claimed beyond the first of each CTA
 };
 
-// Ends a CTA, all threads together, after its last update of *out.  The last
-// CTA of the launch copies the result to pinned host memory and puts the slot
-// back as the next launch expects it: a solve is a kernel between two events,
-// where a copy that set the slot and one that read it back took 6 us of a
-// small solve.
+// The last CTA of a launch: copies the result to pinned host memory and puts
+// the slot back as the next launch expects it.  A solve is a kernel between
+// two events; a copy that set the slot and one that read it back took 6 us of
+// a small solve.
+__device__ __forceinline__ void nsat_publish(LaunchOut* out, LaunchOut* host) {
+    volatile LaunchOut* o = out;
+    volatile LaunchOut* h = host;
+    h->min_idx = o->min_idx;
+    h->count = o->count;
+    h->tree = o->tree;
+    h->any = o->any;
+    o->min_idx = ~0ull;
+    o->count = 0ull;
+    o->tree = 0u;
+    o->ticket = 0u;
+    o->any = 0u;
+}
+
+// Ends a CTA, all threads together, after its last update of *out.
 __device__ __forceinline__ void nsat_finish(LaunchOut* out, LaunchOut* host) {
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
         if (atomicAdd(&out->ticket, 1u) == gridDim.x - 1u) {
             __threadfence();
-            volatile LaunchOut* o = out;
-            volatile LaunchOut* h = host;
-            h->min_idx = o->min_idx;
-            h->count = o->count;
-            h->tree = o->tree;
-            h->any = o->any;
-            o->min_idx = ~0ull;
-            o->count = 0ull;
-            o->tree = 0u;
-            o->ticket = 0u;
-            o->any = 0u;
+            nsat_publish(out, host);
         }
     }
 }
@@ -145,14 +151,6 @@ __device__ __forceinline__ u32 tree_up(u32 y) {
     return y;
 }
 
-__device__ __forceinline__ u32 tree_up_rt(u32 y, int lvl, int cnt) {
-    for (int j = 0; j < cnt; j++) {
-        if ((NSAT_ALLBITS >> (lvl + j)) & 1ull) y &= (y >> (1 << j));
-        else y |= (y >> (1 << j));
-    }
-    return y;
-}
-
 // bits at multiples of 2^k inside a 32-bit node vector
 __device__ __forceinline__ constexpr u32 unit_mask(int k) {
     return k == 0 ? 0xffffffffu : k == 1 ? 0x55555555u : k == 2 ? 0x11111111u
@@ -172,9 +170,105 @@ __device__ constexpr int low_run(u64 allbits) {
     return k;
 }
 
+// The tree above the chunks.  A chunk is the range of items one CTA evaluates
+// at a time (levels below LC); 2^CB chunks make the launch.  The levels from
+// LC up to the units (or the whole launch) are cut into blocks of one
+// quantifier, at most 8 levels each, and every block node counts its children:
+// a child with the deciding value (0 under All, 1 under Exists), or the last
+// of its children, resolves the node, and the node's value goes on to the
+// block above.  A chunk below a resolved node cannot change anything and is
+// not evaluated, nor is one whose units lie above a decisive unit.  A node is
+// 16 bits: 0x8000 once resolved, the count of its undecided children below.
+struct QBlocks {
+    int n;
+    int lo[64], hi[64];    // levels [lo, hi) of block k
+    u32 off[64];           // its nodes' first index
+    u32 nodes;
+};
+constexpr int NSAT_LC = 10 + NSAT_IT + NSAT_WB;
+constexpr int NSAT_TOP = NSAT_M < NSAT_C ? NSAT_M : NSAT_C;
+__device__ constexpr QBlocks make_blocks() {
+    QBlocks b = {};
+    int l = NSAT_LC;
+    while (l < NSAT_TOP) {
+        int h = l + 1;
+        while (h < NSAT_TOP && h - l < 8 && (((NSAT_ALLBITS >> l) ^ (NSAT_ALLBITS >> h)) & 1ull) == 0ull) h++;
+        b.lo[b.n] = l;
+        b.hi[b.n] = h;
+        b.off[b.n] = b.nodes;
+        b.nodes += 1u << (NSAT_C - h);
+        b.n++;
+        l = h;
+    }
+    return b;
+}
+
+// Order of the chunks: 2^UB units side by side, the chunks of each in order.
+// One deciding child ends a node's other children, so the chunks in flight
+// are spread over units; within a unit depth first decides most per chunk.
+// 30 inputs, 1500 gates, alternating blocks of up to six, three formulas: 171,
+// 186 and 272 us with up to 2^7 units side by side, 242, 319 and 268 with 2^4,
+// 643, 457 and 812 with one after another; 1270 us when every chunk is
+// evaluated.
+constexpr int NSAT_UNITS = NSAT_M >= NSAT_LC && NSAT_M < NSAT_C ? NSAT_C - NSAT_M : 0;   // unit bits of a chunk index
+constexpr int NSAT_UB = NSAT_UNITS < 7 ? NSAT_UNITS : 7;
+__device__ __forceinline__ u32 chunk_of(u32 t) {
+    if constexpr (NSAT_UB == 0) {
+        return t;
+    } else {
+        constexpr int IN = NSAT_CB - NSAT_UNITS;           // bits below the units
+        const u32 unit = t & ((1u << NSAT_UB) - 1u);
+        const u32 in = (t >> NSAT_UB) & ((1u << IN) - 1u);
+        const u32 up = t >> (NSAT_UB + IN);
+        return (((up << NSAT_UB) | unit) << IN) | in;
+    }
+}
+
+// Whether chunk c has nothing left to decide.
+__device__ __forceinline__ bool chunk_decided(u32 c, const u32* nodes, const LaunchOut* out) {
+    constexpr QBlocks B = make_blocks();
+    bool done = false;
+#pragma unroll
+    for (int k = 0; k < B.n; k++) {
+        const u32 i = B.off[k] + (c >> (B.hi[k] - NSAT_LC));
+        const u32 w = *(volatile const u32*)(nodes + (i >> 1));
+        done |= ((w >> ((i & 1u) << 4)) & 0x8000u) != 0u;
+    }
+    if constexpr (NSAT_M < NSAT_C) {
+        const u64 lowest = *(volatile const u64*)&out->min_idx;
+        if constexpr (NSAT_M >= NSAT_LC) done |= lowest <= (u64)(c >> (NSAT_M - NSAT_LC));
+        else done |= lowest < ((u64)c << (NSAT_LC - NSAT_M));
+    }
+    return done;
+}
+
+// One thread: chunk c has value v.
+__device__ __forceinline__ void chunk_value(u32 c, u32 v, u32* nodes, LaunchOut* out) {
+    constexpr QBlocks B = make_blocks();
+#pragma unroll
+    for (int k = 0; k < B.n; k++) {
+        const u32 i = B.off[k] + (c >> (B.hi[k] - NSAT_LC));
+        const u32 sh = (i & 1u) << 4;
+        u32* w = nodes + (i >> 1);
+        if (v != (u32)((NSAT_ALLBITS >> B.lo[k]) & 1ull)) {                    // the deciding value
+            if ((atomicOr(w, 0x8000u << sh) >> sh) & 0x8000u) return;
+        } else {
+            const u32 old = (atomicAdd(w, 1u << sh) >> sh) & 0xffffu;
+            if (old != (1u << (B.hi[k] - B.lo[k])) - 1u) return;               // not the last child, or resolved
+            if ((atomicOr(w, 0x8000u << sh) >> sh) & 0x8000u) return;
+        }
+    }
+    if constexpr (NSAT_M >= NSAT_C) out->tree = v;
+    else if (v == (NSAT_Q0ALL ? 0u : 1u)) atomicMin(&out->min_idx, (u64)(c >> (NSAT_M - NSAT_LC)));
+}
+
+// Resident CTAs take chunks until none is left: chunk blockIdx.x first, then
+// from the launch's counter (out->values), one at a time while they need
+// evaluation, up to 32 at once while they turn out decided.  NSAT_ONE: the
+// launch has a CTA for every chunk (the claims' code would cost a small
+// circuit a third of its compile time).
 extern "C" __global__ void NSAT_BOUNDS
-nsat_qsat(u64 launch, LaunchOut* out, LaunchOut* host, unsigned char* __restrict__ scratch,
-          const u32* __restrict__ data) {
+nsat_qsat(u64 launch, LaunchOut* out, LaunchOut* host, u32* nodes, const u32* __restrict__ data) {
     constexpr int M = NSAT_M;
     // Folding.  When levels 0..9 (the word and the warp tile) and the lowest
     // FOLD iteration levels all carry level 0's quantifier and lie below the
@@ -194,170 +288,175 @@ nsat_qsat(u64 launch, LaunchOut* out, LaunchOut* host, unsigned char* __restrict
     constexpr int G2 = IT2 - G1;
     const u32 lane = threadIdx.x & 31u;
     const u32 warp = threadIdx.x >> 5;
-    const u32 cta = blockIdx.x;
-    // launch-relative index of the first item of this warp's range
-    const u64 warp_base = (((u64)cta << NSAT_WB) | warp) << (10 + NSAT_IT);
-    u32 x[NSAT_NIN];
+    __shared__ u32 s_last, s_res[32];
+    u32 cta = chunk_of(blockIdx.x);             // not checked: nothing is decided yet
+#if !NSAT_ONE
+    __shared__ u32 s_cta, s_base, s_mask, s_step;      // warp 0's claim: chunks s_base + the bits of s_mask
+    if (threadIdx.x == 0) { s_base = blockIdx.x; s_mask = 0u; s_step = 1u; }
+    u32 ahead = 0u;        // warp 0, lane 0: the next claim, made while this chunk is evaluated
+    bool claimed = warp == 0;
+    if (threadIdx.x == 0) ahead = atomicAdd(&out->values, 1u);
+#endif
+    for (;;) {
+        // launch-relative index of the first item of this warp's range
+        const u64 warp_base = (((u64)cta << NSAT_WB) | warp) << (10 + NSAT_IT);
+        u32 x[NSAT_NIN];
 #if !NSAT_DATA
-    nsat_inputs_fixed(x, lane, warp, cta, launch);
+        nsat_inputs_fixed(x, lane, warp, cta, launch);
 #endif
-    u64 cand = ~0ull;      // lowest decisive unit seen by this thread (launch-relative)
-    u32 acc1 = 0, acc2 = 0;
-    u32 yacc = LOW_ALL ? 0xffffffffu : 0u;
-    for (u32 it = 0; it < (1u << NSAT_IT); it++) {
+        u64 cand = ~0ull;      // lowest decisive unit seen by this thread (launch-relative)
+        u32 acc1 = 0, acc2 = 0;
+        u32 yacc = LOW_ALL ? 0xffffffffu : 0u;
+        NSAT_UNROLL
+        for (u32 it = 0; it < (1u << NSAT_IT); it++) {
 #if NSAT_DATA
-        const u64 gw = ((u64)launch << (NSAT_C - 5)) + ((warp_base + ((u64)it << 10)) >> 5) + lane;
-        u32 y = data[gw];
+            const u64 gw = ((u64)launch << (NSAT_C - 5)) + ((warp_base + ((u64)it << 10)) >> 5) + lane;
+            u32 y = data[gw];
 #else
-        nsat_inputs_iter(x, it);
-        u32 y = nsat_eval1(x);
+            nsat_inputs_iter(x, it);
+            u32 y = nsat_eval1(x);
 #endif
-        u32 b, git;   // node value at level L0 (bit 0) and its index among the warp's L0 nodes
-        if constexpr (FOLDED) {
-            yacc = LOW_ALL ? (yacc & y) : (yacc | y);
-            if (((it + 1u) & ((1u << FOLD) - 1u)) != 0u) continue;
-            const bool v = LOW_ALL ? (yacc == 0xffffffffu) : (yacc != 0u);
-            yacc = LOW_ALL ? 0xffffffffu : 0u;
-            b = LOW_ALL ? (u32)__all_sync(0xffffffffu, v) : (u32)__any_sync(0xffffffffu, v);
-            git = it >> FOLD;
-        } else {
-            const u64 tile_base = warp_base + ((u64)it << 10);   // first item of this warp tile
-            // stage 0: the 32 lanes of the word (levels 0..4)
-            if constexpr (M < 5) {
-                y = tree_up<0, M>(y);
-                const u32 d = decisive(y, M, 32);
-                if (d != 0u && cand == ~0ull)
-                    cand = ((tile_base + ((u64)lane << 5)) >> M) + (u64)((__ffs(d) - 1) >> M);
-                continue;
+            u32 b, git;   // node value at level L0 (bit 0) and its index among the warp's L0 nodes
+            if constexpr (FOLDED) {
+                yacc = LOW_ALL ? (yacc & y) : (yacc | y);
+                if (((it + 1u) & ((1u << FOLD) - 1u)) != 0u) continue;
+                const bool v = LOW_ALL ? (yacc == 0xffffffffu) : (yacc != 0u);
+                yacc = LOW_ALL ? 0xffffffffu : 0u;
+                b = LOW_ALL ? (u32)__all_sync(0xffffffffu, v) : (u32)__any_sync(0xffffffffu, v);
+                git = it >> FOLD;
             } else {
-                y = tree_up<0, 5>(y);
-            }
-            // stage 1: the 32 words of the warp tile (levels 5..9)
-            b = __ballot_sync(0xffffffffu, y & 1u);
-            if constexpr (M >= 5 && M < 10) {
-                b = tree_up<5, M - 5>(b);
-                const u32 d = decisive(b, M - 5, 32);
-                if (d != 0u && cand == ~0ull)
-                    cand = (tile_base >> M) + (u64)((__ffs(d) - 1) >> (M - 5));
-                continue;
-            } else {
-                b = tree_up<5, 5>(b);
-            }
-            git = it;
-        }
-        // stage 2: the warp's L0 nodes (levels L0..10+IT-1), 2^G1 at a time
-        if constexpr (M >= L0 && IT2 > 0) {
-            const u32 pos = git & ((1u << G1) - 1u);
-            acc1 |= (b & 1u) << pos;
-            if (pos == (1u << G1) - 1u) {
-                const u64 grp_base = warp_base + ((u64)(git - pos) << L0);
-                if constexpr (M < L0 + G1) {
-                    const u32 y1 = tree_up<L0, M - L0>(acc1);
-                    const u32 d = decisive(y1, M - L0, 1 << G1);
+                const u64 tile_base = warp_base + ((u64)it << 10);   // first item of this warp tile
+                // stage 0: the 32 lanes of the word (levels 0..4)
+                if constexpr (M < 5) {
+                    y = tree_up<0, M>(y);
+                    const u32 d = decisive(y, M, 32);
                     if (d != 0u && cand == ~0ull)
-                        cand = (grp_base >> M) + (u64)((__ffs(d) - 1) >> (M - L0));
+                        cand = ((tile_base + ((u64)lane << 5)) >> M) + (u64)((__ffs(d) - 1) >> M);
+                    continue;
                 } else {
-                    const u32 y1 = tree_up<L0, G1>(acc1);
-                    acc2 |= (y1 & 1u) << (git >> G1);
+                    y = tree_up<0, 5>(y);
                 }
-                acc1 = 0;
-            }
-        } else if constexpr (M >= L0) {
-            acc2 = b & 1u;   // IT2 == 0: one L0 node is the warp's whole range
-        }
-    }
-    // stage 2b: groups of L0 nodes (levels L0+G1 .. 10+IT-1)
-    u32 wres = 0;
-    if constexpr (M >= L0 + G1 && IT2 > 0) {
-        if constexpr (M < L0 + IT2) {
-            const u32 y2 = tree_up<L0 + G1, M - L0 - G1>(acc2);
-            const u32 d = decisive(y2, M - L0 - G1, 1 << G2);
-            if (d != 0u && cand == ~0ull)
-                cand = (warp_base >> M) + (u64)((__ffs(d) - 1) >> (M - L0 - G1));
-        } else {
-            wres = tree_up<L0 + G1, G2>(acc2) & 1u;
-        }
-    } else if constexpr (M >= L0 && IT2 == 0) {
-        wres = acc2 & 1u;
-    }
-    // per-warp lowest candidate, one atomic per warp
-    cand = warp_min_u64(cand);
-    if (lane == 0 && cand != ~0ull) atomicMin(&out->min_idx, cand);
-    // stage 3: warps of the CTA (levels 10+IT .. 10+IT+WB-1)
-    if constexpr (M >= 10 + NSAT_IT) {
-        __shared__ u32 s_res[32];
-        __shared__ u32 s_last;
-        if (lane == 0) s_res[warp] = wres;
-        __syncthreads();
-        u32 cres = 0;
-        if (warp == 0) {
-            u32 mbits = __ballot_sync(0xffffffffu, lane < (1u << NSAT_WB) ? s_res[lane] : 0u);
-            const u64 cta_base = (u64)cta << (10 + NSAT_IT + NSAT_WB);
-            if constexpr (M < 10 + NSAT_IT + NSAT_WB) {
-                const u32 y3 = tree_up<10 + NSAT_IT, M - 10 - NSAT_IT>(mbits);
-                const u32 d = decisive(y3, M - 10 - NSAT_IT, 1 << NSAT_WB);
-                if (lane == 0 && d != 0u)
-                    atomicMin(&out->min_idx, (cta_base >> M) + (u64)((__ffs(d) - 1) >> (M - 10 - NSAT_IT)));
-            } else {
-                cres = tree_up<10 + NSAT_IT, NSAT_WB>(mbits) & 1u;
-            }
-        }
-        // stage 4: CTAs of the launch (levels 10+IT+WB .. C-1), last-CTA tail
-        if constexpr (M >= 10 + NSAT_IT + NSAT_WB) {
-            if constexpr (NSAT_CB == 0) {
-                if (threadIdx.x == 0) out->tree = cres;
-            } else {
-                if (threadIdx.x == 0) {
-                    scratch[cta] = (unsigned char)cres;
-                    __threadfence();
-                    const u32 t = atomicAdd(&out->values, 1u);
-                    s_last = (t == (1u << NSAT_CB) - 1u) ? 1u : 0u;
+                // stage 1: the 32 words of the warp tile (levels 5..9)
+                b = __ballot_sync(0xffffffffu, y & 1u);
+                if constexpr (M >= 5 && M < 10) {
+                    b = tree_up<5, M - 5>(b);
+                    const u32 d = decisive(b, M - 5, 32);
+                    if (d != 0u && cand == ~0ull)
+                        cand = (tile_base >> M) + (u64)((__ffs(d) - 1) >> (M - 5));
+                    continue;
+                } else {
+                    b = tree_up<5, 5>(b);
                 }
-                __syncthreads();
-                if (s_last) {
-                    __threadfence();
-                    int lvl = 10 + NSAT_IT + NSAT_WB;
-                    int nodes = 1 << NSAT_CB;
-                    unsigned char* src = scratch;
-                    unsigned char* dst = scratch + (1 << NSAT_CB);
-                    const int nw = NSAT_NT / 32;
-                    bool done = false;
-                    while (!done) {
-                        const int k = nodes >= 32 ? 5 : (31 - __clz(nodes));   // log2(nodes) if < 32
-                        const int groups = nodes >> k;
-                        const bool units_here = M < lvl + k;
-                        for (int gi = (int)warp; gi < groups; gi += nw) {
-                            const int node = (gi << k) + (int)lane;
-                            u32 v = (lane < (1u << k)) ? (u32)__ldcg(src + node) : 0u;
-                            u32 mb = __ballot_sync(0xffffffffu, v & 1u);
-                            if (units_here) {
-                                const int ku = M - lvl;
-                                mb = tree_up_rt(mb, lvl, ku);
-                                const u32 d = decisive(mb, ku, 1 << k);
-                                if (lane == 0 && d != 0u)
-                                    atomicMin(&out->min_idx,
-                                              ((((u64)gi << k) << lvl) >> M) + (u64)((__ffs(d) - 1) >> ku));
-                            } else {
-                                mb = tree_up_rt(mb, lvl, k);
-                                if (lane == 0) dst[gi] = (unsigned char)(mb & 1u);
-                            }
-                        }
-                        __syncthreads();
-                        if (units_here) { done = true; break; }
-                        lvl += k;
-                        nodes = groups;
-                        unsigned char* tmp = src; src = dst; dst = tmp;
-                        if (nodes == 1) {
-                            if (threadIdx.x == 0) out->tree = (u32)__ldcg(src);
-                            done = true;
-                        }
+                git = it;
+            }
+            // stage 2: the warp's L0 nodes (levels L0..10+IT-1), 2^G1 at a time
+            if constexpr (M >= L0 && IT2 > 0) {
+                const u32 pos = git & ((1u << G1) - 1u);
+                acc1 |= (b & 1u) << pos;
+                if (pos == (1u << G1) - 1u) {
+                    const u64 grp_base = warp_base + ((u64)(git - pos) << L0);
+                    if constexpr (M < L0 + G1) {
+                        const u32 y1 = tree_up<L0, M - L0>(acc1);
+                        const u32 d = decisive(y1, M - L0, 1 << G1);
+                        if (d != 0u && cand == ~0ull)
+                            cand = (grp_base >> M) + (u64)((__ffs(d) - 1) >> (M - L0));
+                    } else {
+                        const u32 y1 = tree_up<L0, G1>(acc1);
+                        acc2 |= (y1 & 1u) << (git >> G1);
                     }
-                    if (threadIdx.x == 0) out->values = 0u;
+                    acc1 = 0;
+                }
+            } else if constexpr (M >= L0) {
+                acc2 = b & 1u;   // IT2 == 0: one L0 node is the warp's whole range
+            }
+        }
+        // stage 2b: groups of L0 nodes (levels L0+G1 .. 10+IT-1)
+        u32 wres = 0;
+        if constexpr (M >= L0 + G1 && IT2 > 0) {
+            if constexpr (M < L0 + IT2) {
+                const u32 y2 = tree_up<L0 + G1, M - L0 - G1>(acc2);
+                const u32 d = decisive(y2, M - L0 - G1, 1 << G2);
+                if (d != 0u && cand == ~0ull)
+                    cand = (warp_base >> M) + (u64)((__ffs(d) - 1) >> (M - L0 - G1));
+            } else {
+                wres = tree_up<L0 + G1, G2>(acc2) & 1u;
+            }
+        } else if constexpr (M >= L0 && IT2 == 0) {
+            wres = acc2 & 1u;
+        }
+        // per-warp lowest candidate, one atomic per warp
+        cand = warp_min_u64(cand);
+        if (lane == 0 && cand != ~0ull) atomicMin(&out->min_idx, cand);
+        // stage 3: warps of the CTA (levels 10+IT .. 10+IT+WB-1); its value goes to
+        // the tree above the chunks
+        if constexpr (M >= 10 + NSAT_IT) {
+            if (lane == 0) s_res[warp] = wres;
+            __syncthreads();
+            if (warp == 0) {
+                const u32 mbits = __ballot_sync(0xffffffffu, lane < (1u << NSAT_WB) ? s_res[lane] : 0u);
+                if constexpr (M < NSAT_LC) {
+                    const u64 cta_base = (u64)cta << NSAT_LC;
+                    const u32 y3 = tree_up<10 + NSAT_IT, M - 10 - NSAT_IT>(mbits);
+                    const u32 d = decisive(y3, M - 10 - NSAT_IT, 1 << NSAT_WB);
+                    if (lane == 0 && d != 0u)
+                        atomicMin(&out->min_idx, (cta_base >> M) + (u64)((__ffs(d) - 1) >> (M - 10 - NSAT_IT)));
+                } else {
+                    const u32 cres = tree_up<10 + NSAT_IT, NSAT_WB>(mbits) & 1u;
+                    if (lane == 0) chunk_value(cta, cres, nodes, out);
                 }
             }
         }
+        __syncthreads();       // s_cta and s_res are written again
+#if NSAT_ONE
+        break;
+#else
+        if (warp == 0) {
+            u32 base = s_base, mask = s_mask, step = s_step, c = ~0u;
+            for (;;) {
+                const u32 t = base + lane;
+                c = chunk_of(t);
+                mask = __ballot_sync(0xffffffffu, ((mask >> lane) & 1u) && t < (1u << NSAT_CB) && !chunk_decided(c, nodes, out));
+                if (mask) {
+                    const int f = __ffs(mask) - 1;
+                    c = __shfl_sync(0xffffffffu, c, f);
+                    mask &= mask - 1u;
+                    step = 1u;
+                    break;
+                }
+                c = ~0u;
+                if (base >= (1u << NSAT_CB)) break;
+                const u32 take = claimed ? 1u : step;
+                if (lane == 0) base = gridDim.x + (claimed ? ahead : atomicAdd(&out->values, take));
+                claimed = false;
+                base = __shfl_sync(0xffffffffu, base, 0);
+                mask = take >= 32u ? ~0u : (1u << take) - 1u;
+                step = step < 32u ? step * 2u : 32u;
+            }
+            if (c != ~0u && mask == 0u && !claimed) {
+                if (lane == 0) ahead = atomicAdd(&out->values, 1u);
+                claimed = true;
+            }
+            if (lane == 0) { s_base = base; s_mask = mask; s_step = step; s_cta = c; }
+        }
+        __syncthreads();
+        cta = s_cta;
+        if (cta == ~0u) break;
+#endif
     }
-    nsat_finish(out, host);
+    // the last CTA puts the nodes and the counter back to zero
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(&out->ticket, 1u) == gridDim.x - 1u;
+    }
+    __syncthreads();
+    if (s_last) {
+        __threadfence();
+        for (u32 i = threadIdx.x; i < (make_blocks().nodes + 1u) / 2u; i += NSAT_NT) nodes[i] = 0u;
+        if (threadIdx.x == 0) {
+            out->values = 0u;
+            nsat_publish(out, host);
+        }
+    }
 }
 #endif
 

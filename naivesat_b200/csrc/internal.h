@@ -46,7 +46,8 @@ void ctx_trim(nsat_ctx* ctx);
 // Circuit from the C ABI's flat description (not validated).
 Circuit circuit_from_desc(const nsat_circuit_desc* d);
 
-// nsat_qsat_solve with the last-CTA scratch area supplied by the caller
+// nsat_qsat_solve with the scratch area (the chunk tree's nodes, zero before
+// the first call; every launch leaves it zero) supplied by the caller
 // instead of the context's cudaMalloc'd buffer; fails with NSAT_EUNSUPPORTED
 // when a launch would need more than scratch_bytes.
 int qsat_solve_with_scratch(nsat_ctx* ctx, nsat_circuit* c, const uint8_t* quants,

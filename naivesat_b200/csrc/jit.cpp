@@ -126,6 +126,7 @@ const DriverApi* driver_api(std::string* err) {
                   resolve("cuModuleUnload", &g_api.ModuleUnload) &&
                   resolve("cuLaunchKernel", &g_api.LaunchKernel) &&
                   resolve("cuFuncGetAttribute", &g_api.FuncGetAttribute) &&
+                  resolve("cuOccupancyMaxActiveBlocksPerMultiprocessor", &g_api.OccupancyMaxActiveBlocks) &&
                   resolve("cuGetErrorString", &g_api.GetErrorString);
         g_api.ok = ok;
     }

@@ -6,7 +6,7 @@
 // per-tenant budget), or next to latency-critical streams.  cudaMalloc and
 // cudaFree can synchronize the whole device and stall those streams, and a
 // first-touch allocation can fail or breach the budget in the middle of a
-// request.  nsat_qsat_solve allocates its last-CTA scratch lazily
+// request.  nsat_qsat_solve allocates its chunk tree's nodes lazily
 // (cudaMalloc on first use and whenever a launch needs more); this variant
 // uses the fixed area below instead.
 #include <cuda_runtime.h>
@@ -20,8 +20,8 @@
 
 namespace {
 
-// Scratch of the QSAT last-CTA tail: one byte per CTA plus a ping-pong half
-// (2 << CB bytes per launch).  64 KiB covers launches of up to 2^15 CTAs.
+// Nodes of the QSAT kernel's chunk tree: 16 bits each, fewer nodes than
+// chunks (at most 2 << CB bytes per launch).  64 KiB covers 2^15 chunks.
 // Every GPU that loads libnsat.so holds this array until the process exits.
 constexpr size_t kScratchBytes = NSAT_NOALLOC_SCRATCH_BYTES;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
@@ -58,7 +58,7 @@ extern "C" int nsat_qsat_solve_noalloc(nsat_ctx* ctx, nsat_circuit* c, const uin
     unsigned char* scratch = nullptr;
     int rc = scratch_on(nsat::ctx_device(ctx), &scratch);
     if (rc != NSAT_OK) return rc;
-    // Nothing in the area has to start at zero: every launch writes each
-    // byte it later reads (one per CTA, then the tail's ping-pong half).
+    // The area is zero when the module is loaded, and the last CTA of every
+    // launch puts it back to zero.
     return nsat::qsat_solve_with_scratch(ctx, c, quants, opts, res, scratch, kScratchBytes);
 }

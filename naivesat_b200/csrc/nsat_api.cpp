@@ -60,7 +60,7 @@ struct nsat_ctx {
     int sm_count = 0;
     std::string last_err;
     char* d_fixed = nullptr;          // the device allocation behind d_out, d_join and d_stop
-    char* h_fixed = nullptr;          // the pinned one behind h_out, h_join, h_stop and h_read
+    char* h_fixed = nullptr;          // the pinned one behind h_out, h_join and h_stop
     LaunchOut* d_out = nullptr;       // kRing slots, put back to their first state by each launch
     LaunchOut* h_out = nullptr;       // pinned: a launch's last CTA writes its result here
     cudaEvent_t ev0[kRing]{}, ev1[kRing]{}, evd = nullptr;
@@ -137,6 +137,7 @@ struct QsatMemo {
     std::vector<uint8_t> quants;
     Shape shape;
     QsatPlan plan;
+    unsigned grid = 0;           // resident CTAs, at most one per chunk
     CUfunction fn = nullptr;
     std::shared_ptr<JitModule> mod;
 };
@@ -269,6 +270,21 @@ void choose_shape(uint32_t C, uint32_t block_threads, KernelConfig* kc, uint32_t
     kc->wb = wb; kc->it = it; kc->cb = cb; kc->c = C;
 }
 
+// QSAT chunks (what a CTA evaluates at a time): the smaller, the more of the
+// formula is decided before it is evaluated, but a chunk costs 1-2 us of
+// claim, check and report, so one has at least 2^13 warp LUTs.  Measured at
+// 2^12, 2^13 and 2^14, device time: a 32-input adder with a key (55 LUTs, most
+// of it decided early) 41, 48 and 68 us, the plain adder (38 LUTs, nothing
+// decided early) 259, 244 and 257 us.  At most 2^15 chunks, whose nodes fit
+// the allocation-free solver's area.
+void choose_chunks(uint32_t lop3, KernelConfig* kc) {
+    if (!lop3) return;
+    int log2_lop3 = 0;
+    while ((lop3 >> (log2_lop3 + 1)) != 0) log2_lop3++;
+    const uint32_t it = (uint32_t)std::max(2, 13 - (int)kc->wb - log2_lop3);
+    while (kc->it > it && kc->cb < 15) { kc->it--; kc->cb++; }
+}
+
 // CTAs per SM the evaluator kernels are compiled for when the caller does
 // not say: 24 warps per SM (80 registers per thread, no spills on the
 // 3000-gate circuits) measured 9 % faster than the register-unbounded
@@ -288,6 +304,8 @@ int ensure_scratch(nsat_ctx* ctx, size_t bytes) {
     ctx->d_scratch = nullptr;
     ctx->scratch_bytes = 0;
     CK(cudaMalloc(&ctx->d_scratch, bytes));
+    // the QSAT kernel finds its nodes zero and leaves them so
+    CK(cudaMemsetAsync(ctx->d_scratch, 0, bytes, ctx->stream));
     ctx->scratch_bytes = bytes;
     return NSAT_OK;
 }
@@ -506,6 +524,7 @@ int plan_qsat(uint32_t n, const std::vector<uint8_t>& quants_in, bool data, uint
         kc.in_of_bit[p] = (data || in >= (int)n) ? -1 : in;
     }
     choose_shape(C, block_threads, &kc, sh.cb_max);
+    if (!sh.cb_max) choose_chunks(lop3, &kc);
     kc.minb = min_blocks ? min_blocks : default_min_blocks(kc, lop3);
     kc.sync_every = sync_of(sh);
     kc.m = std::min<uint32_t>(m, 127);
@@ -614,14 +633,13 @@ extern "C" int nsat_create(int device, const nsat_opts* opts, nsat_ctx** out) {
     static_assert(sizeof(LaunchOut) * kRing <= kOut && sizeof(NsatJoinState) <= kJoin && sizeof(NsatStopState) <= kStop,
                   "fixed buffer sizes");
     CK(cudaMalloc(&ctx->d_fixed, kOut + kJoin + kStop));
-    CK(cudaMallocHost(&ctx->h_fixed, kOut + kJoin + kStop + kReadStage));
+    CK(cudaMallocHost(&ctx->h_fixed, kOut + kJoin + kStop));
     ctx->d_out = (LaunchOut*)ctx->d_fixed;
     ctx->d_join = (NsatJoinState*)(ctx->d_fixed + kOut);
     ctx->d_stop = (NsatStopState*)(ctx->d_fixed + kOut + kJoin);
     ctx->h_out = (LaunchOut*)ctx->h_fixed;
     ctx->h_join = (NsatJoinState*)(ctx->h_fixed + kOut);
     ctx->h_stop = (NsatStopState*)(ctx->h_fixed + kOut + kJoin);
-    ctx->h_read = ctx->h_fixed + kOut + kJoin + kStop;
     memset(ctx->h_out, 0, sizeof(LaunchOut) * kRing);
     for (int i = 0; i < kRing; i++) {
         ctx->h_out[i].min_idx = ~0ull;
@@ -648,6 +666,7 @@ extern "C" void nsat_destroy(nsat_ctx* ctx) {
     if (ctx->evd) cudaEventDestroy(ctx->evd);
     cudaFree(ctx->d_fixed);
     cudaFreeHost(ctx->h_fixed);
+    cudaFreeHost(ctx->h_read);
     cudaFree(ctx->d_scratch);
     cudaFree(ctx->d_data);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -897,6 +916,14 @@ int qsat_common(nsat_ctx* ctx, nsat_circuit* c, const std::vector<uint8_t>& quan
         if (int rc = data ? get_kernel(ctx, kc, *net, "nsat_qsat", &memo.fn, &memo.mod)
                           : get_circuit_kernel(ctx, c, out0, kc, *net, "nsat_qsat", &memo.fn, &memo.mod))
             return rc;
+        int per_sm = 0;
+        std::string derr;
+        const DriverApi* api = driver_api(&derr);
+        if (!api || api->OccupancyMaxActiveBlocks(&per_sm, memo.fn, (int)kc.threads(), 0) != CUDA_SUCCESS || per_sm < 1)
+            return fail(ctx, NSAT_ECUDA, "occupancy query failed");
+        memo.grid = kc.cb <= kResidentBits
+                        ? 1u << kc.cb
+                        : (unsigned)std::min<uint64_t>(1ull << kc.cb, (uint64_t)per_sm * ctx->sm_count);
         memo.chunk_bits = chunk_bits;
         memo.prefix_bits = prefix_bits;
         memo.quants = quants_in;
@@ -934,7 +961,7 @@ int qsat_common(nsat_ctx* ctx, nsat_circuit* c, const std::vector<uint8_t>& quan
     FinalResult fr;
     bool have = false;
     uint64_t nl = prefix_count > 1 ? prefix_count : (A == 64 ? ~0ull : (1ull << A));
-    const unsigned grid = 1u << kc.cb, threads = kc.threads();
+    const unsigned grid = memo.grid, threads = kc.threads();
     uint64_t launch_idx_buf[kRing];
     unsigned char* scratch = fixed_scratch ? fixed_scratch : ctx->d_scratch;
     const uint32_t* dd = ctx->d_data;
@@ -1187,6 +1214,7 @@ extern "C" int nsat_table_read(nsat_table* t, uint64_t first, uint64_t count, ui
     const uint64_t mask = t->steps ? 0xffffffffull : ~0ull;
     const uint64_t entry = t->narrow ? 4 : 8;
     const char* src = (const char*)t->buf[t->cur] + first * entry;
+    if (!ctx->h_read && count * entry <= kReadStage) CK(cudaMallocHost(&ctx->h_read, kReadStage));
     if (count * entry <= kReadStage) {       // through pinned memory: 8 us instead of 17 for 16 KB
         CK(cudaMemcpyAsync(ctx->h_read, src, count * entry, cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
