@@ -264,7 +264,7 @@ __device__ __forceinline__ void chunk_value(u32 c, u32 v, u32* nodes, LaunchOut*
 
 // Resident CTAs take chunks until none is left: chunk blockIdx.x first, then
 // from the launch's counter (out->values), one at a time while they need
-// evaluation, up to 32 at once while they turn out decided.  NSAT_ONE: the
+// evaluation, up to 16 at once while they turn out decided.  NSAT_ONE: the
 // launch has a CTA for every chunk (the claims' code would cost a small
 // circuit a third of its compile time).
 extern "C" __global__ void NSAT_BOUNDS
@@ -430,7 +430,7 @@ nsat_qsat(u64 launch, LaunchOut* out, LaunchOut* host, u32* nodes, const u32* __
                 claimed = false;
                 base = __shfl_sync(0xffffffffu, base, 0);
                 mask = take >= 32u ? ~0u : (1u << take) - 1u;
-                step = step < 32u ? step * 2u : 32u;
+                step = step < 16u ? step * 2u : 16u;
             }
             if (c != ~0u && mask == 0u && !claimed) {
                 if (lane == 0) ahead = atomicAdd(&out->values, 1u);
