@@ -8,8 +8,9 @@
 // epoch up to a cap, so new arrivals share the device with long jobs right
 // away.  Completion rules follow the one-shot solvers:
 //   SAT    lowest witness (all lower tiles were evaluated in earlier epochs);
-//   QSAT   lowest decisive unit inside tiles, or a host forall/exists reducer
-//          over per-tile values for quantifiers above the tile;
+//   QSAT   lowest decisive unit, found inside tiles or by the job's tree on the
+//          device; a host forall/exists reducer over per-tile values for jobs
+//          that race a compiled kernel or have more than 2^20 tiles;
 //   TABLE  next-state table built tile by tile, then synchronous doubling
 //          with step counts (naivesatostop semantics, lowest stopping start).
 #include <cuda_runtime.h>
@@ -105,6 +106,7 @@ struct Arena {
 struct Program {
     std::vector<SrvIns> ins;
     std::vector<uint16_t> outs;
+    std::vector<uint8_t> reads;      // per input: the program reads it
     uint32_t nslots = 0;
     uint32_t luts = 0;
     uint32_t nops = 0;
@@ -157,6 +159,8 @@ bool build_program(const Circuit& c, const std::vector<uint32_t>& which, bool ra
         for (int64_t q : groups[g])
             if (q >= 0) for (int i = 0; i < 3; i++) last[net.luts[q].in[i]] = (int64_t)g;
     for (const Output& o : net.outs) last[o.wire] = INT64_MAX;
+    p->reads.assign(c.n, 0);
+    for (uint32_t i = 0; i < c.n; i++) p->reads[i] = last[i] >= 0;
     std::vector<int32_t> slot(W, -1);
     for (uint32_t i = 0; i < c.n; i++) slot[i] = (int32_t)i;
     uint32_t next = c.n;
@@ -232,6 +236,8 @@ struct Job {
     std::unique_ptr<QuantReducer> qr;
     SrvJob rec{};
     size_t prog_off = 0, outs_off = 0, table_off = 0, table2_off = 0, reserve = 0;
+    size_t nodes_off = 0, nodes_bytes = 0;   // QSAT tree (0 bytes: none)
+    std::vector<uint32_t> tree;      // its block table
     bool any_stop = false;
     bool find_all = false;
     bool finished = false;
@@ -426,6 +432,27 @@ size_t outs_bytes(const Job* j) { return j->prog.outs.size() * 2 + 2; }
 // SATOSTOP: two areas of 2^n 8-byte entries (the first holds the 32-bit table)
 size_t table_bytes(const Job* j) { return j->kind == SRV_TABLE ? ((size_t)8 << j->n) : 0; }
 
+// Block table of a QSAT job's tree (serve_common.h) and its size in bytes; 0
+// when the job has none: units inside a part, more parts than a tree holds, or
+// a compiled kernel racing the interpreter (whose block results the host folds
+// in order with the tile values).
+size_t plan_tree(Job* j) {
+    j->tree.clear();
+    if (j->kind != SRV_QSAT || j->m < SRV_PART_BITS || j->tier.load() != TIER_NONE ||
+        j->nb - SRV_PART_BITS > SRV_TREE_BITS)
+        return 0;
+    const uint32_t top = j->m - SRV_PART_BITS, part_bits = j->nb - SRV_PART_BITS;
+    auto all = [j](uint32_t l) { return j->quants[j->nb - 1 - (SRV_PART_BITS + l)] != 0; };
+    uint32_t first = 0;
+    for (uint32_t lo = 0, hi; lo < top; lo = hi) {
+        for (hi = lo + 1; hi < top && hi - lo < 8 && all(hi) == all(lo);) hi++;
+        j->tree.push_back(first);
+        j->tree.push_back(hi);
+        first += 1u << (part_bits - hi);
+    }
+    return (2 * SRV_TREE_BLOCKS + (first + 1) / 2) * sizeof(uint32_t);
+}
+
 int admit(nsat_server* s, Job* j) {
     const size_t pbytes = prog_bytes(j), obytes = outs_bytes(j), tbytes = table_bytes(j);
     size_t offs[4] = {0, 0, 0, 0};
@@ -438,6 +465,9 @@ int admit(nsat_server* s, Job* j) {
             return 1;
         }
     }
+    // a job whose tree does not fit next to it is reduced on the host
+    j->nodes_bytes = plan_tree(j);
+    if (j->nodes_bytes && !s->arena.alloc(j->nodes_bytes, &j->nodes_off)) j->nodes_bytes = 0;
     j->slot = s->free_slots.back();
     s->free_slots.pop_back();
     j->prog_off = offs[0]; j->outs_off = offs[1];
@@ -450,13 +480,29 @@ int admit(nsat_server* s, Job* j) {
     SCK(cudaMemcpyAsync(s->arena.base + j->outs_off, j->prog.outs.data(), j->prog.outs.size() * 2, cudaMemcpyHostToDevice, st));
     SCK(cudaMemcpyAsync(s->d_state + j->slot, s->h_state_init, sizeof(SrvState), cudaMemcpyHostToDevice, st));
     s->h2d_bytes += j->prog.ins.size() * sizeof(SrvIns) + j->prog.outs.size() * 2 + sizeof(SrvState);
+    if (j->nodes_bytes) {
+        SCK(cudaMemsetAsync(s->arena.base + j->nodes_off, 0, j->nodes_bytes, st));
+        if (!j->tree.empty())
+            SCK(cudaMemcpyAsync(s->arena.base + j->nodes_off, j->tree.data(), j->tree.size() * 4, cudaMemcpyHostToDevice,
+                                st));
+        s->h2d_bytes += j->tree.size() * 4;
+        j->qr.reset();       // the decisive unit comes from the device
+    }
     SrvJob& r = j->rec;
     memset(&r, 0, sizeof(r));
     r.prog = (const SrvIns*)(s->arena.base + j->prog_off);
     r.outs = (const uint16_t*)(s->arena.base + j->outs_off);
     r.st = s->d_state + j->slot;
     r.flags = j->find_all ? SRV_JOB_FIND_ALL : 0u;
+    if (s->opts.rollover && j->kind != SRV_QSAT) r.flags |= SRV_JOB_ROLLOVER;
     r.table = tbytes ? (uint32_t*)(s->arena.base + j->table_off) : nullptr;
+    r.nodes = j->nodes_bytes ? (uint32_t*)(s->arena.base + j->nodes_off) : nullptr;
+    r.nblk = (uint32_t)(j->tree.size() / 2);
+    // whole tiles where roll-over moves the cursor by tiles, or the host
+    // reduces their values
+    r.sub = (r.flags & SRV_JOB_ROLLOVER) || (j->kind == SRV_QSAT && j->m >= SRV_PART_BITS && !j->nodes_bytes)
+                ? 0
+                : SRV_SUB_BITS;
     r.ngroups = (uint32_t)(j->prog.ins.size() / kSrvShapes[s->shape].group);
     r.nslots = j->prog.nslots;
     r.kind = j->kind;
@@ -480,6 +526,8 @@ int admit(nsat_server* s, Job* j) {
     } else {
         for (uint32_t p = 0; p < j->n; p++) r.in_slot[p] = (int8_t)p;
     }
+    for (int p = 0; p < SRV_MAX_NB; p++)
+        if (r.in_slot[p] >= 0 && !j->prog.reads[r.in_slot[p]]) r.in_slot[p] = -1;
     j->res.admit_ms = now_ms();
     return 0;
 }
@@ -489,6 +537,7 @@ void release(nsat_server* s, Job* j) {
     j->slot = UINT32_MAX;
     s->arena.release(j->prog_off, prog_bytes(j));
     s->arena.release(j->outs_off, outs_bytes(j));
+    if (j->nodes_bytes) s->arena.release(j->nodes_off, j->nodes_bytes);
     if (j->kind == SRV_TABLE) {
         s->arena.release(j->table_off, table_bytes(j));
         s->arena.release(j->table2_off, table_bytes(j));
@@ -946,11 +995,12 @@ int process_epoch(nsat_server* s, EpochBuf& b) {
         const SrvState& st = b.h_state[j->slot];   // cursor and results as the epoch left them
         j->inflight--;
         if (j->finished) continue;   // answered by an earlier epoch; this slice ran ahead
-        // every tile below the device cursor has been evaluated: the kernels
-        // of this and earlier epochs finished before the state was copied
-        const uint64_t got = st.claim - j->cursor;
-        j->res.tiles += got;
-        j->cursor = st.claim;
+        // every tile below the cursor has been evaluated: the kernels of this
+        // and earlier epochs finished before the state was copied, and without
+        // roll-over they hand out exactly their slices
+        const uint64_t cursor = (r.flags & SRV_JOB_ROLLOVER) ? st.claim : r.tile_end;
+        j->res.tiles += cursor - j->cursor;
+        j->cursor = cursor;
         bool finished = false;
         if (j->kind == SRV_SAT) {
             j->count = st.count;

@@ -26,7 +26,9 @@ static const SrvShape kSrvShapes[SRV_NSHAPES] = {
 };
 #define SRV_MAX_GROUP 4
 #define SRV_MAX_SLOTS 384          // slots per warp (384 x 512 B = 192 KB of shared memory at W = 4)
-#define SRV_TILE_BITS 15           // assignments per warp tile
+#define SRV_TILE_BITS 15           // assignments per tile, the unit of slices
+#define SRV_SUB_BITS 2             // a warp claims a quarter of a tile at a time
+#define SRV_PART_BITS (SRV_TILE_BITS - SRV_SUB_BITS)
 #define SRV_MAX_NB 48              // enumeration bits a serving job may have
 inline uint32_t srv_slot_bytes(uint32_t shape) { return 32u * kSrvShapes[shape].words * 4u; }
 
@@ -64,7 +66,7 @@ struct SrvEpoch {
 typedef unsigned long long srv_u64;   // the device atomics' 64-bit type
 
 struct SrvState {
-    srv_u64 claim;              // next tile to hand out; only grows, never past the epoch's limit
+    srv_u64 claim;              // with roll-over: next tile to hand out; only grows, never past the limit
     srv_u64 count;              // SAT: satisfying assignments in the tiles evaluated so far
     srv_u64 min_idx;            // SAT: lowest witness so far; QSAT (m < tile bits): lowest decisive unit
     uint32_t any;                // TABLE: some state has STOP
@@ -76,6 +78,7 @@ static_assert(sizeof(SrvState) == 64, "SrvState layout");
 // Device job record of one epoch; 256 bytes.  Static fields are written at
 // admission, the slice fields every epoch.
 #define SRV_JOB_FIND_ALL 1u      // flags: a SAT job that counts every solution (no early stop)
+#define SRV_JOB_ROLLOVER 2u      // flags: warps may go on past the slice (tiles are claimed from st->claim)
 
 struct SrvJob {
     // static
@@ -92,7 +95,7 @@ struct SrvJob {
     uint32_t q0all;              // QSAT: first quantifier is All
     uint32_t n;                  // TABLE: state bits
     srv_u64 allbits;            // QSAT: enumeration bit j has quantifier All
-    int8_t in_slot[SRV_MAX_NB];  // enumeration bit -> input slot (-1: dummy)
+    int8_t in_slot[SRV_MAX_NB];  // enumeration bit -> input slot (-1: dummy, or an input the program does not read)
     // per epoch: tiles below tile_end are handed out first; once a warp finds
     // every job's slice used up it may go on to tile_hard (the next slice,
     // without a host round trip), unless the job has already been decided
@@ -100,7 +103,23 @@ struct SrvJob {
     srv_u64 tile_hard;               // roll-over limit (== tile_end: none)
     uint32_t val_off;                // QSAT: offset of the slice's tile values in the epoch buffer
     uint32_t flags;                  // SRV_JOB_FIND_ALL
-    srv_u64 reserved[13];
+    uint32_t* nodes;                 // QSAT tree (below), null when the host reduces the tile values
+    uint32_t nblk;                   // its blocks
+    uint32_t next;                   // parts of the slice claimed so far (0 at the start of every epoch)
+    uint32_t sub;                    // log2 parts per tile: SRV_SUB_BITS, or 0 where whole tiles are needed
+    uint32_t pad;
+    srv_u64 reserved[10];
 };
 
 static_assert(sizeof(SrvJob) == 256, "SrvJob layout");
+
+// Tree of a QSAT job whose units are parts of a tile or larger.  The levels
+// from a part up to the units are cut into blocks of one quantifier, at most 8
+// levels each; a node counts its undecided children in 16 bits, 0x8000 once it
+// is resolved (by a child that decides it, or by its last child).  Parts below
+// a resolved node or above a decisive unit are not evaluated.  `nodes` starts
+// with the block table (two words per block: index of its first node, its
+// upper level above a part), then come the nodes.
+#define SRV_TREE_BLOCKS 32
+#define SRV_TREE_BITS 22             // a job with a tree has at most 2^22 parts (8 MB of nodes)
+

@@ -31,7 +31,13 @@
 // with tiles left checks 32 jobs at a time, one per lane.  When no slice has
 // planned tiles left, warps go on into the next quarter slice of SAT and
 // SATOSTOP jobs that are not decided yet, and end when none has tiles left
-// either (no waiting on anything).
+// either (no waiting on anything).  The parts of a QSAT job report to its
+// tree (serve_common.h), and decided ones are passed over, 32 at a time.
+//
+// A claim is a quarter of a tile (two passes at W = 4): with whole tiles the
+// last wave of an epoch left most warps idle for up to eight passes, and a job
+// of a few tiles used as many warps (2^13 tiles of 1390 LUTs 10.8 ms -> 8.1 ms;
+// 2^9 tiles of 325 LUTs 0.64 ms -> 0.29 ms).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -252,33 +258,78 @@ __device__ __forceinline__ Vals<W> read_out(const char* Sl, const uint16_t* outs
 // bits from SRV_TILE_BITS up are the tile index.  Input slots are rewritten
 // every pass because the program reuses slots of inputs it has finished
 // reading.
+// One block of code per enumeration bit, so a bit's value is a constant or one
+// or two instructions; the slots (-1 for inputs that the program does not
+// read) come four at a time.
 template <int W>
 __device__ __forceinline__ void set_inputs(const SrvJob* J, u64 tile_base, u32 it, u32 lane, char* Sl) {
     constexpr int LOGW = W == 4 ? 2 : 1;
-    const u32 nb = J->nb < SRV_MAX_NB ? J->nb : SRV_MAX_NB;
-    for (u32 p = 0; p < nb; p++) {
-        const int s = J->in_slot[p];
-        if (s < 0) continue;
-        Vals<W> v;
+    const u32* slots = reinterpret_cast<const u32*>(J->in_slot);
 #pragma unroll
-        for (int w = 0; w < W; w++) {
-            u32 x;
-            if (p < 5) x = p == 0 ? 0xAAAAAAAAu : p == 1 ? 0xCCCCCCCCu : p == 2 ? 0xF0F0F0F0u : p == 3 ? 0xFF00FF00u : 0xFFFF0000u;
-            else if (p < 10) x = 0u - ((lane >> (p - 5)) & 1u);
-            else if (p < 10 + LOGW) x = 0u - (((u32)w >> (p - 10)) & 1u);
-            else if (p < SRV_TILE_BITS) x = 0u - ((it >> (p - 10 - LOGW)) & 1u);
-            else x = 0u - (u32)((tile_base >> p) & 1ull);
-            v.v[w] = x;
+    for (int q = 0; q < SRV_MAX_NB / 4; q++) {
+        const u32 four = __ldg(slots + q);
+        if (four == 0xffffffffu) continue;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int p = 4 * q + k;
+            const int s = (int)(four << (24 - 8 * k)) >> 24;
+            if (s < 0) continue;
+            Vals<W> v;
+#pragma unroll
+            for (int w = 0; w < W; w++) {
+                u32 x;
+                if (p < 5) x = p == 0 ? 0xAAAAAAAAu : p == 1 ? 0xCCCCCCCCu : p == 2 ? 0xF0F0F0F0u : p == 3 ? 0xFF00FF00u : 0xFFFF0000u;
+                else if (p < 10) x = 0u - ((lane >> (p - 5)) & 1u);
+                else if (p < 10 + LOGW) x = 0u - (((u32)w >> (p - 10)) & 1u);
+                else if (p < SRV_TILE_BITS) x = 0u - ((it >> (p - 10 - LOGW)) & 1u);
+                else x = 0u - (u32)((tile_base >> p) & 1ull);
+                v.v[w] = x;
+            }
+            sts<W>(Sl + (u32)s * (32u * W * 4u), v);
         }
-        sts<W>(Sl + (u32)s * (32u * W * 4u), v);
     }
 }
 
-// Evaluates tile `tile` of job `J` with this warp.
+// Whether part t of a job with a tree has nothing left to decide.
+__device__ __forceinline__ bool part_decided(const SrvJob* J, u64 t) {
+    const u32* tab = J->nodes;
+    const u32 nblk = J->nblk;
+    bool done = *(volatile const u64*)&J->st->min_idx <= t >> (J->m - SRV_PART_BITS);
+    for (u32 k = 0; k < nblk; k++) {
+        const u32 i = __ldg(tab + 2 * k) + (u32)(t >> __ldg(tab + 2 * k + 1));
+        const u32 w = *(volatile const u32*)(tab + 2 * SRV_TREE_BLOCKS + (i >> 1));
+        done |= ((w >> ((i & 1u) << 4)) & 0x8000u) != 0u;
+    }
+    return done;
+}
+
+// One lane: part t has value v; resolves the nodes above it as far as it goes.
+__device__ __forceinline__ void part_value(const SrvJob* J, u64 t, u32 v) {
+    u32* tab = J->nodes;
+    u32 lo = 0;
+    for (u32 k = 0; k < J->nblk; k++) {
+        const u32 hi = __ldg(tab + 2 * k + 1);
+        const u32 i = __ldg(tab + 2 * k) + (u32)(t >> hi);
+        const u32 sh = (i & 1u) << 4;
+        u32* w = tab + 2 * SRV_TREE_BLOCKS + (i >> 1);
+        if (v != (u32)((J->allbits >> (SRV_PART_BITS + lo)) & 1ull)) {      // the deciding value
+            if ((atomicOr(w, 0x8000u << sh) >> sh) & 0x8000u) return;
+        } else {
+            const u32 old = (atomicAdd(w, 1u << sh) >> sh) & 0xffffu;
+            if (old != (1u << (hi - lo)) - 1u) return;                      // not the last child, or resolved
+            if ((atomicOr(w, 0x8000u << sh) >> sh) & 0x8000u) return;
+        }
+        lo = hi;
+    }
+    if (v == (J->q0all ? 0u : 1u)) atomicMin(&J->st->min_idx, t >> (J->m - SRV_PART_BITS));
+}
+
+// Evaluates part `part` of the 2^J->sub parts of tile `tile` with this warp.
 template <int W, int G, bool DISPATCH>
-__device__ __forceinline__ void do_tile(SrvJob* J, u64 tile, char* __restrict__ Sl, u32 lane, uint8_t* __restrict__ vals,
-                                        const Dec& dc) {
-    constexpr u32 ITERS = 32u / W;                 // program passes per tile
+__device__ __forceinline__ void do_part(SrvJob* J, u64 tile, u32 part, char* __restrict__ Sl, u32 lane,
+                                        uint8_t* __restrict__ vals, const Dec& dc) {
+    const u32 iters = (32u / W) >> J->sub;         // program passes per part
+    const u32 it0 = part * iters;
     const u64 tile_base = tile << SRV_TILE_BITS;     // first assignment of the tile
     const u32 kind = J->kind;
     const SrvIns* prog = J->prog;
@@ -289,7 +340,7 @@ __device__ __forceinline__ void do_tile(SrvJob* J, u64 tile, char* __restrict__ 
     const u32 M = J->m;
     const u64 allbits = J->allbits;
     const u32 dec_all = J->q0all;
-    for (u32 it = 0; it < ITERS; it++) {
+    for (u32 it = it0; it < it0 + iters; it++) {
         set_inputs<W>(J, tile_base, it, lane, Sl);
         run_program<W, G, DISPATCH>(prog, ngroups, Sl, dc);
         if (kind == SRV_SAT) {
@@ -321,7 +372,7 @@ __device__ __forceinline__ void do_tile(SrvJob* J, u64 tile, char* __restrict__ 
                     continue;
                 }
                 b = tree_rt(b, allbits, 5, 5);
-                acc |= (b & 1u) << row;
+                acc |= (b & 1u) << (row - it0 * W);
             }
         } else {   // SRV_TABLE
             const u32 lanes = J->n >= 5 ? 32u : (1u << J->n);
@@ -367,13 +418,20 @@ __device__ __forceinline__ void do_tile(SrvJob* J, u64 tile, char* __restrict__ 
         if (M < 10) {
             cand = warp_min(cand);
             if (lane == 0 && cand != ~0ull) atomicMin(&J->st->min_idx, cand);
-        } else if (M < SRV_TILE_BITS) {
-            const u32 y = tree_rt(acc, allbits, 10, (int)M - 10);
-            const u32 d = (dec_all ? ~y : y) & unit_mask((int)M - 10);
-            if (lane == 0 && d != 0u) atomicMin(&J->st->min_idx, (tile_base >> M) + ((__ffs(d) - 1) >> (M - 10)));
         } else {
-            const u32 y = tree_rt(acc, allbits, 10, 5);
-            if (lane == 0) vals[J->val_off + (tile - J->tile_begin)] = (uint8_t)(y & 1u);
+            const u32 bits = SRV_TILE_BITS - J->sub;      // levels of a part
+            const u64 base = tile_base + ((u64)part << bits);
+            if (M < bits) {
+                const u32 y = tree_rt(acc, allbits, 10, (int)M - 10);
+                const u32 d = (dec_all ? ~y : y) & unit_mask((int)M - 10) & (bits < 15 ? (1u << (1u << (bits - 10))) - 1u : ~0u);
+                if (lane == 0 && d != 0u) atomicMin(&J->st->min_idx, (base >> M) + ((__ffs(d) - 1) >> (M - 10)));
+            } else {
+                const u32 y = tree_rt(acc, allbits, 10, (int)bits - 10);
+                if (lane == 0) {
+                    if (J->nodes) part_value(J, (tile << J->sub) + part, y & 1u);
+                    else vals[J->val_off + (tile - J->tile_begin)] = (uint8_t)(y & 1u);
+                }
+            }
         }
     }
     __syncwarp();
@@ -383,17 +441,35 @@ __device__ __forceinline__ void do_tile(SrvJob* J, u64 tile, char* __restrict__ 
 // phase its next quarter slice, unless it has been decided already (lowest
 // witness or decisive unit found).
 __device__ __forceinline__ u64 claim_limit(const SrvJob* J, u32 phase) {
+    // a decisive unit inside a tile ends a QSAT job (it has no counts to finish)
+    if (J->kind == SRV_QSAT && J->m < SRV_TILE_BITS && *(volatile const u64*)&J->st->min_idx != ~0ull) return 0ull;
     if (!phase) return J->tile_end;
     if (!(J->flags & SRV_JOB_FIND_ALL) && J->kind != SRV_TABLE && *(volatile const u64*)&J->st->min_idx != ~0ull)
         return J->tile_end;
     return J->tile_hard;
 }
 
-// Hands out the job's next tile if it lies below `limit` (~0 otherwise).  A
-// compare-and-swap, so the cursor never passes the limit and stays exact
-// across epochs; a failed swap means another warp took a tile, so the loop
-// ends after at most limit - cursor rounds.
-__device__ __forceinline__ u64 claim_tile(SrvState* st, u64 limit) {
+// The first tile of the job with parts that nobody has claimed.
+__device__ __forceinline__ u64 claimed_to(const SrvJob* J) {
+    if (!(J->flags & SRV_JOB_ROLLOVER)) return J->tile_begin + (*(volatile const u32*)&J->next >> J->sub);
+    return *(volatile const u64*)&J->st->claim;
+}
+
+// Hands out the job's next part of a tile below `limit`, as tile << sub | part
+// (~0: none left).  Without roll-over the tiles are those of the epoch's slice
+// and an add on the epoch's own counter takes them (a compare-and-swap per
+// claim made the claims of a slice quadratic: every success failed the other
+// warps' attempts, 1.5 ms an epoch with 1776 warps).  With roll-over a part is
+// a tile, and a compare-and-swap on the persistent cursor never passes the
+// limit and stays exact across epochs.
+__device__ __forceinline__ u64 claim_part(SrvJob* J, u64 limit) {
+    if (!(J->flags & SRV_JOB_ROLLOVER)) {
+        const u64 count = limit > J->tile_begin ? (limit - J->tile_begin) << J->sub : 0ull;
+        if (*(volatile const u32*)&J->next >= count) return ~0ull;
+        const u32 at = atomicAdd(&J->next, 1u);
+        return at < count ? (J->tile_begin << J->sub) + at : ~0ull;
+    }
+    SrvState* st = J->st;
     u64 cur = *(volatile const u64*)&st->claim;
     while (cur < limit) {
         const u64 prev = atomicCAS(&st->claim, cur, cur + 1);
@@ -422,10 +498,10 @@ __global__ void __launch_bounds__(32, 1) serve_epoch(const SrvEpoch* __restrict_
     while (njobs) {
         // the job this warp is on: one claim, no search
         SrvJob* J = jobs + j;
-        u64 tile = ~0ull;
-        if (lane == 0) tile = claim_tile(J->st, claim_limit(J, phase));
-        tile = __shfl_sync(0xffffffffu, tile, 0);
-        if (tile == ~0ull) {
+        u64 part = ~0ull;
+        if (lane == 0) part = claim_part(J, claim_limit(J, phase));
+        part = __shfl_sync(0xffffffffu, part, 0);
+        if (part == ~0ull) {
             // the next job after j (round robin) with a tile left below its
             // limit: 32 jobs per step, one per lane, so a pass over an epoch
             // of hundreds of jobs costs a few dependent L2 reads, not hundreds
@@ -437,7 +513,7 @@ __global__ void __launch_bounds__(32, 1) serve_epoch(const SrvEpoch* __restrict_
                 if (k < njobs) {
                     jj = j + k;
                     if (jj >= njobs) jj -= njobs;
-                    has = *(volatile const u64*)&jobs[jj].st->claim < claim_limit(&jobs[jj], phase);
+                    has = claimed_to(&jobs[jj]) < claim_limit(&jobs[jj], phase);
                 }
                 const u32 m = __ballot_sync(0xffffffffu, has);
                 if (m) pick = __shfl_sync(0xffffffffu, (int)jj, __ffs(m) - 1);
@@ -451,7 +527,17 @@ __global__ void __launch_bounds__(32, 1) serve_epoch(const SrvEpoch* __restrict_
             }
             continue;
         }
-        do_tile<W, G, DISPATCH>(J, tile, Sl, lane, vals, dc);
+        if (J->nodes && part_decided(J, part)) {
+            // the decided parts that follow the counter are passed over for
+            // everybody, up to 32 at once
+            const u32 cur = __shfl_sync(0xffffffffu, *(volatile const u32*)&J->next, 0);
+            const u64 q = (J->tile_begin << J->sub) + cur + lane;
+            const u32 open = __ballot_sync(0xffffffffu, q >= J->tile_end << J->sub || !part_decided(J, q));
+            const u32 run = open ? (u32)__ffs(open) - 1u : 32u;
+            if (lane == 0 && run) atomicCAS(&J->next, cur, cur + run);
+            continue;
+        }
+        do_part<W, G, DISPATCH>(J, part >> J->sub, (u32)part & ((1u << J->sub) - 1u), Sl, lane, vals, dc);
     }
 }
 
