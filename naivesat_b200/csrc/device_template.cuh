@@ -501,9 +501,10 @@ nsat_table(u64 nwords, u64 w0, void* __restrict__ table, LaunchOut* out, LaunchO
     for (u64 w = (u64)blockIdx.x * NSAT_NT + threadIdx.x; w < nwords; w += stride) {
         u32 x[NSAT_NIN];
         nsat_inputs_word(x, w0 + w);
-        u32 o[64];
+        constexpr int ROWS = NSAT_FMT == 0 ? 32 : 64;
+        u32 o[ROWS];
 #pragma unroll
-        for (int k = 0; k < 64; k++) o[k] = 0u;
+        for (int k = NSAT_NOUT; k < ROWS; k++) o[k] = 0u;
         nsat_eval_all(x, o);
         anystop |= o[NSAT_NOUT - 1];
         constexpr int lanes = NSAT_NB >= 5 ? 32 : (1 << NSAT_NB);
@@ -517,7 +518,7 @@ nsat_table(u64 nwords, u64 w0, void* __restrict__ table, LaunchOut* out, LaunchO
             for (int k = 0; k < 32; k++) st[lane * 33 + k] = o[k];
             __syncwarp();
             u32* dst = reinterpret_cast<u32*>(table) + ((w - lane) << 5);
-#pragma unroll
+#pragma unroll 4
             for (int k = 0; k < 32; k++) dst[k * 32 + lane] = st[k * 33 + lane];
         } else {
             for (int l = 0; l < lanes; l++) reinterpret_cast<u32*>(table)[(w << 5) + l] = o[l];

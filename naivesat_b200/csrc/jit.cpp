@@ -138,7 +138,10 @@ const DriverApi* driver_api(std::string* err) {
 }
 
 namespace {
-const char* const kOpts[] = {"--gpu-architecture=sm_100a", "--std=c++17", "-lineinfo",
+// --minimal leaves out the parts of CUDA's device library that these kernels
+// do not use, and there are no line tables: 3-10 % of a compile (a 300-gate
+// table kernel 166 ms -> 157 ms, 36 inputs and 3018 gates 780 ms -> 690 ms).
+const char* const kOpts[] = {"--gpu-architecture=sm_100a", "--std=c++17", "--minimal",
                              "--ptxas-options=-v", "-DNSAT_JIT=1"};
 const int kNopts = (int)(sizeof(kOpts) / sizeof(kOpts[0]));
 
