@@ -12,6 +12,7 @@
 #include <stdint.h>
 
 #include "greedy_kernels.h"
+#include "pdl.cuh"
 
 typedef unsigned long long u64;
 typedef unsigned int u32;
@@ -151,6 +152,7 @@ __device__ __forceinline__ void chase(u32 (&v)[4], const u32* table, const u32* 
 
 __global__ void __launch_bounds__(256) chase_before(const u32* __restrict__ table, u32 i, u32 lp,
                                                     u32* __restrict__ snap, NsatGreedyState* st) {
+    pdl_wait();
     // only chase_after writes the key: here it is that of an earlier step
     if (*(volatile const u64*)&st->key != ~0ull) {
         if (blockIdx.x == 0 && threadIdx.x == 0) st->done = 1u;
@@ -168,6 +170,7 @@ __global__ void __launch_bounds__(256) chase_before(const u32* __restrict__ tabl
 
 __global__ void __launch_bounds__(256) chase_after(u32* table, const u32* __restrict__ snap, u32 i, u32 lp, u32 n,
                                                    u32 unknowns, u32 step, NsatGreedyState* st) {
+    pdl_wait();
     if (*(volatile const u32*)&st->done) return;
     const u32 stop = 1u << n, before = (u32)((1ull << (n - unknowns)) - 1ull);
     const u32 quads = 1u << (lp - 2), first = i << lp;
@@ -235,7 +238,6 @@ extern "C" int nsat_greedy_find(const uint64_t* dest, uint64_t start, uint64_t c
 extern "C" int nsat_greedy_step(uint32_t* table, uint32_t* snap, uint32_t i, uint32_t lp, uint32_t n,
                                 uint32_t unknowns, uint32_t step, NsatGreedyState* state, int sms, cudaStream_t st) {
     const unsigned g = grid_for((u64)1 << (lp - 2), sms);
-    chase_before<<<g, 256, 0, st>>>(table, i, lp, snap, state);
-    chase_after<<<g, 256, 0, st>>>(table, snap, i, lp, n, unknowns, step, state);
-    return cudaGetLastError() == cudaSuccess ? 0 : -4;
+    if (launch_pdl(chase_before, g, 256, st, table, i, lp, snap, state) != cudaSuccess) return -4;
+    return launch_pdl(chase_after, g, 256, st, table, snap, i, lp, n, unknowns, step, state) == cudaSuccess ? 0 : -4;
 }

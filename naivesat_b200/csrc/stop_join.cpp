@@ -22,13 +22,15 @@ constexpr uint32_t kRoundsPerLevel = 3;   // on a contracted domain
 // of the domain or less remains, for the tables whose rounds take longer than
 // the launches.
 constexpr double kKeepMost = 0.5;
-constexpr uint64_t kContractLeast = 1ull << 20;
+constexpr uint64_t kContractLeast = 1ull << 20;     // of a contracted domain
+constexpr uint64_t kTableLeast = 1ull << 22;        // of the table
+constexpr uint64_t kSecondLook = 1ull << 24;
 constexpr uint32_t kRoundsLeft = 5;       // fewer rounds than this do not pay for one
 // Whether the table contracts is asked of a sample first (256 successors in
 // 65536 are looked at), taken in an early round and read while the next ones
 // run: bijections keep all their states in every round, and marking 2^24
 // successors costs two rounds.  Round 1 tells a random function (0.47) from
-// one that hardly shrinks; those are asked once more, later.
+// one that hardly shrinks; a large table is asked once more, later.
 struct Look {
     uint32_t sample, contract;             // rounds
     double keep;                           // the most that may remain of the sample
@@ -110,7 +112,7 @@ int stop_run(nsat_ctx* ctx, StopRun* x) {
     std::vector<Level> lv;
     uint32_t* sample = nullptr;
     uint32_t* at_dist = nullptr;
-    const uint32_t sample_words = N >= kContractLeast ? (uint32_t)(N >> 13) : 0;
+    const uint32_t sample_words = N >= kTableLeast ? (uint32_t)(N >> 13) : 0;
     const Look looks[2] = {{1, first_rounds(N), 0.85}, {6, 8, kKeepMost}};
     uint32_t look = 0, contract_at = n + 1;
     if (!sample_words || !mem.get(&sample, sample_words)) look = 2;
@@ -118,12 +120,13 @@ int stop_run(nsat_ctx* ctx, StopRun* x) {
     for (uint32_t r = 1; r <= n; r++) {
         if (lv.empty()) {
             const bool sampling = look < 2 && r == looks[look].sample && n > looks[look].contract + kRoundsLeft;
-            if (sampling) JCK(cudaMemsetAsync(sample, 0, (size_t)sample_words * 4, st));
+            if (sampling) {
+                JCK(cudaMemsetAsync(sample, 0, (size_t)sample_words * 4, st));
+                if (look) JCK(cudaMemsetAsync(&d->distinct, 0, 4, st));
+            }
             JRUN(nsat_stop_join(T[(r - 1) & 1], T[r & 1], dist, n, u, r, mode, d, sampling ? sample : nullptr, sms, st));
             if (sampling) {
-                JRUN(nsat_stop_sample_count(sample, sample_words, d, st));
                 JCK(cudaMemcpyAsync(&h->distinct, &d->distinct, 4, cudaMemcpyDeviceToHost, st));
-                JCK(cudaMemsetAsync(&d->distinct, 0, 4, st));
                 JCK(cudaEventRecord(ctx_stop_event(ctx), st));
                 contract_at = looks[look].contract;
                 sampled = true;
@@ -140,7 +143,10 @@ int stop_run(nsat_ctx* ctx, StopRun* x) {
             sampled = false;
             JCK(cudaEventSynchronize(ctx_stop_event(ctx)));
             const double keep = looks[look++].keep;
-            if (256.0 * h->distinct > keep * (double)N) continue;
+            if (256.0 * h->distinct > keep * (double)N) {
+                if (N < kSecondLook) look = 2;
+                continue;
+            }
             look = 2;
         }
         // contract to the successors

@@ -34,6 +34,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "pdl.cuh"
 #include "stop_kernels.h"
 
 typedef unsigned int u32;
@@ -45,13 +46,13 @@ constexpr u32 kNone = 0xffffffffu;
 
 // An odd multiplier is a bijection of the n-bit states; the states whose
 // image has its top 8 bits clear are a 256th of them, spread over the table.
-__device__ __forceinline__ void sample_mark(u32* sample, u32 v, u32 bits) {
+// Returns 1 for the first of equal ones.
+__device__ __forceinline__ u32 sample_mark(u32* sample, u32 v, u32 bits) {
     const u32 h = (v * 0x9E3779B1u) & (u32)((1ull << bits) - 1ull);
-    if ((h >> (bits - 8)) == 0u) {
-        const u32 m = 1u << (h & 31u);
-        u32* w = sample + (h >> 5);
-        if (!(*w & m)) atomicOr(w, m);
-    }
+    if ((h >> (bits - 8)) != 0u) return 0u;
+    const u32 m = 1u << (h & 31u);
+    u32* w = sample + (h >> 5);
+    return !(*w & m) && !(atomicOr(w, m) & m) ? 1u : 0u;
 }
 
 // An answered round ends the loop: later rounds carry the answer forward and
@@ -77,11 +78,12 @@ template <bool DIST, bool SAMPLE>
 __global__ void __launch_bounds__(256) join32(const u32* __restrict__ src, u32* __restrict__ dst,
                                               u32* __restrict__ dist, u64 N, u32 n, u32 u, u32 r, u32 mode,
                                               NsatStopState* __restrict__ st, u32* __restrict__ sample) {
+    pdl_wait();
     if (answered(st, r, mode)) return;
     const u32 stop = 1u << n, nmask = stop - 1u;
     const u32 smask = (u32)((1ull << (n - u)) - 1ull);
     const u32 half = 1u << (r - 1);      // evaluations an entry of src stands for
-    u32 best = kNone;
+    u32 best = kNone, fresh = 0;
     const u64 S = (u64)gridDim.x * blockDim.x;
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += 4 * S) {
         // four independent gathers in flight per thread
@@ -109,9 +111,13 @@ __global__ void __launch_bounds__(256) join32(const u32* __restrict__ src, u32* 
                 }
                 if (((u32)j & smask) == 0u && (u32)j < best) best = (u32)j;
             } else if constexpr (SAMPLE) {
-                sample_mark(sample, w[k], n);
+                fresh += sample_mark(sample, w[k], n);
             }
         }
+    }
+    if constexpr (SAMPLE) {
+        fresh = __reduce_add_sync(0xffffffffu, fresh);
+        if ((threadIdx.x & 31) == 0 && fresh) atomicAdd(&st->distinct, fresh);
     }
     best = __reduce_min_sync(0xffffffffu, best);
     if ((threadIdx.x & 31) == 0 && best != kNone) atomicMin(&st->best[r], best);
@@ -199,14 +205,6 @@ SmallKernel small_kernel(u32 n) {
     case 14: return small_solve<STEPS, 16>;
     default: return small_solve<STEPS, 1>;     // up to 2^10 entries
     }
-}
-
-__global__ void __launch_bounds__(256) sample_count(const u32* __restrict__ sample, u32 words,
-                                                    NsatStopState* __restrict__ st) {
-    u32 c = 0;
-    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < words; i += gridDim.x * blockDim.x) c += __popc(sample[i]);
-    c = __reduce_add_sync(0xffffffffu, c);
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(&st->distinct, c);
 }
 
 // The test before the atomic may read a stale word: bits only get set, so it
@@ -378,6 +376,7 @@ __global__ void __launch_bounds__(256) join_pq(const u64* __restrict__ P, const 
                                                u64* __restrict__ P2, u64* __restrict__ Q2,
                                                const u32* __restrict__ start, u32 count, u32 n, u32 r, u32 mode,
                                                NsatStopState* __restrict__ st) {
+    pdl_wait();
     if (answered(st, r, mode)) return;
     const u32 stop = 1u << n;
     u32 best = kNone;
@@ -482,11 +481,9 @@ extern "C" int nsat_stop_join(const uint32_t* src, uint32_t* dst, uint32_t* dist
                               uint32_t mode, NsatStopState* st, uint32_t* sample, int sms, cudaStream_t s) {
     const u64 N = 1ull << n;
     const unsigned g = blocks_for(N, sms, 4);
-    if (dist && sample) join32<true, true><<<g, 256, 0, s>>>(src, dst, dist, N, n, u, r, mode, st, sample);
-    else if (dist) join32<true, false><<<g, 256, 0, s>>>(src, dst, dist, N, n, u, r, mode, st, nullptr);
-    else if (sample) join32<false, true><<<g, 256, 0, s>>>(src, dst, nullptr, N, n, u, r, mode, st, sample);
-    else join32<false, false><<<g, 256, 0, s>>>(src, dst, nullptr, N, n, u, r, mode, st, nullptr);
-    return ok();
+    const auto fn = dist ? (sample ? join32<true, true> : join32<true, false>)
+                         : (sample ? join32<false, true> : join32<false, false>);
+    return launch_pdl(fn, g, 256, s, src, dst, dist, N, n, u, r, mode, st, sample) == cudaSuccess ? 0 : -4;
 }
 
 extern "C" int nsat_stop_small(const uint32_t* src, uint32_t n, uint32_t u, uint32_t mode, int steps,
@@ -500,12 +497,6 @@ extern "C" int nsat_stop_small(const uint32_t* src, uint32_t n, uint32_t u, uint
                                                  8 << NSAT_STOP_SMALL_BITS) != cudaSuccess)
         return -4;
     fn<<<1, kSmallThreads, smem, s>>>(src, n, u, mode, out32, (u64*)out64, st);
-    return ok();
-}
-
-extern "C" int nsat_stop_sample_count(const uint32_t* sample, uint32_t words, NsatStopState* st, cudaStream_t s) {
-    const unsigned g = (words + 1023) / 1024;
-    sample_count<<<g < 1 ? 1 : (g > 64 ? 64 : g), 256, 0, s>>>(sample, words, st);
     return ok();
 }
 
@@ -560,8 +551,8 @@ extern "C" int nsat_stop_join_pq(const uint64_t* P, const uint64_t* Q, uint64_t*
                                  const uint32_t* start, uint32_t count, uint32_t n, uint32_t r, uint32_t mode,
                                  NsatStopState* st, int sms, cudaStream_t s) {
     const unsigned g = blocks_for(count, sms, 2);
-    join_pq<<<g, 256, 0, s>>>((const u64*)P, (const u64*)Q, (u64*)P2, (u64*)Q2, start, count, n, r, mode, st);
-    return ok();
+    return launch_pdl(join_pq, g, 256, s, (const u64*)P, (const u64*)Q, (u64*)P2, (u64*)Q2, start, count, n, r, mode,
+                      st) == cudaSuccess ? 0 : -4;
 }
 
 extern "C" int nsat_stop_expand64(uint64_t* upQ, uint32_t up_count, const uint64_t* Q, const uint32_t* states,

@@ -22,8 +22,9 @@ extern "C" {
 #endif
 
 // Round r of synchronous doubling, dst = src o src.  dist (or null): distance
-// of the entries that have stopped.  sample (or null): bitmap of
-// 2^(n-8) bits, cleared, in which a 256th of the successors is marked.
+// of the entries that have stopped.  sample (or null): bitmap of 2^(n-8) bits,
+// cleared, in which a 256th of the successors is marked; st->distinct counts
+// the bits set.
 int nsat_stop_join(const uint32_t* src, uint32_t* dst, uint32_t* dist, uint32_t n, uint32_t u, uint32_t r,
                    uint32_t mode, NsatStopState* st, uint32_t* sample, int sms, cudaStream_t s);
 // Every round of a table of n <= NSAT_STOP_SMALL_BITS bits, with distances
@@ -31,8 +32,6 @@ int nsat_stop_join(const uint32_t* src, uint32_t* dst, uint32_t* dist, uint32_t 
 // table after the last one.
 int nsat_stop_small(const uint32_t* src, uint32_t n, uint32_t u, uint32_t mode, int steps, uint32_t* out32,
                     uint64_t* out64, NsatStopState* st, cudaStream_t s);
-// st->distinct = set bits of the sample bitmap
-int nsat_stop_sample_count(const uint32_t* sample, uint32_t words, NsatStopState* st, cudaStream_t s);
 
 // Contraction to the states that a later round can still look up.
 // marks in bits (cleared, items bits) the successors of items entries, unless
