@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(256) join32(const u32* __restrict__ src, u32* 
         for (int k = 0; k < 4; k++) {
             if (!ok[k]) continue;
             const u64 j = i + (u64)k * S;
-            dst[j] = w[k];
+            __stcs(dst + j, w[k]);      // leaves the L2 to src, which the gathers reread (2^24 entries: 5 %)
             if (w[k] & stop) {
                 if constexpr (DIST) {
                     // an entry of src that has stopped has its distance from the
