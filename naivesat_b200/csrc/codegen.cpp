@@ -1,8 +1,11 @@
 // codegen.cpp -- emit the per-circuit CUDA source compiled by NVRTC.
 #include "codegen.h"
 
+#include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <sstream>
+#include <unordered_map>
 
 namespace nsat {
 
@@ -22,47 +25,134 @@ typedef unsigned int u32;
 typedef unsigned long long u64;
 )NSAT";
 
+// LUTs of one asm block without barriers, and where the evaluators use blocks:
+// from 400 LUTs (the compiler's sharing between iterations is worth more
+// below: 24 inputs, 280 LUTs, run 139 instructions a word), for searches of up
+// to 0.1 s.  Blocks compile a 2000-3000-gate circuit 70-120 ms faster and run
+// 0.1-0.9 % slower (33 inputs, 1216 LUTs: first solve 476 -> 350 ms, device
+// time 17.74 -> 17.76 ms).
+constexpr uint32_t kBlockLuts = 128;
+constexpr size_t kBlocksFrom = 400;
+bool use_blocks(const KernelConfig& kc, const LutNet& net) {
+    if (kc.mode == Mode::TABLE) return true;
+    if (net.luts.size() < kBlocksFrom) return false;
+    return kc.mode == Mode::QSAT ||
+           std::ldexp((double)net.luts.size(), (int)kc.nb - 5) < 0.1 * kCompiledLutWordsPerS;
+}
+
 const uint32_t kLanePat[5] = {0xAAAAAAAAu, 0xCCCCCCCCu, 0xF0F0F0F0u, 0xFF00FF00u, 0xFFFF0000u};
 
-// sync_every > 0: a CTA barrier after every sync_every LUTs, so the CTA's
-// warps walk the evaluation code together and share instruction-cache lines
-// (the unrolled evaluation of a large circuit is larger than the
-// instruction cache; c1 at 64: ALU pipe 89 % -> 0.99 of the lop3 peak).  Only
-// for kernels whose every thread runs the same number of evaluations.
-void emit_luts(std::ostringstream& s, const LutNet& net, uint32_t sync_every = 0) {
-    for (uint32_t i : net.used_inputs) s << "    const u32 w" << i << " = x[" << i << "];\n";
-    uint32_t k = 0;
-    // one lop3.b32 per LUT, the truth table as its immediate; written as
-    // inline asm in place (a helper template per call site costs NVVM about
-    // twice the compile time on circuits of a few thousand gates).  The lines
-    // are appended directly: the LUTs are most of the source, and formatting
-    // them through printf took most of the generation time.
+void append_dec(std::string& o, uint32_t v) {
+    char t[10];
+    int d = 0;
+    do { t[d++] = (char)('0' + v % 10); v /= 10; } while (v);
+    while (d) o.push_back(t[--d]);
+}
+
+void append_tt(std::string& o, uint8_t tt) {
     static const char kHex[] = "0123456789abcdef";
-    auto dec = [](std::string& o, uint32_t v) {
-        char t[10];
-        int d = 0;
-        do { t[d++] = (char)('0' + v % 10); v /= 10; } while (v);
-        while (d) o.push_back(t[--d]);
-    };
-    std::string b;
+    o += "0x";
+    o.push_back(kHex[tt >> 4]);
+    o.push_back(kHex[tt & 15]);
+}
+
+// One asm statement per LUT: the compiler hoists and shares single LUTs, which
+// is worth half of a small circuit's work when it unrolls the iterations.
+void emit_single_luts(std::string& b, const LutNet& net, uint32_t sync_every) {
+    uint32_t k = 0;
     b.reserve(net.luts.size() * 112 + (sync_every ? net.luts.size() / sync_every * 20 : 0) + 16);
     for (const Lut& L : net.luts) {
         b += "    u32 w";
-        dec(b, L.wire);
-        b += "; asm(\"lop3.b32 %0, %1, %2, %3, 0x";
-        b.push_back(kHex[L.tt >> 4]);
-        b.push_back(kHex[L.tt & 15]);
+        append_dec(b, L.wire);
+        b += "; asm(\"lop3.b32 %0, %1, %2, %3, ";
+        append_tt(b, L.tt);
         b += ";\" : \"=r\"(w";
-        dec(b, L.wire);
+        append_dec(b, L.wire);
         b += ") : \"r\"(w";
-        dec(b, L.in[0]);
+        append_dec(b, L.in[0]);
         b += "), \"r\"(w";
-        dec(b, L.in[1]);
+        append_dec(b, L.in[1]);
         b += "), \"r\"(w";
-        dec(b, L.in[2]);
+        append_dec(b, L.in[2]);
         b += "));\n";
         if (sync_every && ++k % sync_every == 0) b += "    __syncthreads();\n";
     }
+}
+
+// One asm block per `seg` LUTs, whose operands are the wires that cross the
+// block's ends.  The front end and the optimiser see one statement where there
+// were `seg`: 1229 LUTs compile in 531 ms instead of 701, a
+// 24-bit next-state table in 135 instead of 149.
+void emit_lut_blocks(std::string& b, const LutNet& net, uint32_t seg, bool sync) {
+    const size_t n = net.luts.size();
+    std::unordered_map<uint32_t, size_t> last;       // wire -> last LUT that reads it (n: an output)
+    for (size_t k = 0; k < n; k++)
+        for (int i = 0; i < 3; i++) last[net.luts[k].in[i]] = k;
+    for (const Output& o : net.outs) last[o.wire] = n;
+    b.reserve(n * 48 + 256);
+    std::unordered_map<uint32_t, std::string> name;
+    for (size_t a = 0; a < n; a += seg) {
+        const size_t e = std::min(n, a + seg);
+        name.clear();
+        std::string outs, ins, decl;
+        uint32_t ops = 0, temps = 0;
+        auto operand = [&](uint32_t w) {
+            std::string t = "%";
+            append_dec(t, ops++);
+            name[w] = t;
+        };
+        for (size_t k = a; k < e; k++) {             // outputs first, as asm operands are numbered
+            const uint32_t w = net.luts[k].wire;
+            const auto l = last.find(w);
+            if (l == last.end() || l->second < e) {
+                std::string t = "t";
+                append_dec(t, temps++);
+                name[w] = t;
+                continue;
+            }
+            operand(w);
+            outs += (outs.empty() ? "\"=&r\"(w" : ", \"=&r\"(w");
+            append_dec(outs, w);
+            outs += ")";
+            decl += decl.empty() ? "    u32 w" : ", w";
+            append_dec(decl, w);
+        }
+        for (size_t k = a; k < e; k++)
+            for (int i = 0; i < 3; i++) {
+                const uint32_t w = net.luts[k].in[i];
+                if (name.count(w)) continue;
+                operand(w);
+                ins += (ins.empty() ? "\"r\"(w" : ", \"r\"(w");
+                append_dec(ins, w);
+                ins += ")";
+            }
+        b += decl + ";\n    asm(\"{ .reg .b32 t<";
+        append_dec(b, temps + 1);
+        b += ">;\\n\"\n";
+        for (size_t k = a; k < e; k++) {
+            const Lut& L = net.luts[k];
+            b += "\"lop3.b32 " + name[L.wire] + ", " + name[L.in[0]] + ", " + name[L.in[1]] + ", " + name[L.in[2]] + ", ";
+            append_tt(b, L.tt);
+            b += ";\\n\"\n";
+        }
+        b += "\"}\" : " + outs + " : " + ins + ");\n";
+        if (sync && e - a == seg) b += "    __syncthreads();\n";
+    }
+}
+
+// The evaluation of the LUTs, one lop3.b32 each with the truth table as its
+// immediate.  sync_every > 0: a CTA barrier after every sync_every LUTs, so
+// the CTA's warps walk the evaluation code together and share
+// instruction-cache lines (the unrolled evaluation of a large circuit is larger
+// than the instruction cache; c1 at 64: ALU pipe 89 % -> 0.99 of the lop3
+// peak).  Only for kernels whose every thread runs the same number of
+// evaluations.  The lines are appended directly: formatting them through
+// printf took most of the generation time.
+void emit_luts(std::ostringstream& s, const LutNet& net, bool blocks, uint32_t sync_every = 0) {
+    for (uint32_t i : net.used_inputs) s << "    const u32 w" << i << " = x[" << i << "];\n";
+    std::string b;
+    if (blocks) emit_lut_blocks(b, net, sync_every ? sync_every : kBlockLuts, sync_every != 0);
+    else emit_single_luts(b, net, sync_every);
     s.write(b.data(), (std::streamsize)b.size());
 }
 
@@ -135,7 +225,7 @@ std::string generate_source(const KernelConfig& kc, const LutNet& net) {
     if (kc.mode == Mode::TABLE) {
         s << "__device__ __forceinline__ void nsat_eval1(const u32* x) {}\n";
         s << "__device__ __forceinline__ void nsat_eval_all(const u32* x, u32* o) {\n";
-        emit_luts(s, net);
+        emit_luts(s, net, use_blocks(kc, net));
         for (size_t j = 0; j < net.outs.size(); j++)
             s << "    o[" << j << "] = " << (net.outs[j].neg ? "~" : "") << "w" << net.outs[j].wire << ";\n";
         s << "}\n";
@@ -145,7 +235,7 @@ std::string generate_source(const KernelConfig& kc, const LutNet& net) {
             // the SAT and QSAT kernels run the same number of evaluations in
             // every thread of a CTA, so barriers inside the evaluation are safe
             const bool uniform = kc.mode == Mode::SAT || kc.mode == Mode::QSAT;
-            emit_luts(s, net, uniform && kc.threads() > 32 ? kc.sync_every : 0);
+            emit_luts(s, net, use_blocks(kc, net), uniform && kc.threads() > 32 ? kc.sync_every : 0);
             s << "    return " << (net.outs[0].neg ? "~" : "") << "w" << net.outs[0].wire << ";\n";
         } else {
             s << "    return 0u;\n";
