@@ -139,7 +139,9 @@ typedef struct {
     uint64_t count_lo, count_hi;      /* solutions among the scanned indices */
     uint64_t witness_lo, witness_hi;  /* lowest satisfying index */
     uint64_t scanned_lo, scanned_hi;  /* assignments scanned */
-    double device_ms;                 /* kernel time, CUDA events */
+    double device_ms;                 /* kernel time: CUDA events, or of one launch
+                                         estimated below 0.25 ms the kernel's own
+                                         span (global timer, 32 ns) */
     double wall_ms;                   /* host time of the call */
 } nsat_sat_result;
 
@@ -172,7 +174,7 @@ typedef struct {
     uint32_t chunk_bits;       /* log2 assignments per launch actually used */
     uint64_t scanned;          /* assignments of the launches run (launches x 2^chunk_bits);
                                   what is decided already is not evaluated */
-    double device_ms;
+    double device_ms;          /* as in nsat_sat_result */
     double wall_ms;
 } nsat_qsat_result;
 
@@ -235,7 +237,8 @@ typedef struct {
     int32_t found;
     uint32_t rounds;       /* doubling rounds run */
     uint64_t start, end, steps;   /* steps only with want_steps */
-    double build_ms, join_ms;
+    double build_ms, join_ms;     /* as device_ms of nsat_sat_result: by the global
+                                     timer up to 2^20 states (build), 2^14 (rounds) */
 } nsat_stop_result;
 
 int nsat_stop_solve(nsat_ctx* ctx, nsat_table* t, const nsat_stop_opts* opts,

@@ -37,55 +37,90 @@ struct LaunchOut {
     u32 ticket;    // CTAs finished
     u32 any;       // table build: some STOP output seen
     u32 values;    // QSAT: chunks claimed beyond the first of each CTA
+    u32 t0;        // global timer at the first CTA's start (ns)
+    u32 pad;
 };
 
-// The last CTA of a launch: copies the result to pinned host memory and puts
-// the slot back as the next launch expects it.  A solve is a kernel between
-// two events; a copy that set the slot and one that read it back took 6 us of
-// a small solve.
-__device__ __forceinline__ void nsat_publish(LaunchOut* out, LaunchOut* host) {
-    volatile LaunchOut* o = out;
-    volatile LaunchOut* h = host;
-    h->min_idx = o->min_idx;
-    h->count = o->count;
-    h->tree = o->tree;
-    h->any = o->any;
-    o->min_idx = ~0ull;
-    o->count = 0ull;
-    o->tree = 0u;
-    o->ticket = 0u;
-    o->any = 0u;
+__device__ __forceinline__ u32 nsat_now() {
+    u32 t;
+    asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t));
+    return t;
+}
+
+// First statement of a kernel.
+__device__ __forceinline__ void nsat_begin(LaunchOut* out) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *(volatile u32*)&out->t0 = nsat_now();
+}
+
+// The last CTA of a launch: puts the slot back as the next launch expects it
+// and writes the result to pinned host memory: min_idx, the kind's value and
+// the kernel's time.  The host waits for the stream or, after one short
+// launch, polls; so each 32-bit half goes in a 64-bit word with the launch's
+// number, which vouches for it, and no fence orders the words.  A pair of
+// timing events around a kernel and the wait for the second take 11 us of a
+// small solve; a copy that set the slot and one that read it back took 6 us.
+// One asm block: as statements the compiler took 6 ms for it, a tenth of a
+// small circuit's compile.
+#if NSAT_MODE_SAT
+#define NSAT_VALUE "ld.volatile.global.u64 v, [%0+8];"       // count
+#elif NSAT_MODE_QSAT
+#define NSAT_VALUE "ld.volatile.global.u32 a, [%0+16];\n\tmov.b64 v, {a, 0};"      // tree
+#else
+#define NSAT_VALUE "ld.volatile.global.u32 a, [%0+24];\n\tmov.b64 v, {a, 0};"      // any
+#endif
+__device__ __forceinline__ void nsat_publish(LaunchOut* out, u64* host, u32 seq) {
+    asm volatile(
+        "{\n\t"
+        ".reg .b64 m, v;\n\t"
+        ".reg .b32 a, b, t, t0;\n\t"
+        "ld.volatile.global.u64 m, [%0];\n\t"
+        NSAT_VALUE "\n\t"
+        "ld.volatile.global.u32 t0, [%0+32];\n\t"
+        "mov.u32 t, %%globaltimer_lo;\n\t"
+        "sub.u32 t, t, t0;\n\t"
+        "st.volatile.global.u64 [%0], -1;\n\t"        // min_idx
+        "st.volatile.global.u64 [%0+8], 0;\n\t"       // count
+        "st.volatile.global.u64 [%0+16], 0;\n\t"      // tree, ticket
+        "st.volatile.global.u32 [%0+24], 0;\n\t"      // any
+        "mov.b64 {a, b}, m;\n\t"
+        "mov.b64 m, {a, %2};\n\t"
+        "st.volatile.global.u64 [%1], m;\n\t"
+        "mov.b64 m, {b, %2};\n\t"
+        "st.volatile.global.u64 [%1+8], m;\n\t"
+        "mov.b64 {a, b}, v;\n\t"
+        "mov.b64 m, {a, %2};\n\t"
+        "st.volatile.global.u64 [%1+16], m;\n\t"
+        "mov.b64 m, {b, %2};\n\t"
+        "st.volatile.global.u64 [%1+24], m;\n\t"
+        "mov.b64 m, {t, %2};\n\t"
+        "st.volatile.global.u64 [%1+32], m;\n\t"
+        "}" ::"l"(out), "l"(host), "r"(seq) : "memory");
 }
 
 // Ends a CTA, all threads together, after its last update of *out.
-__device__ __forceinline__ void nsat_finish(LaunchOut* out, LaunchOut* host) {
+__device__ __forceinline__ void nsat_finish(LaunchOut* out, u64* host, u32 seq) {
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
         if (atomicAdd(&out->ticket, 1u) == gridDim.x - 1u) {
             __threadfence();
-            nsat_publish(out, host);
+            nsat_publish(out, host, seq);
         }
     }
-}
-
-__device__ __forceinline__ u64 warp_min_u64(u64 v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        u64 w = __shfl_xor_sync(0xffffffffu, v, o);
-        v = w < v ? w : v;
-    }
-    return v;
 }
 
 #if NSAT_MODE_SAT
 // --------------------------------------------------------------------------
 // SAT: count every satisfying assignment and find the lowest one.
 extern "C" __global__ void NSAT_BOUNDS
-nsat_sat(u64 launch, LaunchOut* out, LaunchOut* host) {
+nsat_sat(u64 launch, LaunchOut* out, u64* host, u32 seq) {
+    nsat_begin(out);
     const u32 lane = threadIdx.x & 31u;
     const u32 warp = threadIdx.x >> 5;
     const u32 cta = blockIdx.x;
+    __shared__ u32 s_idx, s_cnt;
+    if (threadIdx.x == 0) { s_idx = ~0u; s_cnt = 0u; }
+    __syncthreads();
     u32 x[NSAT_NIN];
     nsat_inputs_fixed(x, lane, warp, cta, launch);
     u32 cnt = 0;
@@ -96,40 +131,23 @@ nsat_sat(u64 launch, LaunchOut* out, LaunchOut* host) {
         cnt += __popc(y);
         if (y != 0u && first_it == 0xffffffffu) { first_it = it; first_bit = __ffs(y) - 1; }
     }
-    u64 idx = ~0ull;
-    if (first_it != 0xffffffffu) {
-        const u64 w = ((u64)cta << (5 + NSAT_IT + NSAT_WB)) | ((u64)warp << (5 + NSAT_IT)) |
-                      ((u64)first_it << 5) | lane;
-        idx = (w << 5) | first_bit;
+    // index within the CTA: 10 + IT + WB <= 25 bits, and at most 2^25 solutions
+    // to count.  One pair of atomics per CTA: launches with few iterations per
+    // warp would otherwise queue every warp on the same two addresses.
+    u32 idx = ~0u;
+    if (first_it != ~0u) idx = (((((warp << NSAT_IT) | first_it) << 5) | lane) << 5) | first_bit;
+    idx = __reduce_min_sync(~0u, idx);
+    cnt = __reduce_add_sync(~0u, cnt);
+    if (lane == 0 && cnt != 0u) {
+        atomicMin(&s_idx, idx);
+        atomicAdd(&s_cnt, cnt);
     }
-    idx = warp_min_u64(idx);
-    cnt = __reduce_add_sync(0xffffffffu, cnt);
-    if constexpr (NSAT_NT == 32) {
-        if (lane == 0 && cnt != 0u) {
-            atomicAdd(&out->count, (u64)cnt);
-            atomicMin(&out->min_idx, idx);
-        }
-    } else {
-        // one pair of atomics per CTA: launches with few iterations per warp
-        // would otherwise queue every warp on the same two addresses
-        // (a CTA counts at most 2^(10+IT+WB) <= 2^25 solutions)
-        constexpr int NW = NSAT_NT / 32;
-        __shared__ u64 s_idx[NW];
-        __shared__ u32 s_cnt[NW];
-        if (lane == 0) { s_idx[warp] = idx; s_cnt[warp] = cnt; }
-        __syncthreads();
-        if (warp == 0) {
-            u64 ci = lane < (u32)NW ? s_idx[lane] : ~0ull;
-            u32 cc = lane < (u32)NW ? s_cnt[lane] : 0u;
-            ci = warp_min_u64(ci);
-            cc = __reduce_add_sync(0xffffffffu, cc);
-            if (lane == 0 && cc != 0u) {
-                atomicAdd(&out->count, (u64)cc);
-                atomicMin(&out->min_idx, ci);
-            }
-        }
+    __syncthreads();
+    if (threadIdx.x == 0 && s_cnt != 0u) {
+        atomicAdd(&out->count, (u64)s_cnt);
+        atomicMin(&out->min_idx, ((u64)cta << (10 + NSAT_IT + NSAT_WB)) | s_idx);
     }
-    nsat_finish(out, host);
+    nsat_finish(out, host, seq);
 }
 #endif
 
@@ -268,7 +286,8 @@ __device__ __forceinline__ void chunk_value(u32 c, u32 v, u32* nodes, LaunchOut*
 // launch has a CTA for every chunk (the claims' code would cost a small
 // circuit a third of its compile time).
 extern "C" __global__ void NSAT_BOUNDS
-nsat_qsat(u64 launch, LaunchOut* out, LaunchOut* host, u32* nodes, const u32* __restrict__ data) {
+nsat_qsat(u64 launch, LaunchOut* out, u64* host, u32 seq, u32* nodes, const u32* __restrict__ data) {
+    nsat_begin(out);
     constexpr int M = NSAT_M;
     // Folding.  When levels 0..9 (the word and the warp tile) and the lowest
     // FOLD iteration levels all carry level 0's quantifier and lie below the
@@ -298,19 +317,19 @@ nsat_qsat(u64 launch, LaunchOut* out, LaunchOut* host, u32* nodes, const u32* __
     if (threadIdx.x == 0) ahead = atomicAdd(&out->values, 1u);
 #endif
     for (;;) {
-        // launch-relative index of the first item of this warp's range
-        const u64 warp_base = (((u64)cta << NSAT_WB) | warp) << (10 + NSAT_IT);
+        // index within the chunk (at most 25 bits) of this warp's first item
+        const u32 warp_base = warp << (10 + NSAT_IT);
         u32 x[NSAT_NIN];
 #if !NSAT_DATA
         nsat_inputs_fixed(x, lane, warp, cta, launch);
 #endif
-        u64 cand = ~0ull;      // lowest decisive unit seen by this thread (launch-relative)
+        u32 cand = ~0u;        // lowest decisive unit seen by this thread (within the chunk)
         u32 acc1 = 0, acc2 = 0;
         u32 yacc = LOW_ALL ? 0xffffffffu : 0u;
         NSAT_UNROLL
         for (u32 it = 0; it < (1u << NSAT_IT); it++) {
 #if NSAT_DATA
-            const u64 gw = ((u64)launch << (NSAT_C - 5)) + ((warp_base + ((u64)it << 10)) >> 5) + lane;
+            const u64 gw = ((u64)launch << (NSAT_C - 5)) + ((u64)cta << (NSAT_LC - 5)) + ((warp_base + (it << 10)) >> 5) + lane;
             u32 y = data[gw];
 #else
             nsat_inputs_iter(x, it);
@@ -325,13 +344,13 @@ nsat_qsat(u64 launch, LaunchOut* out, LaunchOut* host, u32* nodes, const u32* __
                 b = LOW_ALL ? (u32)__all_sync(0xffffffffu, v) : (u32)__any_sync(0xffffffffu, v);
                 git = it >> FOLD;
             } else {
-                const u64 tile_base = warp_base + ((u64)it << 10);   // first item of this warp tile
+                const u32 tile_base = warp_base + (it << 10);   // first item of this warp tile
                 // stage 0: the 32 lanes of the word (levels 0..4)
                 if constexpr (M < 5) {
                     y = tree_up<0, M>(y);
                     const u32 d = decisive(y, M, 32);
-                    if (d != 0u && cand == ~0ull)
-                        cand = ((tile_base + ((u64)lane << 5)) >> M) + (u64)((__ffs(d) - 1) >> M);
+                    if (d != 0u && cand == ~0u)
+                        cand = ((tile_base + (lane << 5)) >> M) + ((u32)(__ffs(d) - 1) >> M);
                     continue;
                 } else {
                     y = tree_up<0, 5>(y);
@@ -341,8 +360,8 @@ nsat_qsat(u64 launch, LaunchOut* out, LaunchOut* host, u32* nodes, const u32* __
                 if constexpr (M >= 5 && M < 10) {
                     b = tree_up<5, M - 5>(b);
                     const u32 d = decisive(b, M - 5, 32);
-                    if (d != 0u && cand == ~0ull)
-                        cand = (tile_base >> M) + (u64)((__ffs(d) - 1) >> (M - 5));
+                    if (d != 0u && cand == ~0u)
+                        cand = (tile_base >> M) + ((u32)(__ffs(d) - 1) >> (M - 5));
                     continue;
                 } else {
                     b = tree_up<5, 5>(b);
@@ -354,12 +373,12 @@ nsat_qsat(u64 launch, LaunchOut* out, LaunchOut* host, u32* nodes, const u32* __
                 const u32 pos = git & ((1u << G1) - 1u);
                 acc1 |= (b & 1u) << pos;
                 if (pos == (1u << G1) - 1u) {
-                    const u64 grp_base = warp_base + ((u64)(git - pos) << L0);
+                    const u32 grp_base = warp_base + ((git - pos) << L0);
                     if constexpr (M < L0 + G1) {
                         const u32 y1 = tree_up<L0, M - L0>(acc1);
                         const u32 d = decisive(y1, M - L0, 1 << G1);
-                        if (d != 0u && cand == ~0ull)
-                            cand = (grp_base >> M) + (u64)((__ffs(d) - 1) >> (M - L0));
+                        if (d != 0u && cand == ~0u)
+                            cand = (grp_base >> M) + ((u32)(__ffs(d) - 1) >> (M - L0));
                     } else {
                         const u32 y1 = tree_up<L0, G1>(acc1);
                         acc2 |= (y1 & 1u) << (git >> G1);
@@ -376,8 +395,8 @@ nsat_qsat(u64 launch, LaunchOut* out, LaunchOut* host, u32* nodes, const u32* __
             if constexpr (M < L0 + IT2) {
                 const u32 y2 = tree_up<L0 + G1, M - L0 - G1>(acc2);
                 const u32 d = decisive(y2, M - L0 - G1, 1 << G2);
-                if (d != 0u && cand == ~0ull)
-                    cand = (warp_base >> M) + (u64)((__ffs(d) - 1) >> (M - L0 - G1));
+                if (d != 0u && cand == ~0u)
+                    cand = (warp_base >> M) + ((u32)(__ffs(d) - 1) >> (M - L0 - G1));
             } else {
                 wres = tree_up<L0 + G1, G2>(acc2) & 1u;
             }
@@ -385,8 +404,10 @@ nsat_qsat(u64 launch, LaunchOut* out, LaunchOut* host, u32* nodes, const u32* __
             wres = acc2 & 1u;
         }
         // per-warp lowest candidate, one atomic per warp
-        cand = warp_min_u64(cand);
-        if (lane == 0 && cand != ~0ull) atomicMin(&out->min_idx, cand);
+        if constexpr (M < 10 + NSAT_IT) {
+            cand = __reduce_min_sync(0xffffffffu, cand);
+            if (lane == 0 && cand != ~0u) atomicMin(&out->min_idx, ((u64)cta << (NSAT_LC - M)) + cand);
+        }
         // stage 3: warps of the CTA (levels 10+IT .. 10+IT+WB-1); its value goes to
         // the tree above the chunks
         if constexpr (M >= 10 + NSAT_IT) {
@@ -454,7 +475,7 @@ nsat_qsat(u64 launch, LaunchOut* out, LaunchOut* host, u32* nodes, const u32* __
         for (u32 i = threadIdx.x; i < (make_blocks().nodes + 1u) / 2u; i += NSAT_NT) nodes[i] = 0u;
         if (threadIdx.x == 0) {
             out->values = 0u;
-            nsat_publish(out, host);
+            nsat_publish(out, host, seq);
         }
     }
 }
@@ -466,22 +487,40 @@ nsat_qsat(u64 launch, LaunchOut* out, LaunchOut* host, u32* nodes, const u32* __
 // One thread evaluates 32 states bit-sliced, then transposes the 32x32 bit
 // matrix (rows = outputs, columns = lanes) into per-state entries.
 
+// Block-swap transposition of a 32x32 bit matrix: after the step for size j,
+// rows k and k+j have exchanged their off-diagonal j x j blocks.  Sizes 16 and
+// 8 are byte permutations.  As asm blocks of 16 rows: written as loops, it was
+// two fifths of a small circuit's compile (46 of 114 ms).
+#define NSAT_SWAP16(A, B) \
+    "prmt.b32 t, %" #A ", %" #B ", 0x5410;\n\tprmt.b32 %" #B ", %" #A ", %" #B ", 0x7632;\n\tmov.b32 %" #A ", t;\n\t"
+#define NSAT_SWAP8(A, B) \
+    "prmt.b32 t, %" #A ", %" #B ", 0x6240;\n\tprmt.b32 %" #B ", %" #A ", %" #B ", 0x7351;\n\tmov.b32 %" #A ", t;\n\t"
+// rows A, B <- A & M | (B << J) & ~M, (A >> J) & M | B & ~M
+#define NSAT_SWAP(A, B, J, M) \
+    "shl.b32 t, %" #B ", " #J ";\n\tshr.b32 s, %" #A ", " #J ";\n\t" \
+    "lop3.b32 %" #A ", %" #A ", t, " #M ", 0xe4;\n\tlop3.b32 %" #B ", s, %" #B ", " #M ", 0xe4;\n\t"
+#define NSAT_STEP(S, a, b, c, d, e, f, g, h, i, j, k, l, m, n, o, p) \
+    S(a, b) S(c, d) S(e, f) S(g, h) S(i, j) S(k, l) S(m, n) S(o, p)
+#define NSAT_SWAP4(A, B) NSAT_SWAP(A, B, 4, 0x0f0f0f0f)
+#define NSAT_SWAP2(A, B) NSAT_SWAP(A, B, 2, 0x33333333)
+#define NSAT_SWAP1(A, B) NSAT_SWAP(A, B, 1, 0x55555555)
+#define NSAT_ROWS(A, k, B, l)                                                                                      \
+    "+r"(A[k]), "+r"(A[k + 1]), "+r"(A[k + 2]), "+r"(A[k + 3]), "+r"(A[k + 4]), "+r"(A[k + 5]), "+r"(A[k + 6]),     \
+        "+r"(A[k + 7]), "+r"(B[l]), "+r"(B[l + 1]), "+r"(B[l + 2]), "+r"(B[l + 3]), "+r"(B[l + 4]), "+r"(B[l + 5]), \
+        "+r"(B[l + 6]), "+r"(B[l + 7])
+
 __device__ __forceinline__ void transpose32(u32* a) {
-    // block-swap transpose: after the step for size j, row k and row k+j
-    // exchange their off-diagonal j x j blocks
 #pragma unroll
-    for (int j = 16; j > 0; j >>= 1) {
-        const u32 m = j == 16 ? 0x0000ffffu : j == 8 ? 0x00ff00ffu : j == 4 ? 0x0f0f0f0fu
-                    : j == 2 ? 0x33333333u : 0x55555555u;
+    for (int k = 0; k < 16; k += 8)
+        asm("{ .reg .b32 t;\n\t"
+            NSAT_STEP(NSAT_SWAP16, 0, 8, 1, 9, 2, 10, 3, 11, 4, 12, 5, 13, 6, 14, 7, 15) "}" : NSAT_ROWS(a, k, a, k + 16));
 #pragma unroll
-        for (int k = 0; k < 32; k++) {
-            if ((k & j) == 0) {
-                const u32 t = ((a[k] >> j) ^ a[k + j]) & m;
-                a[k + j] ^= t;
-                a[k] ^= t << j;
-            }
-        }
-    }
+    for (int k = 0; k < 32; k += 16)
+        asm("{ .reg .b32 s, t;\n\t"
+            NSAT_STEP(NSAT_SWAP8, 0, 8, 1, 9, 2, 10, 3, 11, 4, 12, 5, 13, 6, 14, 7, 15)
+            NSAT_STEP(NSAT_SWAP4, 0, 4, 1, 5, 2, 6, 3, 7, 8, 12, 9, 13, 10, 14, 11, 15)
+            NSAT_STEP(NSAT_SWAP2, 0, 2, 1, 3, 4, 6, 5, 7, 8, 10, 9, 11, 12, 14, 13, 15)
+            NSAT_STEP(NSAT_SWAP1, 0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15) "}" : NSAT_ROWS(a, k, a, k + 8));
 }
 
 // Tables of 32-bit entries of 2^10 states and more are whole warps of words:
@@ -491,7 +530,8 @@ __device__ __forceinline__ void transpose32(u32* a) {
 constexpr bool NSAT_STAGED = NSAT_FMT == 0 && NSAT_NB >= 10;
 
 extern "C" __global__ void NSAT_BOUNDS
-nsat_table(u64 nwords, u64 w0, void* __restrict__ table, LaunchOut* out, LaunchOut* host) {
+nsat_table(u64 nwords, u64 w0, void* __restrict__ table, LaunchOut* out, u64* host, u32 seq) {
+    nsat_begin(out);
     // entries of words w0 .. w0+nwords-1 (32 states each), stored from table[0]
     const u64 stride = (u64)gridDim.x * NSAT_NT;
     u32 anystop = 0;
@@ -541,6 +581,6 @@ nsat_table(u64 nwords, u64 w0, void* __restrict__ table, LaunchOut* out, LaunchO
 #endif
     }
     if (__any_sync(0xffffffffu, anystop != 0u) && (threadIdx.x & 31u) == 0) atomicOr(&out->any, 1u);
-    nsat_finish(out, host);
+    nsat_finish(out, host, seq);
 }
 #endif

@@ -35,6 +35,12 @@ void ctx_free(nsat_ctx* ctx, void* p);
 // The context's device state of a SATOSTOP solve and its pinned host copy.
 void ctx_stop_state(nsat_ctx* ctx, NsatStopState** dev, NsatStopState** host);
 cudaEvent_t ctx_stop_event(nsat_ctx* ctx);
+// A short kernel that reports in up to 5 words of pinned memory, each with the
+// launch's number (ctx_next_seq) in its upper half; ctx_poll_words waits for
+// the first `words`.
+uint32_t ctx_next_seq(nsat_ctx* ctx);
+volatile uint64_t* ctx_words(nsat_ctx* ctx);
+int ctx_poll_words(nsat_ctx* ctx, int words);
 // A pair of timing events of the context, for one interval at a time.
 void ctx_timing_events(nsat_ctx* ctx, cudaEvent_t* begin, cudaEvent_t* end);
 // Bytes that the pool holds and no buffer uses.

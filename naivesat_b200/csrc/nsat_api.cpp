@@ -11,6 +11,7 @@
 #include <chrono>
 #include <cstdio>
 #include <cstdlib>
+#include <cmath>
 #include <cstring>
 #include <map>
 #include <memory>
@@ -41,8 +42,27 @@ struct LaunchOut {
     uint32_t ticket;
     uint32_t any;
     uint32_t values;
+    uint32_t t0;
+    uint32_t pad;
 };
-static_assert(sizeof(LaunchOut) == 32, "LaunchOut layout");
+static_assert(sizeof(LaunchOut) == 40, "LaunchOut layout");
+
+// A launch's result in pinned memory: 32 bits and the launch's number in each
+// word (nsat_publish).
+constexpr int kWords = 5;
+struct HostOut {
+    volatile uint64_t word[kWords];
+    uint64_t pad[3];
+    bool there(uint32_t seq, int words = kWords) const {
+        for (int i = 0; i < words; i++)
+            if ((uint32_t)(word[i] >> 32) != seq) return false;
+        return true;
+    }
+    uint32_t half(int i) const { return (uint32_t)word[i]; }
+    uint64_t lowest() const { return (uint64_t)half(1) << 32 | half(0); }
+    uint64_t value() const { return (uint64_t)half(3) << 32 | half(2); }
+    double ms() const { return half(4) * 1e-6; }
+};
 
 constexpr uint64_t kReadStage = 64 * 1024;
 constexpr int kRing = 4;   // launches in flight before the host reads results
@@ -59,10 +79,12 @@ struct nsat_ctx {
     cudaStream_t stream = nullptr;
     int sm_count = 0;
     std::string last_err;
+    std::shared_ptr<CUstream_st> stream_life;   // owns stream
     char* d_fixed = nullptr;          // the device allocation behind d_out, d_join and d_stop
     char* h_fixed = nullptr;          // the pinned one behind h_out, h_join and h_stop
     LaunchOut* d_out = nullptr;       // kRing slots, put back to their first state by each launch
-    LaunchOut* h_out = nullptr;       // pinned: a launch's last CTA writes its result here
+    HostOut* h_out = nullptr;         // pinned: a launch's last CTA writes its result here
+    uint32_t seq = 0;                 // the last launch's number
     cudaEvent_t ev0[kRing]{}, ev1[kRing]{}, evd = nullptr;
     unsigned char* d_scratch = nullptr;
     size_t scratch_bytes = 0;
@@ -127,6 +149,7 @@ struct SatMemo {
     uint32_t chunk_bits = 0;
     u128 begin = 0, end = 0;
     Shape shape;
+    uint32_t lop3 = 0;
     SatPlan plan;
     CUfunction fn = nullptr;
     std::shared_ptr<JitModule> mod;
@@ -137,6 +160,7 @@ struct QsatMemo {
     std::vector<uint8_t> quants;
     Shape shape;
     QsatPlan plan;
+    uint32_t lop3 = 0;
     unsigned grid = 0;           // resident CTAs, at most one per chunk
     CUfunction fn = nullptr;
     std::shared_ptr<JitModule> mod;
@@ -160,6 +184,16 @@ struct nsat_circuit {
     SatMemo sat_memo;
     QsatMemo qsat_memo;
     TableMemo table_memo[2];     // by entry format
+    // stream of the last solve whose result was polled for: its kernel may
+    // still be returning when the solve does
+    std::weak_ptr<CUstream_st> polled;
+    ~nsat_circuit() { polled_on(nullptr); }
+    // Notes that a solve on st will be polled for (null: none).
+    void polled_on(const std::shared_ptr<CUstream_st>& st) {
+        if (std::shared_ptr<CUstream_st> last = polled.lock())
+            if (last != st) cudaStreamSynchronize(last.get());
+        polled = st;
+    }
 };
 
 struct nsat_table {
@@ -405,6 +439,40 @@ uint64_t reverse_bits(uint64_t v, uint32_t bits) {
     return r;
 }
 
+// Short launches.  Two timing events and the wait for the second take 11 us of
+// a small solve (18.4 us against 7.5 us for an empty launch that is polled
+// for), so a solve of one launch that is estimated at less than 0.25 ms polls
+// its words in pinned memory, and the kernel times itself by the global timer:
+// there the events would be 4 % or more.  When the words are there, all that
+// the kernel writes is written; its CTAs may still be returning.  Later work
+// follows in stream order, and a circuit waits before it lets its kernels go.
+bool short_launch(uint32_t log2_assignments, uint32_t lop3) {
+    return std::ldexp((double)lop3 + 32.0, (int)log2_assignments - 5) < 0.25e-3 * kCompiledLutWordsPerS;
+}
+
+uint32_t next_seq(nsat_ctx* ctx) { return ctx->seq = ctx->seq + 1 ? ctx->seq + 1 : 1; }
+
+// Waits until the first words of h carry the current number: by polling, and
+// after 2 ms for the stream (another process may have the GPU, or the launch
+// failed).
+int poll_out(nsat_ctx* ctx, const HostOut& h, int words = kWords) {
+    const double until = now_ms() + 2.0;
+    for (uint32_t spin = 1; !h.there(ctx->seq, words); spin++) {
+        if ((spin & 63) || now_ms() < until) continue;
+        CK(cudaStreamSynchronize(ctx->stream));
+        if (!h.there(ctx->seq, words)) return fail(ctx, NSAT_ECUDA, "a launch left no result");
+    }
+    return NSAT_OK;
+}
+
+// Where a launch reports.
+struct Report {
+    LaunchOut* out;
+    HostOut* host;
+    uint32_t seq;
+    Report(nsat_ctx* ctx, int slot) : out(ctx->d_out + slot), host(ctx->h_out + slot), seq(next_seq(ctx)) {}
+};
+
 // Runs a sequence of launches of one kernel with a ring of result slots:
 // `issue(k, slot)` enqueues launch k, `consume(k, out, ms)` sees its result and
 // returns false to stop issuing.  Device time is the sum of the per-launch
@@ -412,13 +480,22 @@ uint64_t reverse_bits(uint64_t v, uint32_t bits) {
 // `claim(k, slot)`, when given, is asked before launch k is prepared and
 // returns false when there is nothing more to issue (a shared chunk queue ran
 // out); launches already issued are still consumed.
+// `polled`: there is one launch and it is short (short_launch).
 struct ClaimAll {
     bool operator()(uint64_t, int) const { return true; }
 };
 
 template <typename Issue, typename Consume, typename Claim = ClaimAll>
-int run_ring(nsat_ctx* ctx, uint64_t total, Issue issue, Consume consume, double* dev_ms,
+int run_ring(nsat_ctx* ctx, uint64_t total, bool polled, Issue issue, Consume consume, double* dev_ms,
              uint32_t* launches, Claim claim = Claim()) {
+    if (polled) {
+        if (int rc = issue(0, 0)) return rc;
+        if (int rc = poll_out(ctx, ctx->h_out[0])) return rc;
+        *dev_ms = ctx->h_out[0].ms();
+        *launches = 1;
+        consume(0, ctx->h_out[0]);
+        return NSAT_OK;
+    }
     uint64_t issued = 0, done = 0;
     bool stop = false;
     *dev_ms = 0;
@@ -619,6 +696,7 @@ extern "C" int nsat_create(int device, const nsat_opts* opts, nsat_ctx** out) {
     CK(cudaFree(nullptr));
     CK(cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device));
     CK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
+    ctx->stream_life = std::shared_ptr<CUstream_st>(ctx->stream, [](cudaStream_t st) { cudaStreamDestroy(st); });
     cudaMemPoolProps pp{};
     pp.allocType = cudaMemAllocationTypePinned;
     pp.handleTypes = cudaMemHandleTypeNone;
@@ -630,25 +708,26 @@ extern "C" int nsat_create(int device, const nsat_opts* opts, nsat_ctx** out) {
     // the small fixed buffers in one allocation each: page-locking is the
     // slowest part of creating a context, and a server creates a dozen
     constexpr size_t kOut = 256, kJoin = 1024, kStop = 512;
-    static_assert(sizeof(LaunchOut) * kRing <= kOut && sizeof(NsatJoinState) <= kJoin && sizeof(NsatStopState) <= kStop,
+    static_assert(sizeof(HostOut) * kRing <= kOut && sizeof(LaunchOut) * kRing <= kOut && sizeof(NsatJoinState) <= kJoin && sizeof(NsatStopState) <= kStop,
                   "fixed buffer sizes");
     CK(cudaMalloc(&ctx->d_fixed, kOut + kJoin + kStop));
     CK(cudaMallocHost(&ctx->h_fixed, kOut + kJoin + kStop));
     ctx->d_out = (LaunchOut*)ctx->d_fixed;
     ctx->d_join = (NsatJoinState*)(ctx->d_fixed + kOut);
     ctx->d_stop = (NsatStopState*)(ctx->d_fixed + kOut + kJoin);
-    ctx->h_out = (LaunchOut*)ctx->h_fixed;
+    ctx->h_out = (HostOut*)ctx->h_fixed;
     ctx->h_join = (NsatJoinState*)(ctx->h_fixed + kOut);
     ctx->h_stop = (NsatStopState*)(ctx->h_fixed + kOut + kJoin);
-    memset(ctx->h_out, 0, sizeof(LaunchOut) * kRing);
+    memset(ctx->h_fixed, 0, kOut);
+    LaunchOut* clean = (LaunchOut*)ctx->h_fixed;
     for (int i = 0; i < kRing; i++) {
-        ctx->h_out[i].min_idx = ~0ull;
+        clean[i].min_idx = ~0ull;
         CK(cudaEventCreate(&ctx->ev0[i]));
         CK(cudaEventCreate(&ctx->ev1[i]));
     }
     CK(cudaEventCreateWithFlags(&ctx->evd, cudaEventDisableTiming));
     // in order before every launch, whose results are the next writes of h_out
-    CK(cudaMemcpyAsync(ctx->d_out, ctx->h_out, sizeof(LaunchOut) * kRing, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(ctx->d_out, clean, sizeof(LaunchOut) * kRing, cudaMemcpyHostToDevice, ctx->stream));
     std::string err;
     if (!driver_api(&err)) return NSAT_ECUDA;
     *out = c.release();
@@ -669,7 +748,7 @@ extern "C" void nsat_destroy(nsat_ctx* ctx) {
     cudaFreeHost(ctx->h_read);
     cudaFree(ctx->d_scratch);
     cudaFree(ctx->d_data);
-    if (ctx->stream) cudaStreamDestroy(ctx->stream);
+    ctx->stream_life.reset();
     if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     delete ctx;
 }
@@ -784,6 +863,7 @@ extern "C" int nsat_sat_solve(nsat_ctx* ctx, nsat_circuit* c, const nsat_sat_opt
         if (int rc = plan_sat(c->circ.n, o, shape, &memo.plan, &perr, (uint32_t)net.luts.size()))
             return fail(ctx, rc, perr);
         if (int rc = get_circuit_kernel(ctx, c, out0, memo.plan.kc, net, "nsat_sat", &memo.fn, &memo.mod)) return rc;
+        memo.lop3 = (uint32_t)net.luts.size();
         memo.chunk_bits = o.chunk_bits;
         memo.begin = o_begin;
         memo.end = o_end;
@@ -804,23 +884,24 @@ extern "C" int nsat_sat_solve(nsat_ctx* ctx, nsat_circuit* c, const nsat_sat_opt
     uint64_t consumed = 0;
     double dev_ms = 0;
     uint32_t launches = 0;
-    uint64_t launch_idx_buf[kRing];
     uint64_t chunk_of_slot[kRing];
     nsat_sat_share* share = o.find_all ? nullptr : o.share;
+    const bool polled = !share && nl == 1 && short_launch(C, memo.lop3);
+    if (polled) c->polled_on(ctx->stream_life);
     int rc = run_ring(
-        ctx, nl,
+        ctx, nl, polled,
         [&](uint64_t k, int slot) {
-            launch_idx_buf[slot] = L0 + (share ? chunk_of_slot[slot] : k);
-            LaunchOut *po = ctx->d_out + slot, *ph = ctx->h_out + slot;
-            void* params[] = {&launch_idx_buf[slot], &po, &ph};
+            uint64_t index = L0 + (share ? chunk_of_slot[slot] : k);
+            Report to(ctx, slot);
+            void* params[] = {&index, &to.out, &to.host, &to.seq};
             return launch(ctx, fn, grid, threads, params);
         },
-        [&](uint64_t k, const LaunchOut& r) {
+        [&](uint64_t k, const HostOut& r) {
             const uint64_t chunk = share ? chunk_of_slot[k % kRing] : k;
             consumed++;
-            count += r.count;
-            if (r.min_idx != ~0ull) {
-                const u128 w = (((u128)(L0 + chunk)) << C) + r.min_idx;
+            count += r.value();
+            if (r.lowest() != ~0ull) {
+                const u128 w = (((u128)(L0 + chunk)) << C) + r.lowest();
                 if (!found || w < witness) witness = w;
                 found = true;
                 if (share) {
@@ -924,6 +1005,7 @@ int qsat_common(nsat_ctx* ctx, nsat_circuit* c, const std::vector<uint8_t>& quan
         memo.grid = kc.cb <= kResidentBits
                         ? 1u << kc.cb
                         : (unsigned)std::min<uint64_t>(1ull << kc.cb, (uint64_t)per_sm * ctx->sm_count);
+        memo.lop3 = (uint32_t)net->luts.size();
         memo.chunk_bits = chunk_bits;
         memo.prefix_bits = prefix_bits;
         memo.quants = quants_in;
@@ -962,25 +1044,27 @@ int qsat_common(nsat_ctx* ctx, nsat_circuit* c, const std::vector<uint8_t>& quan
     bool have = false;
     uint64_t nl = prefix_count > 1 ? prefix_count : (A == 64 ? ~0ull : (1ull << A));
     const unsigned grid = memo.grid, threads = kc.threads();
-    uint64_t launch_idx_buf[kRing];
     unsigned char* scratch = fixed_scratch ? fixed_scratch : ctx->d_scratch;
     const uint32_t* dd = ctx->d_data;
     double dev_ms = 0;
     uint32_t launches = 0;
+    // (a data reduction's kernel is let go when this returns)
+    const bool polled = !data && nl == 1 && short_launch(C, memo.lop3);
+    if (polled) c->polled_on(ctx->stream_life);
     int rc = run_ring(
-        ctx, nl,
+        ctx, nl, polled,
         [&](uint64_t k, int slot) {
-            launch_idx_buf[slot] = L0 + k;
-            LaunchOut *po = ctx->d_out + slot, *ph = ctx->h_out + slot;
-            void* params[] = {&launch_idx_buf[slot], &po, &ph, &scratch, &dd};
+            uint64_t index = L0 + k;
+            Report to(ctx, slot);
+            void* params[] = {&index, &to.out, &to.host, &to.seq, &scratch, &dd};
             return launch(ctx, fn, grid, threads, params);
         },
-        [&](uint64_t k, const LaunchOut& r) {
+        [&](uint64_t k, const HostOut& r) {
             if (A == 0) {
                 fr.reversed = q0all;
                 fr.solution_bits = f;
-                fr.has_solution = r.min_idx != ~0ull;
-                fr.solution = fr.has_solution ? reverse_bits(r.min_idx, f) : 0;
+                fr.has_solution = r.lowest() != ~0ull;
+                fr.solution = fr.has_solution ? reverse_bits(r.lowest(), f) : 0;
                 have = true;
                 if (prefix_count > 1) {
                     nsat_qsat_result b{};
@@ -994,8 +1078,8 @@ int qsat_common(nsat_ctx* ctx, nsat_circuit* c, const std::vector<uint8_t>& quan
                 return false;
             }
             bool value;
-            if (m < C) value = (r.min_idx != ~0ull) ? dec : !dec;
-            else value = r.tree != 0;
+            if (m < C) value = (r.lowest() != ~0ull) ? dec : !dec;
+            else value = r.value() != 0;
             qr->push(value);
             FinalResult t;
             if (qr->final_result(&t)) {
@@ -1003,7 +1087,7 @@ int qsat_common(nsat_ctx* ctx, nsat_circuit* c, const std::vector<uint8_t>& quan
                 fr.solution_bits = f;
                 fr.has_solution = t.has_solution;
                 if (t.has_solution && f > A)
-                    fr.solution = t.solution | (reverse_bits(r.min_idx, f - A) << A);
+                    fr.solution = t.solution | (reverse_bits(r.lowest(), f - A) << A);
                 else
                     fr.solution = t.has_solution ? t.solution : 0;
                 have = true;
@@ -1071,6 +1155,9 @@ void nsat::ctx_stop_state(nsat_ctx* ctx, NsatStopState** dev, NsatStopState** ho
     *host = ctx->h_stop;
 }
 cudaEvent_t nsat::ctx_stop_event(nsat_ctx* ctx) { return ctx->evd; }
+uint32_t nsat::ctx_next_seq(nsat_ctx* ctx) { return next_seq(ctx); }
+volatile uint64_t* nsat::ctx_words(nsat_ctx* ctx) { return ctx->h_out[0].word; }
+int nsat::ctx_poll_words(nsat_ctx* ctx, int words) { return poll_out(ctx, ctx->h_out[0], words); }
 void nsat::ctx_timing_events(nsat_ctx* ctx, cudaEvent_t* begin, cudaEvent_t* end) {
     *begin = ctx->ev0[0];
     *end = ctx->ev1[0];
@@ -1150,18 +1237,26 @@ extern "C" int nsat_stop_table_build(nsat_ctx* ctx, nsat_circuit* c, const nsat_
     const unsigned threads = memo.threads;
     uint64_t want = (nwords + threads - 1) / threads;
     unsigned grid = (unsigned)std::min<uint64_t>(want, (uint64_t)ctx->sm_count * 16);
-    LaunchOut *po = ctx->d_out, *ph = ctx->h_out;
     void* tb = t->buf[0];
     uint64_t w0 = 0;
-    void* params[] = {&nwords, &w0, &tb, &po, &ph};
-    CK(cudaEventRecord(ctx->ev0[0], ctx->stream));
+    // up to 2^20 entries the kernel takes less than the events
+    const bool polled = n <= 20;
+    if (polled) c->polled_on(ctx->stream_life);
+    Report to(ctx, 0);
+    void* params[] = {&nwords, &w0, &tb, &to.out, &to.host, &to.seq};
+    if (!polled) CK(cudaEventRecord(ctx->ev0[0], ctx->stream));
     if (int rc = launch(ctx, memo.fn, grid, threads, params)) return rc;
-    CK(cudaEventRecord(ctx->ev1[0], ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    float ms = 0;
-    CK(cudaEventElapsedTime(&ms, ctx->ev0[0], ctx->ev1[0]));
-    t->build_ms = ms;
-    t->any_stop = ctx->h_out[0].any != 0;
+    if (polled) {
+        if (int rc = poll_out(ctx, *to.host)) return rc;
+        t->build_ms = to.host->ms();
+    } else {
+        CK(cudaEventRecord(ctx->ev1[0], ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        float ms = 0;
+        CK(cudaEventElapsedTime(&ms, ctx->ev0[0], ctx->ev1[0]));
+        t->build_ms = ms;
+    }
+    t->any_stop = to.host->value() != 0;
     t->cur = 0;
     *out = t.release();
     return NSAT_OK;
@@ -1185,15 +1280,15 @@ int table_chunk(nsat_ctx* ctx, nsat_circuit* c, uint64_t first_state, uint64_t c
     const unsigned threads = memo.threads;
     const uint64_t want = (nwords + threads - 1) / threads;
     const unsigned grid = (unsigned)std::min<uint64_t>(want, (uint64_t)ctx->sm_count * 16);
-    LaunchOut *po = ctx->d_out, *ph = ctx->h_out;
+    Report to(ctx, 0);
     void* tb = dev_out;
-    void* params[] = {&nwords, &w0, &tb, &po, &ph};
+    void* params[] = {&nwords, &w0, &tb, &to.out, &to.host, &to.seq};
     CK(cudaEventRecord(ctx->ev0[0], ctx->stream));
     if (int rc = launch(ctx, memo.fn, grid, threads, params)) return rc;
     CK(cudaEventRecord(ctx->ev1[0], ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     if (ms) CK(cudaEventElapsedTime(ms, ctx->ev0[0], ctx->ev1[0]));
-    if (any_stop) *any_stop = ctx->h_out[0].any != 0;
+    if (any_stop) *any_stop = to.host->value() != 0;
     return NSAT_OK;
 }
 
@@ -1220,7 +1315,10 @@ extern "C" int nsat_table_read(nsat_table* t, uint64_t first, uint64_t count, ui
         CK(cudaStreamSynchronize(ctx->stream));
         for (uint64_t i = 0; i < count; i++)
             out[i] = t->narrow ? ((const uint32_t*)ctx->h_read)[i] : ((const uint64_t*)ctx->h_read)[i] & mask;
-    } else if (t->narrow) {
+        return NSAT_OK;
+    }
+    CK(cudaStreamSynchronize(ctx->stream));      // the copies below are on another stream
+    if (t->narrow) {
         std::vector<uint32_t> tmp(count);
         CK(cudaMemcpy(tmp.data(), src, count * 4, cudaMemcpyDeviceToHost));
         for (uint64_t i = 0; i < count; i++) out[i] = tmp[i];
@@ -1247,6 +1345,7 @@ extern "C" int nsat_stop_solve(nsat_ctx* ctx, nsat_table* t, const nsat_stop_opt
         x.unknowns = opts->unknowns;
         x.mode = opts->mode;
         x.steps = t->steps;
+        x.begin = ctx->ev0[0];
         x.done = ctx->ev1[0];
         if (t->steps) {       // both 32-bit tables share buffer 0; buffer 1 takes the 64-bit result
             x.a = (uint32_t*)t->buf[0];
@@ -1256,11 +1355,14 @@ extern "C" int nsat_stop_solve(nsat_ctx* ctx, nsat_table* t, const nsat_stop_opt
             x.a = (uint32_t*)t->buf[t->cur];
             x.b = (uint32_t*)t->buf[t->cur ^ 1];
         }
-        CK(cudaEventRecord(ctx->ev0[0], ctx->stream));
         const int rc = stop_run(ctx, &x);
         if (rc == NSAT_OK) {
-            CK(cudaEventElapsedTime(&ms, ctx->ev0[0], ctx->ev1[0]));
-            res->join_ms = ms;
+            if (x.polled) {
+                res->join_ms = x.ms;
+            } else {
+                CK(cudaEventElapsedTime(&ms, ctx->ev0[0], ctx->ev1[0]));
+                res->join_ms = ms;
+            }
             res->rounds = x.rounds;
             if (t->steps) {
                 t->narrow = false;

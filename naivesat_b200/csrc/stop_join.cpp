@@ -89,18 +89,21 @@ int stop_run(nsat_ctx* ctx, StopRun* x) {
     x->launches = 0;
     bool answered = false;
     if (n <= NSAT_STOP_SMALL_BITS && n > 0) {
-        // the state goes to pinned host memory straight from the kernel
-        JRUN(nsat_stop_small(x->a, n, u, mode, x->steps, x->steps ? nullptr : x->b, x->out64, h, st));
-        if (x->done) JCK(cudaEventRecord(x->done, st));
-        JCK(cudaStreamSynchronize(st));
-        x->rounds = h->final_round;
+        const uint32_t seq = ctx_next_seq(ctx);
+        const volatile uint64_t* w = ctx_words(ctx);
+        JRUN(nsat_stop_small(x->a, n, u, mode, x->steps, x->steps ? nullptr : x->b, x->out64, (uint64_t*)w, seq, st));
+        if (int rc = ctx_poll_words(ctx, 5)) return rc;
+        x->polled = true;
+        x->rounds = (uint32_t)w[0];
         x->table = x->b;
-        x->found = h->best[x->rounds] != ~0u;
-        x->start = h->best[x->rounds];
-        x->entry = h->entry;
-        x->steps_of = h->dist;
+        x->start = (uint32_t)w[1];
+        x->found = x->start != ~0u;
+        x->entry = (uint32_t)w[2];
+        x->steps_of = (uint32_t)w[3];
+        x->ms = (uint32_t)w[4] * 1e-6;
         return NSAT_OK;
     }
+    if (x->begin) JCK(cudaEventRecord(x->begin, st));
     Scratch mem(ctx);
     uint32_t* dist = x->steps ? x->dist : nullptr;
     if (x->steps && !dist && !mem.get(&dist, N)) return NSAT_ENOMEM;

@@ -14,7 +14,8 @@ struct StopRun {
     uint32_t* b = nullptr;
     bool steps = false;            // distances wanted
     uint32_t* dist = nullptr;      // steps: 2^n words, or null to take them from the context's pool
-    cudaEvent_t done = nullptr;    // recorded behind the last kernel (null: not wanted)
+    cudaEvent_t begin = nullptr;   // recorded before the first kernel (null: not wanted)
+    cudaEvent_t done = nullptr;    // and behind the last
     uint64_t* out64 = nullptr;     // steps: the 64-bit table after the last round (null: not wanted)
     // out
     uint32_t rounds = 0;
@@ -22,6 +23,8 @@ struct StopRun {
     uint32_t start = 0, entry = 0, steps_of = 0;   // entry: halting state | STOP << n
     uint32_t* table = nullptr;     // a or b: the table after the last round (not written when out64 was)
     uint32_t launches = 0;
+    bool polled = false;           // one short kernel: no events, its own time is in ms
+    double ms = 0;
 };
 
 // Runs the rounds on the context's stream and waits for the answer.

@@ -131,9 +131,11 @@ constexpr int kSmallThreads = 1024;
 template <bool STEPS, int E>
 __global__ void __launch_bounds__(kSmallThreads) small_solve(const u32* __restrict__ src, u32 n, u32 u, u32 mode,
                                                              u32* __restrict__ out32, u64* __restrict__ out64,
-                                                             NsatStopState* __restrict__ st) {
+                                                             volatile u64* words, u32 seq) {
     extern __shared__ u32 sm[];
     __shared__ u32 s_best;        // lowest start that has stopped so far
+    u32 t0;
+    asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t0));
     const u32 N = 1u << n, stop = N, smask = (1u << (n - u)) - 1u;
     u32* table = sm;
     u32* dist = sm + N;
@@ -187,15 +189,21 @@ __global__ void __launch_bounds__(kSmallThreads) small_solve(const u32* __restri
             out32[i] = v[k];
         }
     }
+    __syncthreads();
     if (tid == 0) {
-        st->final_round = r;
-        st->best[r] = best;
-        st->entry = best != kNone ? table[best] : 0u;
-        st->dist = STEPS && best != kNone ? dist[best] : 0u;
+        __threadfence();          // the host may go on when it sees the words
+        u32 t1;
+        asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t1));
+        const u64 number = (u64)seq << 32;
+        words[0] = number | r;
+        words[1] = number | best;
+        words[2] = number | (best != kNone ? table[best] : 0u);
+        words[3] = number | (STEPS && best != kNone ? dist[best] : 0u);
+        words[4] = number | (t1 - t0);
     }
 }
 
-typedef void (*SmallKernel)(const u32*, u32, u32, u32, u32*, u64*, NsatStopState*);
+typedef void (*SmallKernel)(const u32*, u32, u32, u32, u32*, u64*, volatile u64*, u32);
 template <bool STEPS>
 SmallKernel small_kernel(u32 n) {
     switch (n) {
@@ -487,7 +495,7 @@ extern "C" int nsat_stop_join(const uint32_t* src, uint32_t* dst, uint32_t* dist
 }
 
 extern "C" int nsat_stop_small(const uint32_t* src, uint32_t n, uint32_t u, uint32_t mode, int steps,
-                               uint32_t* out32, uint64_t* out64, NsatStopState* st, cudaStream_t s) {
+                               uint32_t* out32, uint64_t* out64, uint64_t* words, uint32_t seq, cudaStream_t s) {
     if (n > NSAT_STOP_SMALL_BITS) return -1;
     const size_t smem = ((size_t)(steps ? 8 : 4)) << n;
     const SmallKernel fn = steps ? small_kernel<true>(n) : small_kernel<false>(n);
@@ -496,7 +504,7 @@ extern "C" int nsat_stop_small(const uint32_t* src, uint32_t n, uint32_t u, uint
     if (smem >= 48 * 1024 && cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  8 << NSAT_STOP_SMALL_BITS) != cudaSuccess)
         return -4;
-    fn<<<1, kSmallThreads, smem, s>>>(src, n, u, mode, out32, (u64*)out64, st);
+    fn<<<1, kSmallThreads, smem, s>>>(src, n, u, mode, out32, (u64*)out64, (volatile u64*)words, seq);
     return ok();
 }
 

@@ -13,7 +13,7 @@ typedef struct {
     uint32_t final_round;     // round whose answer ended the loop early (0 = none)
     uint32_t distinct;        // sampled distinct successors (see the sample of nsat_stop_join)
     uint32_t count;           // distinct successors (nsat_stop_rank)
-    uint32_t entry, dist;     // nsat_stop_small: the answer's entry and distance
+    uint32_t entry, dist;     // the answer's entry and distance
     uint32_t pad[3];
 } NsatStopState;
 
@@ -29,9 +29,11 @@ int nsat_stop_join(const uint32_t* src, uint32_t* dst, uint32_t* dist, uint32_t 
                    uint32_t mode, NsatStopState* st, uint32_t* sample, int sms, cudaStream_t s);
 // Every round of a table of n <= NSAT_STOP_SMALL_BITS bits, with distances
 // when steps is set; out32 or (with steps) out64, where not null, receive the
-// table after the last one.
+// table after the last one.  words (pinned host memory, 5) receive the
+// rounds run, the lowest start (~0: none), its entry, its distance and the
+// kernel's time in ns, each under seq << 32.
 int nsat_stop_small(const uint32_t* src, uint32_t n, uint32_t u, uint32_t mode, int steps, uint32_t* out32,
-                    uint64_t* out64, NsatStopState* st, cudaStream_t s);
+                    uint64_t* out64, uint64_t* words, uint32_t seq, cudaStream_t s);
 
 // Contraction to the states that a later round can still look up.
 // marks in bits (cleared, items bits) the successors of items entries, unless

@@ -1,0 +1,69 @@
+"""Short launches, whose results the host polls for: past the wrap of the
+launch number, mixed with launches timed by events, at the sizes around the
+lines between the two, and with handles freed straight after a solve."""
+import numpy as np
+import pytest
+
+from naivesat_b200 import workloads as W
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def oc(c):
+    return O.Circuit(c.n, c.gates, c.outputs)
+
+
+def test_launch_numbers_wrap(ctx):
+    a, b = W.random_dag(61, 11, 40, output="live"), W.planted_dag(62, 13, 80, plant_bits=7)
+    q = "AE" * 10
+    qc = W.random_dag(63, 20, 60, output="live")
+    s = W.lfsr_stop(64, 10, 60)
+    want = [O.sat_range(oc(a)), O.sat_range(oc(b))]
+    ha, hb, hq, hs = (ctx.circuit(x) for x in (a, b, qc, s))
+    events = hq.qsat(q, chunk_bits=15)          # several launches: timed by events
+    table = O.stop_table(oc(s)).astype(np.uint64)
+    first = hs.stop_table(want_steps=True).solve(10, mode=1)
+    for i in range(16500):                       # four launches each
+        for h, (cnt, low) in ((ha, want[0]), (hb, want[1])):
+            r = h.sat(find_all=True)
+            assert (r["count"], r["witness"]) == (cnt, low)
+        if i % 1500:
+            r = hq.qsat(q)
+            assert (r["value"], r["solution_bits"]) == (events["value"], events["solution_bits"])
+            continue
+        assert hb.sat(find_all=True, chunk_bits=10)["count"] == want[1][0]
+        t = hs.stop_table(want_steps=True)
+        assert (t.read() == table).all()
+        r = t.solve(10, mode=1)
+        assert [r.get(k) for k in ("found", "start", "end", "steps", "rounds")] == \
+               [first.get(k) for k in ("found", "start", "end", "steps", "rounds")]
+        assert r["build_ms"] < 1.0 and r["join_ms"] < 2.2
+
+
+@pytest.mark.parametrize("n,gates", [(10, 20), (15, 60), (24, 3000), (28, 60), (28, 700), (29, 300), (31, 40), (32, 40)])
+def test_both_sides_of_the_line(ctx, n, gates):
+    c = W.random_dag(n * 1000 + gates, n, gates, output="live")
+    q = ("AEE" * n)[:n]
+    for _ in range(2):
+        h = ctx.circuit(c)
+        one = h.sat(find_all=True)
+        halves = [h.sat(find_all=True, begin=k << (n - 1), end=(k + 1) << (n - 1), chunk_bits=min(n - 1, 24))
+                  for k in range(2)] if n > 10 else [one, {"count": 0, "satisfiable": False}]
+        assert one["count"] == sum(r["count"] for r in halves)
+        low = [r["witness"] for r in halves if r["satisfiable"]]
+        assert one["satisfiable"] == bool(low) and (not low or one["witness"] == low[0])
+        a = h.qsat(q)
+        h.close()                                # its kernel may still be returning
+        b = ctx.circuit(c).qsat(q, chunk_bits=min(n, max(15, n - 5)))
+        assert [a[k] for k in ("value", "solution")] == [b[k] for k in ("value", "solution")]
+
+
+@pytest.mark.parametrize("n", [2, 5, 14, 15, 20, 21])
+def test_table_builds(ctx, n):
+    c = W.counter_stop(n)
+    want = O.stop_table(oc(c)).astype(np.uint64)
+    for steps in (False, True):
+        t = ctx.circuit(c).stop_table(want_steps=steps)
+        assert (t.read() == want).all()
+        t.solve(n, mode=1)
