@@ -28,16 +28,16 @@ typedef unsigned long long u64;
 // LUTs of one asm block without barriers, and where the evaluators use blocks:
 // from 400 LUTs (the compiler's sharing between iterations is worth more
 // below: 24 inputs, 280 LUTs, run 139 instructions a word), for searches of up
-// to 0.1 s.  Blocks compile a 2000-3000-gate circuit 70-120 ms faster and run
+// to 2 ms.  Blocks compile a 2000-3000-gate circuit 70-120 ms faster and run
 // 0.1-0.9 % slower (33 inputs, 1216 LUTs: first solve 476 -> 350 ms, device
-// time 17.74 -> 17.76 ms).
+// time 17.74 -> 17.76 ms): longer searches keep the faster loop.
 constexpr uint32_t kBlockLuts = 128;
 constexpr size_t kBlocksFrom = 400;
 bool use_blocks(const KernelConfig& kc, const LutNet& net) {
     if (kc.mode == Mode::TABLE) return true;
     if (net.luts.size() < kBlocksFrom) return false;
     return kc.mode == Mode::QSAT ||
-           std::ldexp((double)net.luts.size(), (int)kc.nb - 5) < 0.1 * kCompiledLutWordsPerS;
+           std::ldexp((double)net.luts.size(), (int)kc.nb - 5) < 2e-3 * kCompiledLutWordsPerS;
 }
 
 const uint32_t kLanePat[5] = {0xAAAAAAAAu, 0xCCCCCCCCu, 0xF0F0F0F0u, 0xFF00FF00u, 0xFFFF0000u};
@@ -156,6 +156,79 @@ void emit_luts(std::ostringstream& s, const LutNet& net, bool blocks, uint32_t s
     s.write(b.data(), (std::streamsize)b.size());
 }
 
+// Iterations evaluated together: 2^inner copies of the LUTs that depend on the
+// iteration's lowest inner bits (own), beside one of the rest (shared).
+// In each copy those bits are constants, which fold into its LUTs and, under
+// quantifiers, into the node trees; a copy that folds to a constant costs
+// nothing, as half of the copies do for each bit that a conjunction tests.
+struct Parts {
+    uint32_t inner = 0;
+    LutNet shared, own;
+    std::vector<uint32_t> cross;     // shared wires that the copies (or the output) read
+};
+
+// inner is the largest (up to 4) whose code stays within a budget, which is
+// about what the compiler's own unrolling took: 2400 LUTs or two copies for
+// SAT, 640 (a quantifier tree's share of a copy counted as 40) or little more
+// than one copy for QSAT, whose calls are shorter.  Device time in us and first
+// call in ms, left to the compiler and now: SAT 81 LUTs, 32 inputs 395, 76 and
+// 116, 70; 201 LUTs, 33 inputs 2993, 102 and 1384, 73; 652 LUTs, 30 inputs
+// 1190, 198 and 1147, 108.  QSAT 14 LUTs, 30 inputs 61, 90 and 33, 100; 339
+// LUTs, 26 inputs 41, 121 and 34, 122.
+constexpr uint32_t kMostInner = 4;
+Parts split(const KernelConfig& kc, const LutNet& net) {
+    const bool sat = kc.mode == Mode::SAT;
+    const size_t n = net.luts.size();
+    uint32_t wires = kc.nin;
+    for (const Lut& l : net.luts) wires = std::max(wires, l.wire + 1);
+    for (const Output& o : net.outs) wires = std::max(wires, o.wire + 1);
+    // the lowest iteration bit that a wire depends on
+    std::vector<uint8_t> lowest(wires, kMostInner);
+    const uint32_t most = std::min(kc.it, kMostInner);
+    for (uint32_t k = most; k-- > 0;)
+        if (kc.in_of_bit[10 + k] >= 0) lowest[kc.in_of_bit[10 + k]] = (uint8_t)k;
+    size_t own[kMostInner + 1] = {};     // LUTs whose lowest bit is k
+    for (const Lut& l : net.luts) {
+        lowest[l.wire] = std::min({lowest[l.in[0]], lowest[l.in[1]], lowest[l.in[2]]});
+        own[lowest[l.wire]]++;
+    }
+    Parts p;
+    const size_t budget = sat ? std::max<size_t>(2400, 2 * n + 16) : std::max<size_t>(640, n + n / 8 + 80);
+    size_t copied = 0;
+    for (uint32_t k = 1; k <= most; k++) {
+        copied += own[k - 1];
+        if (n - copied + ((copied + (sat ? 8 : 40)) << k) <= budget) p.inner = k;
+    }
+    if (!p.inner) {
+        p.own = net;
+        return p;
+    }
+    std::vector<uint8_t> seen(wires, 0);     // 1: in cross or used_inputs of own, 2: of shared
+    const auto is_own = [&](uint32_t w) { return lowest[w] < p.inner; };
+    const auto own_reads = [&](uint32_t w) {
+        if (seen[w] & 1) return;
+        seen[w] |= 1;
+        if (w < kc.nin) p.own.used_inputs.push_back(w);
+        else if (!is_own(w)) p.cross.push_back(w);
+    };
+    for (const Lut& l : net.luts) {
+        const bool mine = is_own(l.wire);
+        (mine ? p.own : p.shared).luts.push_back(l);
+        for (const uint32_t w : l.in) {
+            if (mine) {
+                own_reads(w);
+            } else if (w < kc.nin && !(seen[w] & 2)) {
+                seen[w] |= 2;
+                p.shared.used_inputs.push_back(w);
+            }
+        }
+    }
+    for (const Output& o : net.outs) own_reads(o.wire);
+    for (const uint32_t w : p.cross) p.shared.outs.push_back(Output{w, false});
+    p.own.outs = net.outs;
+    return p;
+}
+
 }  // namespace
 
 std::string generate_source(const KernelConfig& kc, const LutNet& net) {
@@ -181,11 +254,10 @@ std::string generate_source(const KernelConfig& kc, const LutNet& net) {
     s << "constexpr int NSAT_Q0ALL = " << (kc.q0all ? 1 : 0) << ";\n";
     s << "constexpr u64 NSAT_ALLBITS = " << kc.allbits << "ull;\n";
 
-    // few iterations of a large evaluation are not unrolled: four copies of 665
-    // LUTs doubled the compile time and gained nothing; the loop of a 38-LUT
-    // adder is (244 us against 351 us)
     s << "#define NSAT_ONE " << (kc.cb <= kResidentBits ? 1 : 0) << "\n";
-    s << "#define NSAT_UNROLL " << (net.luts.size() > 64 ? "_Pragma(\"unroll 1\")" : "") << "\n";
+    const Parts parts = kc.mode == Mode::TABLE || kc.data ? Parts() : split(kc, net);
+    s << "#define NSAT_INNER " << parts.inner << "\n";
+    s << "constexpr int NSAT_SHARED = " << std::max<size_t>(1, parts.cross.size()) << ";\n";
 
     // enumeration: which circuit input each bit drives
     const uint32_t it_lo = 10, wb_lo = 10 + kc.it, cb_lo = wb_lo + kc.wb, c_lo = cb_lo + kc.cb;
@@ -223,25 +295,30 @@ std::string generate_source(const KernelConfig& kc, const LutNet& net) {
 
     // circuit evaluation
     if (kc.mode == Mode::TABLE) {
-        s << "__device__ __forceinline__ void nsat_eval1(const u32* x) {}\n";
         s << "__device__ __forceinline__ void nsat_eval_all(const u32* x, u32* o) {\n";
         emit_luts(s, net, use_blocks(kc, net));
         for (size_t j = 0; j < net.outs.size(); j++)
             s << "    o[" << j << "] = " << (net.outs[j].neg ? "~" : "") << "w" << net.outs[j].wire << ";\n";
         s << "}\n";
     } else {
-        s << "__device__ __forceinline__ u32 nsat_eval1(const u32* x) {\n";
+        // the SAT and QSAT kernels run the same number of evaluations in every
+        // thread of a CTA, so barriers inside the evaluation are safe
+        const uint32_t sync = kc.threads() > 32 ? kc.sync_every : 0;
+        const bool blocks = use_blocks(kc, net);
+        s << "__device__ __forceinline__ void nsat_shared(const u32* x, u32* sh) {\n";
+        emit_luts(s, parts.shared, blocks, sync);
+        for (size_t k = 0; k < parts.cross.size(); k++) s << "    sh[" << k << "] = w" << parts.cross[k] << ";\n";
+        s << "}\n";
+        s << "__device__ __forceinline__ u32 nsat_eval1(const u32* x, const u32* sh) {\n";
         if (!kc.data) {
-            // the SAT and QSAT kernels run the same number of evaluations in
-            // every thread of a CTA, so barriers inside the evaluation are safe
-            const bool uniform = kc.mode == Mode::SAT || kc.mode == Mode::QSAT;
-            emit_luts(s, net, use_blocks(kc, net), uniform && kc.threads() > 32 ? kc.sync_every : 0);
+            for (size_t k = 0; k < parts.cross.size(); k++)
+                s << "    const u32 w" << parts.cross[k] << " = sh[" << k << "];\n";
+            emit_luts(s, parts.own, blocks, sync);
             s << "    return " << (net.outs[0].neg ? "~" : "") << "w" << net.outs[0].wire << ";\n";
         } else {
             s << "    return 0u;\n";
         }
         s << "}\n";
-        s << "__device__ __forceinline__ void nsat_eval_all(const u32* x, u32* o) {}\n";
     }
     s << kDeviceTemplate;
     return s.str();

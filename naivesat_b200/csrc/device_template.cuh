@@ -4,8 +4,8 @@
 //   constexpr ints NSAT_NIN, NSAT_NOUT, NSAT_NB (enumeration bits), NSAT_NT
 //   (threads per CTA), NSAT_IT / NSAT_WB / NSAT_CB (log2 of iterations per
 //   warp, warps per CTA and CTAs per launch; QSAT: chunks per launch),
-//   NSAT_ONE (QSAT: a CTA per chunk), NSAT_UNROLL (a pragma for the loop over
-//   iterations), NSAT_BOUNDS (the kernels'
+//   NSAT_ONE (QSAT: a CTA per chunk), NSAT_INNER (log2 of iterations
+//   evaluated together, at most IT), NSAT_BOUNDS (the kernels'
 //   __launch_bounds__), NSAT_C (= 10+IT+WB+CB, log2 of
 //   assignments per launch), NSAT_M (QSAT unit level), NSAT_Q0ALL,
 //   NSAT_ALLBITS (bit j = quantifier of enumeration bit j is All),
@@ -14,7 +14,8 @@
 // and the generated device functions
 //   nsat_inputs_fixed(x, lane, warp, cta, launch)  -- inputs that stay fixed
 //   nsat_inputs_iter(x, it)                        -- inputs that follow `it`
-//   nsat_eval1(x) -> u32          output 0 as a 32-lane word
+//   nsat_shared(x, sh)            what 2^NSAT_INNER iterations share
+//   nsat_eval1(x, sh) -> u32      output 0 as a 32-lane word
 //   nsat_eval_all(x, o)           all outputs (table mode)
 //   nsat_inputs_word(x, w)        inputs of word index w (table mode)
 //
@@ -125,11 +126,19 @@ nsat_sat(u64 launch, LaunchOut* out, u64* host, u32 seq) {
     nsat_inputs_fixed(x, lane, warp, cta, launch);
     u32 cnt = 0;
     u32 first_it = 0xffffffffu, first_bit = 0;
-    for (u32 it = 0; it < (1u << NSAT_IT); it++) {
-        nsat_inputs_iter(x, it);
-        const u32 y = nsat_eval1(x);
-        cnt += __popc(y);
-        if (y != 0u && first_it == 0xffffffffu) { first_it = it; first_bit = __ffs(y) - 1; }
+#pragma unroll 1
+    for (u32 outer = 0; outer < (1u << NSAT_IT); outer += 1u << NSAT_INNER) {
+        u32 sh[NSAT_SHARED];
+        nsat_inputs_iter(x, outer);
+        nsat_shared(x, sh);
+#pragma unroll
+        for (u32 inner = 0; inner < (1u << NSAT_INNER); inner++) {
+            const u32 it = outer | inner;
+            nsat_inputs_iter(x, it);
+            const u32 y = nsat_eval1(x, sh);
+            cnt += __popc(y);
+            if (y != 0u && first_it == 0xffffffffu) { first_it = it; first_bit = __ffs(y) - 1; }
+        }
     }
     // index within the CTA: 10 + IT + WB <= 25 bits, and at most 2^25 solutions
     // to count.  One pair of atomics per CTA: launches with few iterations per
@@ -326,14 +335,22 @@ nsat_qsat(u64 launch, LaunchOut* out, u64* host, u32 seq, u32* nodes, const u32*
         u32 cand = ~0u;        // lowest decisive unit seen by this thread (within the chunk)
         u32 acc1 = 0, acc2 = 0;
         u32 yacc = LOW_ALL ? 0xffffffffu : 0u;
-        NSAT_UNROLL
-        for (u32 it = 0; it < (1u << NSAT_IT); it++) {
+#pragma unroll 1
+        for (u32 outer = 0; outer < (1u << NSAT_IT); outer += 1u << NSAT_INNER) {
+#if !NSAT_DATA
+        u32 sh[NSAT_SHARED];
+        nsat_inputs_iter(x, outer);
+        nsat_shared(x, sh);
+#endif
+#pragma unroll
+        for (u32 inner = 0; inner < (1u << NSAT_INNER); inner++) {
+            const u32 it = outer | inner;
 #if NSAT_DATA
             const u64 gw = ((u64)launch << (NSAT_C - 5)) + ((u64)cta << (NSAT_LC - 5)) + ((warp_base + (it << 10)) >> 5) + lane;
             u32 y = data[gw];
 #else
             nsat_inputs_iter(x, it);
-            u32 y = nsat_eval1(x);
+            u32 y = nsat_eval1(x, sh);
 #endif
             u32 b, git;   // node value at level L0 (bit 0) and its index among the warp's L0 nodes
             if constexpr (FOLDED) {
@@ -388,6 +405,7 @@ nsat_qsat(u64 launch, LaunchOut* out, u64* host, u32 seq, u32* nodes, const u32*
             } else if constexpr (M >= L0) {
                 acc2 = b & 1u;   // IT2 == 0: one L0 node is the warp's whole range
             }
+        }
         }
         // stage 2b: groups of L0 nodes (levels L0+G1 .. 10+IT-1)
         u32 wres = 0;
