@@ -35,6 +35,7 @@ void ctx_free(nsat_ctx* ctx, void* p);
 // The context's device state of a SATOSTOP solve and its pinned host copy.
 void ctx_stop_state(nsat_ctx* ctx, NsatStopState** dev, NsatStopState** host);
 cudaEvent_t ctx_stop_event(nsat_ctx* ctx);
+NsatGridState* ctx_grid_state(nsat_ctx* ctx);
 // A short kernel that reports in up to 5 words of pinned memory, each with the
 // launch's number (ctx_next_seq) in its upper half; ctx_poll_words waits for
 // the first `words`.

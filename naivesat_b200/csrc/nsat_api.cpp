@@ -93,6 +93,7 @@ struct nsat_ctx {
     NsatJoinState* d_join = nullptr;
     NsatJoinState* h_join = nullptr;
     NsatStopState* d_stop = nullptr;
+    NsatGridState* d_grid = nullptr;  // put back to its first state by each solve
     NsatStopState* h_stop = nullptr;
     void* h_read = nullptr;           // pinned, kReadStage bytes (nsat_table_read)
     // loaded kernels by everything their generated source depends on (the
@@ -707,14 +708,15 @@ extern "C" int nsat_create(int device, const nsat_opts* opts, nsat_ctx** out) {
     CK(cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep));
     // the small fixed buffers in one allocation each: page-locking is the
     // slowest part of creating a context, and a server creates a dozen
-    constexpr size_t kOut = 256, kJoin = 1024, kStop = 512;
+    constexpr size_t kOut = 256, kJoin = 1024, kStop = 512, kGrid = 128;
     static_assert(sizeof(HostOut) * kRing <= kOut && sizeof(LaunchOut) * kRing <= kOut && sizeof(NsatJoinState) <= kJoin && sizeof(NsatStopState) <= kStop,
                   "fixed buffer sizes");
-    CK(cudaMalloc(&ctx->d_fixed, kOut + kJoin + kStop));
+    CK(cudaMalloc(&ctx->d_fixed, kOut + kJoin + kStop + kGrid));
     CK(cudaMallocHost(&ctx->h_fixed, kOut + kJoin + kStop));
     ctx->d_out = (LaunchOut*)ctx->d_fixed;
     ctx->d_join = (NsatJoinState*)(ctx->d_fixed + kOut);
     ctx->d_stop = (NsatStopState*)(ctx->d_fixed + kOut + kJoin);
+    ctx->d_grid = (NsatGridState*)(ctx->d_fixed + kOut + kJoin + kStop);
     ctx->h_out = (HostOut*)ctx->h_fixed;
     ctx->h_join = (NsatJoinState*)(ctx->h_fixed + kOut);
     ctx->h_stop = (NsatStopState*)(ctx->h_fixed + kOut + kJoin);
@@ -728,6 +730,9 @@ extern "C" int nsat_create(int device, const nsat_opts* opts, nsat_ctx** out) {
     CK(cudaEventCreateWithFlags(&ctx->evd, cudaEventDisableTiming));
     // in order before every launch, whose results are the next writes of h_out
     CK(cudaMemcpyAsync(ctx->d_out, clean, sizeof(LaunchOut) * kRing, cudaMemcpyHostToDevice, ctx->stream));
+    static_assert(sizeof(NsatGridState) <= kGrid, "fixed buffer sizes");
+    CK(cudaMemsetAsync(ctx->d_grid, 0, kGrid, ctx->stream));
+    CK(cudaMemsetAsync(ctx->d_grid, 0xff, sizeof(ctx->d_grid->best), ctx->stream));
     std::string err;
     if (!driver_api(&err)) return NSAT_ECUDA;
     *out = c.release();
@@ -1155,6 +1160,7 @@ void nsat::ctx_stop_state(nsat_ctx* ctx, NsatStopState** dev, NsatStopState** ho
     *host = ctx->h_stop;
 }
 cudaEvent_t nsat::ctx_stop_event(nsat_ctx* ctx) { return ctx->evd; }
+NsatGridState* nsat::ctx_grid_state(nsat_ctx* ctx) { return ctx->d_grid; }
 uint32_t nsat::ctx_next_seq(nsat_ctx* ctx) { return next_seq(ctx); }
 volatile uint64_t* nsat::ctx_words(nsat_ctx* ctx) { return ctx->h_out[0].word; }
 int nsat::ctx_poll_words(nsat_ctx* ctx, int words) { return poll_out(ctx, ctx->h_out[0], words); }

@@ -64,6 +64,20 @@ struct Scratch {
     }
 };
 
+// The words of nsat_stop_small and nsat_stop_grid.
+int polled_answer(nsat_ctx* ctx, StopRun* x) {
+    if (int rc = ctx_poll_words(ctx, 5)) return rc;
+    const volatile uint64_t* w = ctx_words(ctx);
+    x->polled = true;
+    x->rounds = (uint32_t)w[0];
+    x->start = (uint32_t)w[1];
+    x->found = x->start != ~0u;
+    x->entry = (uint32_t)w[2];
+    x->steps_of = (uint32_t)w[3];
+    x->ms = (uint32_t)w[4] * 1e-6;
+    return NSAT_OK;
+}
+
 }  // namespace
 
 #define JCK(call)                                                                              \
@@ -90,23 +104,29 @@ int stop_run(nsat_ctx* ctx, StopRun* x) {
     bool answered = false;
     if (n <= NSAT_STOP_SMALL_BITS && n > 0) {
         const uint32_t seq = ctx_next_seq(ctx);
-        const volatile uint64_t* w = ctx_words(ctx);
-        JRUN(nsat_stop_small(x->a, n, u, mode, x->steps, x->steps ? nullptr : x->b, x->out64, (uint64_t*)w, seq, st));
-        if (int rc = ctx_poll_words(ctx, 5)) return rc;
-        x->polled = true;
-        x->rounds = (uint32_t)w[0];
+        JRUN(nsat_stop_small(x->a, n, u, mode, x->steps, x->steps ? nullptr : x->b, x->out64,
+                             (uint64_t*)ctx_words(ctx), seq, st));
+        if (int rc = polled_answer(ctx, x)) return rc;
         x->table = x->b;
-        x->start = (uint32_t)w[1];
-        x->found = x->start != ~0u;
-        x->entry = (uint32_t)w[2];
-        x->steps_of = (uint32_t)w[3];
-        x->ms = (uint32_t)w[4] * 1e-6;
         return NSAT_OK;
     }
-    if (x->begin) JCK(cudaEventRecord(x->begin, st));
     Scratch mem(ctx);
     uint32_t* dist = x->steps ? x->dist : nullptr;
     if (x->steps && !dist && !mem.get(&dist, N)) return NSAT_ENOMEM;
+    if (n > NSAT_STOP_SMALL_BITS && n <= NSAT_STOP_GRID_BITS) {
+        const uint32_t seq = ctx_next_seq(ctx);
+        const int rc = nsat_stop_grid(x->a, x->b, dist, n, u, mode, x->steps, x->out64, ctx_grid_state(ctx),
+                                      (uint64_t*)ctx_words(ctx), seq, st);
+        if (rc < 0) return ctx_fail(ctx, NSAT_ECUDA, "doubling launch failed");
+        if (rc == 0) {
+            x->launches++;
+            if (int e = polled_answer(ctx, x)) return e;
+            if (x->rounds == ~0u) return ctx_fail(ctx, NSAT_ECUDA, "the doubling's grid barrier gave up");
+            x->table = (x->rounds & 1) ? x->b : x->a;
+            return NSAT_OK;
+        }
+    }
+    if (x->begin) JCK(cudaEventRecord(x->begin, st));
     memset(h, 0, sizeof(*h));
     memset(h->best, 0xff, sizeof(h->best));
     JCK(cudaMemcpyAsync(d, h, sizeof(*h), cudaMemcpyHostToDevice, st));

@@ -30,7 +30,13 @@
 //
 // - tables of up to 2^14 entries run every round in one CTA with the table in
 //   shared memory (2^12 entries with distances, 12 rounds: 53 us as launches,
-//   24 us).
+//   24 us);
+//
+// - and tables of up to 2^20 in one cooperative launch with a grid barrier per
+//   round: a launch per round costs 3 us, and the rounds behind the answer
+//   were launched too (a solve answered after 6 rounds of 2^16 entries with
+//   distances 91 -> 35 us, after 15 rounds of 2^15 without 86 -> 55 us, after
+//   5 rounds of 2^20 with 147 -> 54 us).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -212,6 +218,117 @@ SmallKernel small_kernel(u32 n) {
     case 13: return small_solve<STEPS, 8>;
     case 14: return small_solve<STEPS, 16>;
     default: return small_solve<STEPS, 1>;     // up to 2^10 entries
+    }
+}
+
+// All rounds of a table of 2^15 .. 2^20 entries in one cooperative launch of
+// N / (1024 E) CTAs: a thread keeps its E entries in registers, a round
+// gathers from one buffer, writes the other and ends in a grid barrier.  The
+// buffers and distances change while the kernel runs, so they are read through
+// the L2.  The barrier counts arrivals up; its spin is bounded, and a CTA that
+// gives up lets the others go too.  The last CTA to end reports as small_solve
+// does (rounds ~0: given up) and leaves the state as it was.
+constexpr u32 kGridThreads = 1024;
+constexpr u32 kSpinLimit = 1u << 22;
+
+template <bool STEPS, int E>
+__global__ void __launch_bounds__(kGridThreads) grid_solve(u32* a, u32* b, u32* dist, u32 n, u32 u, u32 mode,
+                                                           u64* __restrict__ out64, NsatGridState* st,
+                                                           volatile u64* words, u32 seq) {
+    __shared__ u32 s_best, s_round;      // lowest start in this CTA, lowest of all after the round
+    __shared__ bool s_failed;
+    const u32 tid = threadIdx.x, S = gridDim.x * kGridThreads, i0 = blockIdx.x * kGridThreads + tid;
+    const u32 stop = 1u << n, smask = (1u << (n - u)) - 1u;
+    if (tid == 0) {
+        s_best = kNone;
+        if (blockIdx.x == 0) asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(*(volatile u32*)&st->t0));
+    }
+    __syncthreads();
+    u32 v[E], d[E];
+#pragma unroll
+    for (int k = 0; k < E; k++) {
+        const u32 i = i0 + k * S;
+        v[k] = __ldcg(a + i);
+        d[k] = 1u;
+        if (STEPS && (v[k] & stop)) __stcg(dist + i, 1u);
+    }
+    u32 *src = a, *dst = b;
+    u32 r = 1, best = kNone;
+    bool failed = false;
+    for (;; r++) {
+        u32 w[E], low = kNone;
+#pragma unroll
+        for (int k = 0; k < E; k++) w[k] = (v[k] & stop) ? v[k] : __ldcg(src + v[k]);
+#pragma unroll
+        for (int k = 0; k < E; k++) {
+            const u32 i = i0 + k * S;
+            if constexpr (STEPS) {
+                if ((w[k] & ~v[k]) & stop) {
+                    // dist[v] belongs to an entry that stopped before this round
+                    d[k] = (1u << (r - 1)) + (r == 1 ? 1u : __ldcg(dist + v[k]));
+                    __stcg(dist + i, d[k]);
+                }
+            }
+            __stcg(dst + i, w[k]);
+            if ((w[k] & stop) && (i & smask) == 0u) low = min(low, i);
+            v[k] = w[k];
+        }
+        low = __reduce_min_sync(0xffffffffu, low);
+        if ((tid & 31u) == 0 && low != kNone) atomicMin(&s_best, low);
+        __syncthreads();
+        if (tid == 0) {
+            if (s_best != kNone) atomicMin(&st->best[r], s_best);
+            __threadfence();
+            atomicAdd(&st->arrived, 1u);
+            const u32 all = r * gridDim.x;
+            u32 spins = 0;
+            while (*(volatile u32*)&st->arrived < all && !*(volatile u32*)&st->failed)
+                if (++spins == kSpinLimit) *(volatile u32*)&st->failed = 1u;
+            __threadfence();
+            s_failed = *(volatile u32*)&st->failed != 0u;
+            s_round = *(volatile u32*)&st->best[r];
+        }
+        __syncthreads();
+        best = s_round;
+        failed = s_failed;
+        if (failed || r == n || (best != kNone && (mode == 0 || best == 0))) break;
+        u32* t = src;
+        src = dst;
+        dst = t;
+    }
+    if (STEPS && out64) {
+#pragma unroll
+        for (int k = 0; k < E; k++) out64[i0 + k * S] = (u64)v[k] | ((u64)((v[k] & stop) ? d[k] : 1u << r) << 32);
+    }
+    __syncthreads();
+    if (tid != 0) return;
+    __threadfence();
+    if (atomicAdd(&st->ended, 1u) != gridDim.x - 1u) return;
+    __threadfence();
+    failed |= *(volatile u32*)&st->failed != 0u;
+    u32 t1;
+    asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t1));
+    const u32 t = t1 - *(volatile u32*)&st->t0;
+    for (u32 k = 0; k < sizeof(st->best) / 4; k++) st->best[k] = kNone;
+    st->arrived = 0u;
+    st->ended = 0u;
+    st->failed = 0u;
+    const u64 number = (u64)seq << 32;
+    words[0] = number | (failed ? ~0u : r);
+    words[1] = number | best;
+    words[2] = number | (best != kNone ? __ldcg(dst + best) : 0u);
+    words[3] = number | (STEPS && best != kNone ? __ldcg(dist + best) : 0u);
+    words[4] = number | t;
+}
+
+typedef void (*GridKernel)(u32*, u32*, u32*, u32, u32, u32, u64*, NsatGridState*, volatile u64*, u32);
+template <bool STEPS>
+GridKernel grid_kernel(u32 per_thread) {
+    switch (per_thread) {
+    case 1: return grid_solve<STEPS, 1>;
+    case 2: return grid_solve<STEPS, 2>;
+    case 4: return grid_solve<STEPS, 4>;
+    default: return grid_solve<STEPS, 8>;
     }
 }
 
@@ -506,6 +623,22 @@ extern "C" int nsat_stop_small(const uint32_t* src, uint32_t n, uint32_t u, uint
         return -4;
     fn<<<1, kSmallThreads, smem, s>>>(src, n, u, mode, out32, (u64*)out64, (volatile u64*)words, seq);
     return ok();
+}
+
+extern "C" int nsat_stop_grid(uint32_t* a, uint32_t* b, uint32_t* dist, uint32_t n, uint32_t u, uint32_t mode,
+                              int steps, uint64_t* out64, NsatGridState* st, uint64_t* words, uint32_t seq,
+                              cudaStream_t s) {
+    if (n <= NSAT_STOP_SMALL_BITS || n > NSAT_STOP_GRID_BITS) return -1;
+    // 128 CTAs from 2^17 entries on
+    const u32 e = n <= 17 ? 1u : 1u << (n - 17);
+    const GridKernel fn = steps ? grid_kernel<true>(e) : grid_kernel<false>(e);
+    volatile u64* w = (volatile u64*)words;
+    u64* o = (u64*)out64;
+    void* args[] = {&a, &b, &dist, &n, &u, &mode, &o, &st, &w, &seq};
+    if (cudaLaunchCooperativeKernel((const void*)fn, dim3((1u << n) / (kGridThreads * e)), dim3(kGridThreads), args, 0, s) == cudaSuccess)
+        return 0;
+    cudaGetLastError();
+    return 1;        // more CTAs than the device holds at once
 }
 
 extern "C" int nsat_stop_mark32(const uint32_t* entries, uint64_t items, uint32_t n, uint32_t* bits, uint32_t r,

@@ -7,6 +7,14 @@
 
 #define NSAT_STOP_SMALL_BITS 14     // tables of up to 2^14 entries are solved in one CTA
 
+#define NSAT_STOP_GRID_BITS 20      // up to 2^20 in one cooperative launch
+
+// Device state of nsat_stop_grid: best all ~0, the rest 0 before and after.
+typedef struct {
+    uint32_t best[28];
+    uint32_t arrived, ended, failed, t0;
+} NsatGridState;
+
 // Device state of one solve.
 typedef struct {
     uint32_t best[40];        // best[r]: lowest resolved start after round r (~0 = none)
@@ -34,6 +42,12 @@ int nsat_stop_join(const uint32_t* src, uint32_t* dst, uint32_t* dist, uint32_t 
 // kernel's time in ns, each under seq << 32.
 int nsat_stop_small(const uint32_t* src, uint32_t n, uint32_t u, uint32_t mode, int steps, uint32_t* out32,
                     uint64_t* out64, uint64_t* words, uint32_t seq, cudaStream_t s);
+
+// The same for NSAT_STOP_SMALL_BITS < n <= NSAT_STOP_GRID_BITS in one cooperative
+// launch between a (the table, also after an even number of rounds) and b.
+// dist: 2^n words, with steps.  1: the device does not hold the grid.
+int nsat_stop_grid(uint32_t* a, uint32_t* b, uint32_t* dist, uint32_t n, uint32_t u, uint32_t mode, int steps,
+                   uint64_t* out64, NsatGridState* st, uint64_t* words, uint32_t seq, cudaStream_t s);
 
 // Contraction to the states that a later round can still look up.
 // marks in bits (cleared, items bits) the successors of items entries, unless

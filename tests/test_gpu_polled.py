@@ -67,3 +67,28 @@ def test_table_builds(ctx, n):
         t = ctx.circuit(c).stop_table(want_steps=steps)
         assert (t.read() == want).all()
         t.solve(n, mode=1)
+
+
+@pytest.mark.parametrize("n", [14, 15, 16, 17, 18, 19, 20, 21])
+def test_one_launch_doubling(ctx, n):
+    """Plain rounds in numpy against the solves of one launch and, at n = 21, a
+    launch a round; twice, as each leaves the next one's state."""
+    c = W.lfsr_stop(n, n, 80)
+    table = O.stop_table(oc(c))
+    for mode in (0, 1, 0):
+        for u in (0, 3, n):
+            want = O.stop_solve(n, u, table, mode=mode)
+            for steps in (False, True):
+                t = ctx.circuit(c).stop_table(want_steps=steps)
+                r = t.solve(u, mode=mode)
+                assert r["found"] == (want is not None)
+                if want:
+                    assert (r["start"], r["end"], r["rounds"]) == (want["start"], want["end"], want["rounds"])
+                    if steps:
+                        assert r["steps"] == want["steps"]
+                # the table left behind: 2^rounds evaluations on
+                after = table.copy()
+                for _ in range(r["rounds"]):
+                    stop = (after >> np.uint64(n)) != 0
+                    after = np.where(stop, after, after[np.where(stop, 0, after).astype(np.int64)])
+                assert r["rounds"] == 0 or (t.read() == after).all()
