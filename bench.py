@@ -183,6 +183,10 @@ class SatWorkload:
                 "traffic_note": "dram bytes per launch from ncu on a 2^32 launch (instruction and "
                                 "parameter fetch only; the kernel reads no data)",
                 "peak_source": "measured lop3.b32 chain microbenchmark on this GPU (%.0f MHz)" % probe_mhz,
+                "note": "counts every mapped lop3 for every word; iterations evaluated together share the LUTs "
+                        "that their own bits do not reach, and copies in which those bits decide the output fold "
+                        "away (c1: 638 warp instructions per 32-lane word instead of 1258, ALU pipe 98 % busy), "
+                        "so frac can exceed 1",
                 "lop3_per_word": self.lop3, "live_gates": self.live}
 
     def cpu(self, threads, target_s=12.0):
@@ -237,6 +241,8 @@ class QsatWorkload:
         return {"bound": "alu", "achieved": rate, "peak": peak_lop3, "unit": "lop3/s",
                 "frac": rate / peak_lop3, "traffic": None,
                 "peak_source": "measured lop3.b32 chain microbenchmark on this GPU (%.0f MHz)" % probe_mhz,
+                "note": "counts every assignment of the launches run; what the tree has decided before it is "
+                        "reached is not evaluated, so frac can exceed 1",
                 "lop3_per_word": self.lop3, "live_gates": self.live}
 
     def cpu(self, threads, target_s=12.0):
@@ -336,7 +342,10 @@ class StopWorkload:
         ach = self.join_bytes() / (self.join_ms * 1e-3) / 1e9
         out = {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
                "traffic": None, "peak_source": "%s hbm_gbs (MEASURED_PEAKS.json)" % src,
-               "kernel": "join_round", "algorithmic_bytes_per_entry_round": 3 * self.eb,
+               "kernel": "join32, join_pq",
+               "note": "algorithmic bytes of plain rounds over the whole table; later rounds run on the image of "
+                       "the earlier ones, so frac can exceed 1",
+               "algorithmic_bytes_per_entry_round": 3 * self.eb,
                "rounds": self.rounds, "join_ms": self.join_ms, "build_ms": self.build_ms}
         # probe table of the same bytes as this table (u64 probe entries)
         out["gather_roofline"] = gather_roofline(self.ctx, self.circ.n - (1 if self.eb == 4 else 0),
@@ -406,7 +415,8 @@ class StopPartWorkload:
         r = self.last
         ach = self.join_bytes() / (r["join_ms"] * 1e-3) / 1e9
         out = {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak, "traffic": None,
-               "peak_source": "%s hbm_gbs (MEASURED_PEAKS.json)" % src, "kernel": "join_packed_kernel",
+               "peak_source": "%s hbm_gbs (MEASURED_PEAKS.json)" % src, 
+               "kernel": "join_packed_kernel" if self.spill else "chase_before, chase_after",
                "algorithmic_bytes_per_entry_join": 8 + 16 / self.P,
                "joins": r["joins"], "join_ms": r["join_ms"], "build_ms": r["build_ms"], "wall_ms": r["wall_ms"],
                "storage": ["device", "pinned host", "file"][r["storage"]]}

@@ -322,7 +322,7 @@ int nsat_greedy_image(nsat_ctx* ctx, nsat_circuit* c, uint32_t partitions, const
  * new circuit costs no compilation; jobs are admitted in arrival order while
  * their device memory fits the server's budget; every nsat_server_step runs
  * one epoch (one CUDA-graph replay) over a slice of tiles (2^15 assignments)
- * of every active job, slices doubling from one tile, and retires finished
+ * of every active job, sized by the job's work and the epoch's budget, and retires finished
  * jobs.  Answers equal the one-shot solvers': SAT the lowest witness, QSAT
  * the QuantReducer result, SATOSTOP the lowest stopping start with steps. */
 typedef struct nsat_server nsat_server;

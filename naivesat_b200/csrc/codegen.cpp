@@ -182,6 +182,8 @@ Parts split(const KernelConfig& kc, const LutNet& net) {
     uint32_t wires = kc.nin;
     for (const Lut& l : net.luts) wires = std::max(wires, l.wire + 1);
     for (const Output& o : net.outs) wires = std::max(wires, o.wire + 1);
+    std::vector<uint8_t> gate(wires, 0);     // kc.nin counts a small circuit's padding too
+    for (const Lut& l : net.luts) gate[l.wire] = 1;
     // the lowest iteration bit that a wire depends on
     std::vector<uint8_t> lowest(wires, kMostInner);
     const uint32_t most = std::min(kc.it, kMostInner);
@@ -208,7 +210,7 @@ Parts split(const KernelConfig& kc, const LutNet& net) {
     const auto own_reads = [&](uint32_t w) {
         if (seen[w] & 1) return;
         seen[w] |= 1;
-        if (w < kc.nin) p.own.used_inputs.push_back(w);
+        if (!gate[w]) p.own.used_inputs.push_back(w);
         else if (!is_own(w)) p.cross.push_back(w);
     };
     for (const Lut& l : net.luts) {
@@ -217,7 +219,7 @@ Parts split(const KernelConfig& kc, const LutNet& net) {
         for (const uint32_t w : l.in) {
             if (mine) {
                 own_reads(w);
-            } else if (w < kc.nin && !(seen[w] & 2)) {
+            } else if (!gate[w] && !(seen[w] & 2)) {
                 seen[w] |= 2;
                 p.shared.used_inputs.push_back(w);
             }

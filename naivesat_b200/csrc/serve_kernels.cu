@@ -26,8 +26,8 @@
 // computes.
 //
 // Scheduling is on the device: every warp starts at its own job of the epoch
-// table and claims tiles from the job's persistent cursor, moving on
-// round-robin when the job's slice is used up.  The search for the next job
+// table and claims parts of its slice from the job's counter of the epoch, by
+// one atomic add each, moving on round-robin when the slice is used up.  The search for the next job
 // with tiles left checks 32 jobs at a time, one per lane.  When no slice has
 // planned tiles left, warps go on into the next quarter slice of SAT and
 // SATOSTOP jobs that are not decided yet, and end when none has tiles left

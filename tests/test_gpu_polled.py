@@ -92,3 +92,22 @@ def test_one_launch_doubling(ctx, n):
                     stop = (after >> np.uint64(n)) != 0
                     after = np.where(stop, after, after[np.where(stop, 0, after).astype(np.int64)])
                 assert r["rounds"] == 0 or (t.read() == after).all()
+
+
+@pytest.mark.parametrize("n,gates,threads", [(11, 30, 32), (14, 60, 64), (16, 90, 32), (18, 400, 64), (19, 700, 256)])
+def test_iterations_together(n, gates, threads):
+    """Fewer CTAs, so more iterations per warp, than the default shape's, padded
+    inputs included (n < 15), against the oracle."""
+    from naivesat_b200 import api
+    c = W.random_dag(n * 100 + gates, n, gates, output="live")
+    cnt, low = O.sat_range(oc(c))
+    q = ("AEEA" * n)[:n]
+    with api.Context(0, block_threads=threads) as small:
+        h = small.circuit(c)
+        want = h.qsat(q)
+        for kind, qs in (("sat", None), ("qsat", q)):
+            h.autotune(kind, quants=qs)
+        r = h.sat(find_all=True)
+        assert (r["count"], r["witness"]) == (cnt, low)
+        got = h.qsat(q)
+        assert [got[k] for k in ("value", "solution")] == [want[k] for k in ("value", "solution")]
