@@ -184,9 +184,9 @@ class SatWorkload:
                                 "parameter fetch only; the kernel reads no data)",
                 "peak_source": "measured lop3.b32 chain microbenchmark on this GPU (%.0f MHz)" % probe_mhz,
                 "note": "counts every mapped lop3 for every word; iterations evaluated together share the LUTs "
-                        "that their own bits do not reach, and copies in which those bits decide the output fold "
-                        "away (c1: 638 warp instructions per 32-lane word instead of 1258, ALU pipe 98 % busy), "
-                        "so frac can exceed 1",
+                        "that their own bits do not reach, and copies whose constant bits decide the output (a "
+                        "planted comparison) fold away before the kernel is compiled, so value and frac can "
+                        "exceed what the ALU issues",
                 "lop3_per_word": self.lop3, "live_gates": self.live}
 
     def cpu(self, threads, target_s=12.0):

@@ -157,78 +157,136 @@ void emit_luts(std::ostringstream& s, const LutNet& net, bool blocks, uint32_t s
 }
 
 // Iterations evaluated together: 2^inner copies of the LUTs that depend on the
-// iteration's lowest inner bits (own), beside one of the rest (shared).
-// In each copy those bits are constants, which fold into its LUTs and, under
-// quantifiers, into the node trees; a copy that folds to a constant costs
-// nothing, as half of the copies do for each bit that a conjunction tests.
+// iteration's lowest inner bits, beside one of the rest (shared).  In copy c
+// those bits are the constants of c, which are folded here: the compiler does
+// not fold every lop3 (36 inputs, 3018 gates, planted block: 83 or 163 ms by
+// the circuit, 7.1 ms folded here, first call 314 -> 99 ms).  A copy that folds to a constant costs nothing, as half of the copies
+// do for each bit that a conjunction tests.
 struct Parts {
     uint32_t inner = 0;
-    LutNet shared, own;
-    std::vector<uint32_t> cross;     // shared wires that the copies (or the output) read
+    LutNet shared;                       // used_inputs: of the copies too
+    std::vector<LutNet> copies;          // wires renamed; outs empty: constant
+    std::vector<uint8_t> constant;       // the output, where a copy's is constant
+    size_t luts() const {
+        size_t n = shared.luts.size();
+        for (const LutNet& c : copies) n += c.luts.size();
+        return n;
+    }
 };
+
+Parts fold(const KernelConfig& kc, const LutNet& net, uint32_t inner) {
+    Parts p;
+    p.inner = inner;
+    uint32_t wires = kc.nin;
+    for (const Lut& l : net.luts) wires = std::max(wires, l.wire + 1);
+    for (const Output& o : net.outs) wires = std::max(wires, o.wire + 1);
+    std::vector<uint8_t> gate(wires, 0), own(wires, 0);   // kc.nin counts a small circuit's padding too
+    for (uint32_t k = 0; k < inner; k++)
+        if (kc.in_of_bit[10 + k] >= 0) own[kc.in_of_bit[10 + k]] = 1;
+    for (const Lut& l : net.luts) {
+        gate[l.wire] = 1;
+        own[l.wire] = own[l.in[0]] | own[l.in[1]] | own[l.in[2]];
+    }
+    std::vector<uint8_t> need(wires, 0);                  // wires that the copies read
+    for (uint32_t c = 0; c < (1u << inner); c++) {
+        const auto renamed = [&](uint32_t w) { return own[w] && gate[w] ? wires * (c + 1) + w : w; };
+        std::vector<int8_t> value(wires, -1);             // constant value or -1
+        for (uint32_t k = 0; k < inner; k++)
+            if (kc.in_of_bit[10 + k] >= 0) value[kc.in_of_bit[10 + k]] = (int8_t)((c >> k) & 1u);
+        std::vector<Lut> luts;
+        for (const Lut& l : net.luts) {
+            if (!own[l.wire]) continue;
+            // fix the constant operands, and equal ones to each other
+            uint32_t any = l.wire;
+            for (const uint32_t w : l.in)
+                if (value[w] < 0) any = w;
+            uint8_t tt = 0;
+            bool ones = true, zeros = true;
+            for (uint32_t row = 0; row < 8; row++) {
+                uint32_t at = 0;
+                bool real = true;                         // the row gives equal wires equal values
+                for (int i = 0; i < 3; i++) {
+                    const uint32_t bit = (row >> (2 - i)) & 1u;
+                    at = at << 1 | (value[l.in[i]] >= 0 ? (uint32_t)value[l.in[i]] : bit);
+                    for (int h = 0; h < i; h++) {
+                        const bool same = value[l.in[i]] < 0 && l.in[h] == l.in[i];
+                        if (same && ((row >> (2 - h)) & 1u) != bit) real = false;
+                    }
+                }
+                const uint32_t v = (l.tt >> at) & 1u;
+                tt |= (uint8_t)(v << row);
+                if (real) (v ? zeros : ones) = false;
+            }
+            if (zeros || ones) {
+                value[l.wire] = ones ? 1 : 0;
+                continue;
+            }
+            Lut m = l;
+            m.tt = tt;
+            for (uint32_t& w : m.in)
+                if (value[w] >= 0) w = any;
+            luts.push_back(m);
+        }
+        LutNet net_c;
+        const Output out = net.outs[0];
+        if (value[out.wire] >= 0) {
+            p.constant.push_back((uint8_t)(value[out.wire] ^ (out.neg ? 1 : 0)));
+        } else {
+            p.constant.push_back(0);
+            std::vector<uint8_t> live(wires, 0);
+            live[out.wire] = 1;
+            for (size_t k = luts.size(); k-- > 0;)
+                if (live[luts[k].wire])
+                    for (const uint32_t w : luts[k].in) live[w] = 1;
+            for (uint32_t w = 0; w < wires; w++)
+                if (live[w] && !(own[w] && gate[w])) need[w] = 1;
+            for (Lut m : luts) {
+                if (!live[m.wire]) continue;
+                m.wire = renamed(m.wire);
+                for (uint32_t& w : m.in) w = renamed(w);
+                net_c.luts.push_back(m);
+            }
+            net_c.outs.push_back(Output{renamed(out.wire), out.neg});
+        }
+        p.copies.push_back(std::move(net_c));
+    }
+    for (uint32_t w = 0; w < wires; w++)
+        if (need[w] && gate[w]) p.shared.outs.push_back(Output{w, false});
+    std::vector<uint8_t> keep(net.luts.size(), 0);
+    for (size_t k = net.luts.size(); k-- > 0;) {
+        const Lut& l = net.luts[k];
+        if (own[l.wire] || !need[l.wire]) continue;
+        keep[k] = 1;
+        for (const uint32_t w : l.in) need[w] = 1;
+    }
+    for (size_t k = 0; k < net.luts.size(); k++)
+        if (keep[k]) p.shared.luts.push_back(net.luts[k]);
+    for (uint32_t w = 0; w < wires; w++)
+        if (need[w] && !gate[w]) p.shared.used_inputs.push_back(w);
+    return p;
+}
 
 // inner is the largest (up to 4) whose code stays within a budget, which is
 // about what the compiler's own unrolling took: 2400 LUTs or two copies for
 // SAT, 640 (a quantifier tree's share of a copy counted as 40) or little more
 // than one copy for QSAT, whose calls are shorter.  Device time in us and first
-// call in ms, left to the compiler and now: SAT 81 LUTs, 32 inputs 395, 76 and
+// call in ms, left to the compiler and so: SAT 81 LUTs, 32 inputs 395, 76 and
 // 116, 70; 201 LUTs, 33 inputs 2993, 102 and 1384, 73; 652 LUTs, 30 inputs
 // 1190, 198 and 1147, 108.  QSAT 14 LUTs, 30 inputs 61, 90 and 33, 100; 339
-// LUTs, 26 inputs 41, 121 and 34, 122.
+// LUTs, 26 inputs 41, 121 and 34, 122.  With 400 for QSAT a 38-LUT adder takes
+// 68 instead of 60 us and compiles no faster.
 constexpr uint32_t kMostInner = 4;
 Parts split(const KernelConfig& kc, const LutNet& net) {
     const bool sat = kc.mode == Mode::SAT;
     const size_t n = net.luts.size();
-    uint32_t wires = kc.nin;
-    for (const Lut& l : net.luts) wires = std::max(wires, l.wire + 1);
-    for (const Output& o : net.outs) wires = std::max(wires, o.wire + 1);
-    std::vector<uint8_t> gate(wires, 0);     // kc.nin counts a small circuit's padding too
-    for (const Lut& l : net.luts) gate[l.wire] = 1;
-    // the lowest iteration bit that a wire depends on
-    std::vector<uint8_t> lowest(wires, kMostInner);
-    const uint32_t most = std::min(kc.it, kMostInner);
-    for (uint32_t k = most; k-- > 0;)
-        if (kc.in_of_bit[10 + k] >= 0) lowest[kc.in_of_bit[10 + k]] = (uint8_t)k;
-    size_t own[kMostInner + 1] = {};     // LUTs whose lowest bit is k
-    for (const Lut& l : net.luts) {
-        lowest[l.wire] = std::min({lowest[l.in[0]], lowest[l.in[1]], lowest[l.in[2]]});
-        own[lowest[l.wire]]++;
-    }
-    Parts p;
     const size_t budget = sat ? std::max<size_t>(2400, 2 * n + 16) : std::max<size_t>(640, n + n / 8 + 80);
-    size_t copied = 0;
-    for (uint32_t k = 1; k <= most; k++) {
-        copied += own[k - 1];
-        if (n - copied + ((copied + (sat ? 8 : 40)) << k) <= budget) p.inner = k;
+    Parts best = fold(kc, net, 0);
+    for (uint32_t k = 1; k <= std::min(kc.it, kMostInner); k++) {
+        Parts p = fold(kc, net, k);
+        if (p.luts() + ((sat ? 8u : 40u) << k) > budget) break;
+        best = std::move(p);
     }
-    if (!p.inner) {
-        p.own = net;
-        return p;
-    }
-    std::vector<uint8_t> seen(wires, 0);     // 1: in cross or used_inputs of own, 2: of shared
-    const auto is_own = [&](uint32_t w) { return lowest[w] < p.inner; };
-    const auto own_reads = [&](uint32_t w) {
-        if (seen[w] & 1) return;
-        seen[w] |= 1;
-        if (!gate[w]) p.own.used_inputs.push_back(w);
-        else if (!is_own(w)) p.cross.push_back(w);
-    };
-    for (const Lut& l : net.luts) {
-        const bool mine = is_own(l.wire);
-        (mine ? p.own : p.shared).luts.push_back(l);
-        for (const uint32_t w : l.in) {
-            if (mine) {
-                own_reads(w);
-            } else if (!gate[w] && !(seen[w] & 2)) {
-                seen[w] |= 2;
-                p.shared.used_inputs.push_back(w);
-            }
-        }
-    }
-    for (const Output& o : net.outs) own_reads(o.wire);
-    for (const uint32_t w : p.cross) p.shared.outs.push_back(Output{w, false});
-    p.own.outs = net.outs;
-    return p;
+    return best;
 }
 
 }  // namespace
@@ -259,7 +317,6 @@ std::string generate_source(const KernelConfig& kc, const LutNet& net) {
     s << "#define NSAT_ONE " << (kc.cb <= kResidentBits ? 1 : 0) << "\n";
     const Parts parts = kc.mode == Mode::TABLE || kc.data ? Parts() : split(kc, net);
     s << "#define NSAT_INNER " << parts.inner << "\n";
-    s << "constexpr int NSAT_SHARED = " << std::max<size_t>(1, parts.cross.size()) << ";\n";
 
     // enumeration: which circuit input each bit drives
     const uint32_t it_lo = 10, wb_lo = 10 + kc.it, cb_lo = wb_lo + kc.wb, c_lo = cb_lo + kc.cb;
@@ -307,18 +364,14 @@ std::string generate_source(const KernelConfig& kc, const LutNet& net) {
         // thread of a CTA, so barriers inside the evaluation are safe
         const uint32_t sync = kc.threads() > 32 ? kc.sync_every : 0;
         const bool blocks = use_blocks(kc, net);
-        s << "__device__ __forceinline__ void nsat_shared(const u32* x, u32* sh) {\n";
+        s << "__device__ __forceinline__ void nsat_eval(const u32* x, u32* y) {\n";
         emit_luts(s, parts.shared, blocks, sync);
-        for (size_t k = 0; k < parts.cross.size(); k++) s << "    sh[" << k << "] = w" << parts.cross[k] << ";\n";
-        s << "}\n";
-        s << "__device__ __forceinline__ u32 nsat_eval1(const u32* x, const u32* sh) {\n";
-        if (!kc.data) {
-            for (size_t k = 0; k < parts.cross.size(); k++)
-                s << "    const u32 w" << parts.cross[k] << " = sh[" << k << "];\n";
-            emit_luts(s, parts.own, blocks, sync);
-            s << "    return " << (net.outs[0].neg ? "~" : "") << "w" << net.outs[0].wire << ";\n";
-        } else {
-            s << "    return 0u;\n";
+        for (size_t k = 0; k < parts.copies.size(); k++) {
+            const LutNet& copy = parts.copies[k];
+            emit_luts(s, copy, blocks, sync);
+            s << "    y[" << k << "] = ";
+            if (copy.outs.empty()) s << (parts.constant[k] ? "~0u" : "0u") << ";\n";
+            else s << (copy.outs[0].neg ? "~" : "") << "w" << copy.outs[0].wire << ";\n";
         }
         s << "}\n";
     }

@@ -14,8 +14,8 @@
 // and the generated device functions
 //   nsat_inputs_fixed(x, lane, warp, cta, launch)  -- inputs that stay fixed
 //   nsat_inputs_iter(x, it)                        -- inputs that follow `it`
-//   nsat_shared(x, sh)            what 2^NSAT_INNER iterations share
-//   nsat_eval1(x, sh) -> u32      output 0 as a 32-lane word
+//   nsat_eval(x, y)               output 0 of 2^NSAT_INNER iterations, a
+//                                 32-lane word each
 //   nsat_eval_all(x, o)           all outputs (table mode)
 //   nsat_inputs_word(x, w)        inputs of word index w (table mode)
 //
@@ -128,14 +128,13 @@ nsat_sat(u64 launch, LaunchOut* out, u64* host, u32 seq) {
     u32 first_it = 0xffffffffu, first_bit = 0;
 #pragma unroll 1
     for (u32 outer = 0; outer < (1u << NSAT_IT); outer += 1u << NSAT_INNER) {
-        u32 sh[NSAT_SHARED];
+        u32 ys[1 << NSAT_INNER];
         nsat_inputs_iter(x, outer);
-        nsat_shared(x, sh);
+        nsat_eval(x, ys);
 #pragma unroll
         for (u32 inner = 0; inner < (1u << NSAT_INNER); inner++) {
             const u32 it = outer | inner;
-            nsat_inputs_iter(x, it);
-            const u32 y = nsat_eval1(x, sh);
+            const u32 y = ys[inner];
             cnt += __popc(y);
             if (y != 0u && first_it == 0xffffffffu) { first_it = it; first_bit = __ffs(y) - 1; }
         }
@@ -338,9 +337,9 @@ nsat_qsat(u64 launch, LaunchOut* out, u64* host, u32 seq, u32* nodes, const u32*
 #pragma unroll 1
         for (u32 outer = 0; outer < (1u << NSAT_IT); outer += 1u << NSAT_INNER) {
 #if !NSAT_DATA
-        u32 sh[NSAT_SHARED];
+        u32 ys[1 << NSAT_INNER];
         nsat_inputs_iter(x, outer);
-        nsat_shared(x, sh);
+        nsat_eval(x, ys);
 #endif
 #pragma unroll
         for (u32 inner = 0; inner < (1u << NSAT_INNER); inner++) {
@@ -349,8 +348,7 @@ nsat_qsat(u64 launch, LaunchOut* out, u64* host, u32 seq, u32* nodes, const u32*
             const u64 gw = ((u64)launch << (NSAT_C - 5)) + ((u64)cta << (NSAT_LC - 5)) + ((warp_base + (it << 10)) >> 5) + lane;
             u32 y = data[gw];
 #else
-            nsat_inputs_iter(x, it);
-            u32 y = nsat_eval1(x, sh);
+            u32 y = ys[inner];
 #endif
             u32 b, git;   // node value at level L0 (bit 0) and its index among the warp's L0 nodes
             if constexpr (FOLDED) {
