@@ -489,6 +489,10 @@ nsat_qsat(u64 launch, LaunchOut* out, u64* host, u32 seq, u32* nodes, const u32*
     if (s_last) {
         __threadfence();
         for (u32 i = threadIdx.x; i < (make_blocks().nodes + 1u) / 2u; i += NSAT_NT) nodes[i] = 0u;
+        // the words release the host, and a launch of another stream may take
+        // the nodes over then: every thread's zeros come before them
+        __threadfence();
+        __syncthreads();
         if (threadIdx.x == 0) {
             out->values = 0u;
             nsat_publish(out, host, seq);

@@ -445,8 +445,9 @@ uint64_t reverse_bits(uint64_t v, uint32_t bits) {
 // for), so a solve of one launch that is estimated at less than 0.25 ms polls
 // its words in pinned memory, and the kernel times itself by the global timer:
 // there the events would be 4 % or more.  When the words are there, all that
-// the kernel writes is written; its CTAs may still be returning.  Later work
-// follows in stream order, and a circuit waits before it lets its kernels go.
+// the kernel writes in global memory is written (the QSAT nodes put back to
+// zero among it); its CTAs may still be returning.  Later work follows in
+// stream order, and a circuit waits before it lets its kernels go.
 bool short_launch(uint32_t log2_assignments, uint32_t lop3) {
     return std::ldexp((double)lop3 + 32.0, (int)log2_assignments - 5) < 0.25e-3 * kCompiledLutWordsPerS;
 }
