@@ -189,7 +189,9 @@ int nsat_qsat_solve(nsat_ctx* ctx, nsat_circuit* c, const uint8_t* quants,
  * The chunk tree's scratch comes from a static device array of
  * NSAT_NOALLOC_SCRATCH_BYTES (64 KiB) inside libnsat.so instead of the
  * context's lazily allocated buffer; every GPU that loads the library holds it
- * until exit.  A solve whose launches need more scratch (2 << CB bytes, CB =
+ * until exit, and every solve clears the part that it uses (on the context's
+ * stream, before its first launch), so what an earlier call left there does not
+ * matter.  A solve whose launches need more scratch (2 << CB bytes, CB =
  * log2 CTAs per launch, so launches of up to 2^15 CTAs fit) fails with
  * NSAT_EUNSUPPORTED before any kernel is compiled; lower chunk_bits then.
  * The first call on a device looks the array up (cudaGetSymbolAddress) and the

@@ -53,8 +53,8 @@ void ctx_trim(nsat_ctx* ctx);
 // Circuit from the C ABI's flat description (not validated).
 Circuit circuit_from_desc(const nsat_circuit_desc* d);
 
-// nsat_qsat_solve with the scratch area (the chunk tree's nodes, zero before
-// the first call; every launch leaves it zero) supplied by the caller
+// nsat_qsat_solve with the scratch area (the chunk tree's nodes, cleared before
+// the first launch) supplied by the caller
 // instead of the context's cudaMalloc'd buffer; fails with NSAT_EUNSUPPORTED
 // when a launch would need more than scratch_bytes.
 int qsat_solve_with_scratch(nsat_ctx* ctx, nsat_circuit* c, const uint8_t* quants,
@@ -79,3 +79,7 @@ int table_chunk(nsat_ctx* ctx, nsat_circuit* c, uint64_t first_state, uint64_t c
 const Circuit& circuit_of(const nsat_circuit* c);
 
 }  // namespace nsat
+
+// For the tests only: leaves the static area of nsat_qsat_solve_noalloc as a
+// launch that was cut short might.
+extern "C" int nsat_test_fill_noalloc(nsat_ctx* ctx, int byte);

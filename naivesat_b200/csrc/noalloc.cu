@@ -58,7 +58,13 @@ extern "C" int nsat_qsat_solve_noalloc(nsat_ctx* ctx, nsat_circuit* c, const uin
     unsigned char* scratch = nullptr;
     int rc = scratch_on(nsat::ctx_device(ctx), &scratch);
     if (rc != NSAT_OK) return rc;
-    // The area is zero when the module is loaded, and the last CTA of every
-    // launch puts it back to zero.
+    // The solve clears the nodes that it uses before its first launch; the
+    // last CTA of every launch puts them back to zero for the next.
     return nsat::qsat_solve_with_scratch(ctx, c, quants, opts, res, scratch, kScratchBytes);
+}
+
+int nsat_test_fill_noalloc(nsat_ctx* ctx, int byte) {
+    unsigned char* scratch = nullptr;
+    if (int rc = scratch_on(nsat::ctx_device(ctx), &scratch)) return rc;
+    return cudaMemsetAsync(scratch, byte, kScratchBytes, nsat::ctx_stream(ctx)) == cudaSuccess ? NSAT_OK : NSAT_ECUDA;
 }

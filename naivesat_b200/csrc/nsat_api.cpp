@@ -1021,6 +1021,10 @@ int qsat_common(nsat_ctx* ctx, nsat_circuit* c, const std::vector<uint8_t>& quan
     const CUfunction fn = memo.fn;
     if (!fixed_scratch) {
         if (int rc = ensure_scratch(ctx, (size_t)2 << kc.cb)) return rc;
+    } else {
+        // launches leave their nodes zero, but this area is shared: one that was
+        // cut short, or overlapped another, does not reach this solve
+        CK(cudaMemsetAsync(fixed_scratch, 0, (size_t)2 << kc.cb, ctx->stream));
     }
     if (data) {
         // expand 2^n items to 2^np (each item repeated 2^d times)
@@ -1103,7 +1107,10 @@ int qsat_common(nsat_ctx* ctx, nsat_circuit* c, const std::vector<uint8_t>& quan
             return true;
         },
         &dev_ms, &launches);
-    if (rc) return rc;
+    if (rc) {
+        ctx->scratch_bytes = 0;      // nodes that a failed launch may have left are not used again
+        return rc;
+    }
     if (!have) return fail(ctx, NSAT_ECUDA, "QSAT reduction did not finish");
     res->reversed = fr.reversed;
     res->solution_bits = fr.solution_bits;
