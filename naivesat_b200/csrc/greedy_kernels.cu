@@ -150,8 +150,8 @@ __device__ __forceinline__ void chase(u32 (&v)[4], const u32* table, const u32* 
     }
 }
 
-__global__ void __launch_bounds__(256) chase_before(const u32* __restrict__ table, u32 i, u32 lp,
-                                                    u32* __restrict__ snap, NsatGreedyState* st) {
+__global__ void __launch_bounds__(256) chase_before(const u32* table, u32 i, u32 lp, u32* snap,
+                                                    NsatGreedyState* st) {
     pdl_wait();
     // only chase_after writes the key: here it is that of an earlier step
     if (*(volatile const u64*)&st->key != ~0ull) {
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(256) chase_before(const u32* __restrict__ tabl
     }
 }
 
-__global__ void __launch_bounds__(256) chase_after(u32* table, const u32* __restrict__ snap, u32 i, u32 lp, u32 n,
+__global__ void __launch_bounds__(256) chase_after(u32* table, const u32* snap, u32 i, u32 lp, u32 n,
                                                    u32 unknowns, u32 step, NsatGreedyState* st) {
     pdl_wait();
     if (*(volatile const u32*)&st->done) return;

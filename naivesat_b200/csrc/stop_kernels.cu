@@ -81,8 +81,7 @@ __device__ __forceinline__ bool moot(const NsatStopState* st, u32 r, u32 mode) {
 }
 
 template <bool DIST, bool SAMPLE>
-__global__ void __launch_bounds__(256) join32(const u32* __restrict__ src, u32* __restrict__ dst,
-                                              u32* __restrict__ dist, u64 N, u32 n, u32 u, u32 r, u32 mode,
+__global__ void __launch_bounds__(256) join32(const u32* src, u32* dst, u32* dist, u64 N, u32 n, u32 u, u32 r, u32 mode,
                                               NsatStopState* __restrict__ st, u32* __restrict__ sample) {
     pdl_wait();
     if (answered(st, r, mode)) return;
@@ -497,10 +496,8 @@ __global__ void __launch_bounds__(256) starts64(const u64* __restrict__ upQ, con
     }
 }
 
-__global__ void __launch_bounds__(256) join_pq(const u64* __restrict__ P, const u64* __restrict__ Q,
-                                               u64* __restrict__ P2, u64* __restrict__ Q2,
-                                               const u32* __restrict__ start, u32 count, u32 n, u32 r, u32 mode,
-                                               NsatStopState* __restrict__ st) {
+__global__ void __launch_bounds__(256) join_pq(const u64* P, const u64* Q, u64* P2, u64* Q2, const u32* start,
+                                               u32 count, u32 n, u32 r, u32 mode, NsatStopState* __restrict__ st) {
     pdl_wait();
     if (answered(st, r, mode)) return;
     const u32 stop = 1u << n;

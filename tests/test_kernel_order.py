@@ -19,3 +19,23 @@ def test_nodes_are_zero_before_the_host_is_released():
     tail = text[text.index("nodes[i] = 0u;"):]
     tail = tail[:tail.index("nsat_publish(")]
     assert re.search(r"__threadfence\(\);\s*__syncthreads\(\);\s*if \(threadIdx\.x == 0\)", tail)
+
+
+def test_overlapped_kernels_take_no_const_restrict():
+    """A kernel that waits for its predecessor by pdl_wait can be resident while
+    its inputs are still being written, so none of them may be read through the
+    non-coherent path."""
+    seen = 0
+    for name in sorted(os.listdir(CSRC)):
+        if not name.endswith((".cu", ".cuh")):
+            continue
+        text = source(name)
+        for k in re.finditer(r"__global__[^{;]*\)\s*\{", text):
+            body = text[k.end():]
+            body = body[:body.index("\n}\n")]
+            if "pdl_wait()" not in body:
+                continue
+            seen += 1
+            assert not re.search(r"const\s+\w+\s*\*\s*__restrict__", k.group(0)), k.group(0)
+            assert "__ldg(" not in body
+    assert seen == 4
