@@ -499,13 +499,13 @@ int run_ring(nsat_ctx* ctx, uint64_t total, bool polled, Issue issue, Consume co
         return NSAT_OK;
     }
     uint64_t issued = 0, done = 0;
-    bool stop = false;
+    bool stop = false;       // the result is known: what is in flight does not count any more
     *dev_ms = 0;
     *launches = 0;
     while (done < issued || (!stop && issued < total)) {
         if (!stop && issued < total && issued - done < (uint64_t)kRing && !claim(issued, (int)(issued % kRing))) {
-            stop = true;
-            continue;      // nothing more to issue: consume what is in flight, if anything
+            total = issued;      // nothing more to issue: consume what is in flight, if anything
+            continue;
         }
         if (!stop && issued < total && issued - done < (uint64_t)kRing) {
             const int slot = (int)(issued % kRing);
