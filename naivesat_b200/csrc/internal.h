@@ -36,6 +36,8 @@ void ctx_free(nsat_ctx* ctx, void* p);
 void ctx_stop_state(nsat_ctx* ctx, NsatStopState** dev, NsatStopState** host);
 cudaEvent_t ctx_stop_event(nsat_ctx* ctx);
 NsatGridState* ctx_grid_state(nsat_ctx* ctx);
+uint32_t ctx_grid_spins(nsat_ctx* ctx);
+void ctx_grid_gave_up(nsat_ctx* ctx);
 // A short kernel that reports in up to 5 words of pinned memory, each with the
 // launch's number (ctx_next_seq) in its upper half; ctx_poll_words waits for
 // the first `words`.
@@ -83,3 +85,6 @@ const Circuit& circuit_of(const nsat_circuit* c);
 // For the tests only: leaves the static area of nsat_qsat_solve_noalloc as a
 // launch that was cut short might.
 extern "C" int nsat_test_fill_noalloc(nsat_ctx* ctx, int byte);
+// For the tests only: sets the polls after which grid_solve's barrier gives up;
+// returns how many times it has since the last call.
+extern "C" int nsat_test_grid_spins(nsat_ctx* ctx, uint32_t spins);

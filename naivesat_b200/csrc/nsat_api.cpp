@@ -94,6 +94,7 @@ struct nsat_ctx {
     NsatJoinState* h_join = nullptr;
     NsatStopState* d_stop = nullptr;
     NsatGridState* d_grid = nullptr;  // put back to its first state by each solve
+    uint32_t grid_spins = NSAT_STOP_SPINS, grid_gave_up = 0;
     NsatStopState* h_stop = nullptr;
     void* h_read = nullptr;           // pinned, kReadStage bytes (nsat_table_read)
     // loaded kernels by everything their generated source depends on (the
@@ -1169,6 +1170,14 @@ void nsat::ctx_stop_state(nsat_ctx* ctx, NsatStopState** dev, NsatStopState** ho
 }
 cudaEvent_t nsat::ctx_stop_event(nsat_ctx* ctx) { return ctx->evd; }
 NsatGridState* nsat::ctx_grid_state(nsat_ctx* ctx) { return ctx->d_grid; }
+uint32_t nsat::ctx_grid_spins(nsat_ctx* ctx) { return ctx->grid_spins; }
+void nsat::ctx_grid_gave_up(nsat_ctx* ctx) { ctx->grid_gave_up++; }
+int nsat_test_grid_spins(nsat_ctx* ctx, uint32_t spins) {
+    const int gave_up = (int)ctx->grid_gave_up;
+    ctx->grid_spins = spins;
+    ctx->grid_gave_up = 0;
+    return gave_up;
+}
 uint32_t nsat::ctx_next_seq(nsat_ctx* ctx) { return next_seq(ctx); }
 volatile uint64_t* nsat::ctx_words(nsat_ctx* ctx) { return ctx->h_out[0].word; }
 int nsat::ctx_poll_words(nsat_ctx* ctx, int words) { return poll_out(ctx, ctx->h_out[0], words); }

@@ -113,17 +113,23 @@ int stop_run(nsat_ctx* ctx, StopRun* x) {
     Scratch mem(ctx);
     uint32_t* dist = x->steps ? x->dist : nullptr;
     if (x->steps && !dist && !mem.get(&dist, N)) return NSAT_ENOMEM;
-    if (n > NSAT_STOP_SMALL_BITS && n <= NSAT_STOP_GRID_BITS) {
+    uint32_t* keep = nullptr;
+    if (n > NSAT_STOP_SMALL_BITS && n <= NSAT_STOP_GRID_BITS && mem.get(&keep, N)) {
         const uint32_t seq = ctx_next_seq(ctx);
-        const int rc = nsat_stop_grid(x->a, x->b, dist, n, u, mode, x->steps, x->out64, ctx_grid_state(ctx),
-                                      (uint64_t*)ctx_words(ctx), seq, st);
+        const int rc = nsat_stop_grid(x->a, x->b, keep, dist, n, u, mode, x->steps, x->out64, ctx_grid_state(ctx),
+                                      ctx_grid_spins(ctx), (uint64_t*)ctx_words(ctx), seq, st);
         if (rc < 0) return ctx_fail(ctx, NSAT_ECUDA, "doubling launch failed");
         if (rc == 0) {
             x->launches++;
             if (int e = polled_answer(ctx, x)) return e;
-            if (x->rounds == ~0u) return ctx_fail(ctx, NSAT_ECUDA, "the doubling's grid barrier gave up");
-            x->table = (x->rounds & 1) ? x->b : x->a;
-            return NSAT_OK;
+            if (x->rounds != ~0u) {
+                x->table = (x->rounds & 1) ? x->b : x->a;
+                return NSAT_OK;
+            }
+            // the barrier gave up: a launch per round, from the table as built
+            x->polled = false;
+            ctx_grid_gave_up(ctx);
+            JCK(cudaMemcpyAsync(x->a, keep, N * 4, cudaMemcpyDeviceToDevice, st));
         }
     }
     if (x->begin) JCK(cudaEventRecord(x->begin, st));

@@ -225,15 +225,18 @@ SmallKernel small_kernel(u32 n) {
 // gathers from one buffer, writes the other and ends in a grid barrier.  The
 // buffers and distances change while the kernel runs, so they are read through
 // the L2.  The barrier counts arrivals up; its spin is bounded, and a CTA that
-// gives up lets the others go too.  The last CTA to end reports as small_solve
-// does (rounds ~0: given up) and leaves the state as it was.
+// gives up lets the others go too.  keep receives the table as built, so that
+// the rounds can start again from it then (a third buffer in place of a in the
+// rounds took 8 us more than this copy at 2^20 entries).  The last CTA to end
+// reports as small_solve does (rounds ~0: given up) and leaves the state as it
+// was.
 constexpr u32 kGridThreads = 1024;
-constexpr u32 kSpinLimit = 1u << 22;
 
 template <bool STEPS, int E>
-__global__ void __launch_bounds__(kGridThreads) grid_solve(u32* a, u32* b, u32* dist, u32 n, u32 u, u32 mode,
-                                                           u64* __restrict__ out64, NsatGridState* st,
-                                                           volatile u64* words, u32 seq) {
+__global__ void __launch_bounds__(kGridThreads) grid_solve(u32* a, u32* b, u32* __restrict__ keep, u32* dist, u32 n,
+                                                           u32 u, u32 mode, u64* __restrict__ out64,
+                                                           NsatGridState* st, u32 spin_limit, volatile u64* words,
+                                                           u32 seq) {
     __shared__ u32 s_best, s_round;      // lowest start in this CTA, lowest of all after the round
     __shared__ bool s_failed;
     const u32 tid = threadIdx.x, S = gridDim.x * kGridThreads, i0 = blockIdx.x * kGridThreads + tid;
@@ -248,6 +251,7 @@ __global__ void __launch_bounds__(kGridThreads) grid_solve(u32* a, u32* b, u32* 
     for (int k = 0; k < E; k++) {
         const u32 i = i0 + k * S;
         v[k] = __ldcg(a + i);
+        __stcs(keep + i, v[k]);
         d[k] = 1u;
         if (STEPS && (v[k] & stop)) __stcg(dist + i, 1u);
     }
@@ -282,7 +286,7 @@ __global__ void __launch_bounds__(kGridThreads) grid_solve(u32* a, u32* b, u32* 
             const u32 all = r * gridDim.x;
             u32 spins = 0;
             while (*(volatile u32*)&st->arrived < all && !*(volatile u32*)&st->failed)
-                if (++spins == kSpinLimit) *(volatile u32*)&st->failed = 1u;
+                if (++spins == spin_limit) *(volatile u32*)&st->failed = 1u;
             __threadfence();
             s_failed = *(volatile u32*)&st->failed != 0u;
             s_round = *(volatile u32*)&st->best[r];
@@ -320,7 +324,7 @@ __global__ void __launch_bounds__(kGridThreads) grid_solve(u32* a, u32* b, u32* 
     words[4] = number | t;
 }
 
-typedef void (*GridKernel)(u32*, u32*, u32*, u32, u32, u32, u64*, NsatGridState*, volatile u64*, u32);
+typedef void (*GridKernel)(u32*, u32*, u32*, u32*, u32, u32, u32, u64*, NsatGridState*, u32, volatile u64*, u32);
 template <bool STEPS>
 GridKernel grid_kernel(u32 per_thread) {
     switch (per_thread) {
@@ -622,16 +626,16 @@ extern "C" int nsat_stop_small(const uint32_t* src, uint32_t n, uint32_t u, uint
     return ok();
 }
 
-extern "C" int nsat_stop_grid(uint32_t* a, uint32_t* b, uint32_t* dist, uint32_t n, uint32_t u, uint32_t mode,
-                              int steps, uint64_t* out64, NsatGridState* st, uint64_t* words, uint32_t seq,
-                              cudaStream_t s) {
+extern "C" int nsat_stop_grid(uint32_t* a, uint32_t* b, uint32_t* keep, uint32_t* dist, uint32_t n, uint32_t u,
+                              uint32_t mode, int steps, uint64_t* out64, NsatGridState* st, uint32_t spin_limit,
+                              uint64_t* words, uint32_t seq, cudaStream_t s) {
     if (n <= NSAT_STOP_SMALL_BITS || n > NSAT_STOP_GRID_BITS) return -1;
     // 128 CTAs from 2^17 entries on
     const u32 e = n <= 17 ? 1u : 1u << (n - 17);
     const GridKernel fn = steps ? grid_kernel<true>(e) : grid_kernel<false>(e);
     volatile u64* w = (volatile u64*)words;
     u64* o = (u64*)out64;
-    void* args[] = {&a, &b, &dist, &n, &u, &mode, &o, &st, &w, &seq};
+    void* args[] = {&a, &b, &keep, &dist, &n, &u, &mode, &o, &st, &spin_limit, &w, &seq};
     if (cudaLaunchCooperativeKernel((const void*)fn, dim3((1u << n) / (kGridThreads * e)), dim3(kGridThreads), args, 0, s) == cudaSuccess)
         return 0;
     cudaGetLastError();

@@ -45,9 +45,13 @@ int nsat_stop_small(const uint32_t* src, uint32_t n, uint32_t u, uint32_t mode, 
 
 // The same for NSAT_STOP_SMALL_BITS < n <= NSAT_STOP_GRID_BITS in one cooperative
 // launch between a (the table, also after an even number of rounds) and b.
-// dist: 2^n words, with steps.  1: the device does not hold the grid.
-int nsat_stop_grid(uint32_t* a, uint32_t* b, uint32_t* dist, uint32_t n, uint32_t u, uint32_t mode, int steps,
-                   uint64_t* out64, NsatGridState* st, uint64_t* words, uint32_t seq, cudaStream_t s);
+// dist: 2^n words, with steps.  1: the device does not hold the grid.  A CTA
+// that has polled the barrier spin_limit times in vain ends the launch: rounds
+// ~0, and of the buffers only keep (2^n words), a copy of a, is of use.
+#define NSAT_STOP_SPINS (1u << 22)
+int nsat_stop_grid(uint32_t* a, uint32_t* b, uint32_t* keep, uint32_t* dist, uint32_t n, uint32_t u, uint32_t mode,
+                   int steps, uint64_t* out64, NsatGridState* st, uint32_t spin_limit, uint64_t* words, uint32_t seq,
+                   cudaStream_t s);
 
 // Contraction to the states that a later round can still look up.
 // marks in bits (cleared, items bits) the successors of items entries, unless
