@@ -765,7 +765,7 @@ extern "C" int nsat_server_create(nsat_ctx* ctx, const nsat_server_opts* opts, n
     if (!s->opts.arena_bytes) s->opts.arena_bytes = 1ull << 30;
     if (!s->opts.max_active || s->opts.max_active > kMaxActive) s->opts.max_active = kMaxActive;
     if (!s->opts.max_queue) s->opts.max_queue = 1u << 20;
-    if (!s->opts.max_slice_tiles) s->opts.max_slice_tiles = 4096;
+    s->opts.max_slice_tiles = srv_slice_cap(s->opts.max_slice_tiles);
     // a new job starts with 256 tiles (2^23 assignments, well under a
     // millisecond of interpreter time for the trace's circuits): on the mixed
     // serving trace that measured 663 solves/s and p99 85 ms at 150/s, against

@@ -30,6 +30,12 @@ static const SrvShape kSrvShapes[SRV_NSHAPES] = {
 #define SRV_SUB_BITS 2             // a warp claims a quarter of a tile at a time
 #define SRV_PART_BITS (SRV_TILE_BITS - SRV_SUB_BITS)
 #define SRV_MAX_NB 48              // enumeration bits a serving job may have
+// Tiles of one job's slice: 4096 unless the caller says, at most 2^28, whose
+// parts SrvJob::next counts in 32 bits with room for every warp's last claim.
+#define SRV_MAX_SLICE (1u << 28)
+inline uint32_t srv_slice_cap(uint32_t wanted) {
+    return wanted == 0 ? 4096u : wanted < SRV_MAX_SLICE ? wanted : SRV_MAX_SLICE;
+}
 inline uint32_t srv_slot_bytes(uint32_t shape) { return 32u * kSrvShapes[shape].words * 4u; }
 
 // One instruction: slot[d] = LUT(slot[a], slot[b], slot[c]), 16 bytes:
