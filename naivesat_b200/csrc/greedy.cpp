@@ -29,6 +29,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -74,6 +75,7 @@ uint64_t packed_bytes(uint64_t count, uint32_t bits) { return ((count * bits) >>
 struct Work {
     nsat_ctx* ctx = nullptr;
     int storage = DEVICE;
+    bool reuses = false;              // sized by what the pool holds, not by the free memory
     uint64_t bytes = 0;
     uint64_t* dev_image = nullptr;    // DEVICE
     uint64_t* host_image = nullptr;   // HOST (pinned)
@@ -139,9 +141,11 @@ int check_opts(nsat_ctx* ctx, uint32_t n, const nsat_greedy_opts* o, uint32_t* p
     return NSAT_OK;
 }
 
-// Chooses where the image lives and allocates the image and work buffers.
+// Chooses where the image lives and allocates the image and work buffers;
+// reuse: without a look at the free memory where the pool's unused bytes are
+// enough.
 int setup(nsat_ctx* ctx, Work& w, uint32_t n, uint64_t L, uint64_t chunk, const nsat_greedy_opts* o,
-          bool joins) {
+          bool joins, bool reuse) {
     w.ctx = ctx;
     const uint32_t P = o->partitions;
     const uint32_t bits = n + 1;
@@ -155,7 +159,8 @@ int setup(nsat_ctx* ctx, Work& w, uint32_t n, uint64_t L, uint64_t chunk, const 
     } else {
         budget = o->device_bytes;
         const uint64_t take = n <= 31 && joins ? table32 : w.bytes + work_dev;   // what is allocated below
-        if (!budget && take <= ctx_pool_unused(ctx)) {
+        w.reuses = reuse && !budget && take <= ctx_pool_unused(ctx);
+        if (w.reuses) {
             // buffers that an earlier call gave back to the pool are enough: no
             // need to ask the driver for the free memory (70 us, and on a host
             // shared with other jobs now and then tens of milliseconds)
@@ -419,8 +424,19 @@ extern "C" int nsat_greedy_solve(nsat_ctx* ctx, nsat_circuit* c, const nsat_gree
     const uint64_t chunk = 1ull << (n - lb);
     const uint64_t pbytes = packed_bytes(L, bits), pwords = pbytes / 8;
     GCK(cudaSetDevice(ctx_device(ctx)));
-    Work w;
-    if (int rc = setup(ctx, w, n, L, chunk, o, true)) return rc;
+    std::unique_ptr<Work> work(new Work());
+    int src = setup(ctx, *work, n, L, chunk, o, true, true);
+    if (src == NSAT_ENOMEM && work->reuses) {
+        // the pool's unused bytes lie in pieces: give them back and go by the
+        // free memory
+        cudaGetLastError();
+        work.reset();
+        ctx_trim(ctx);
+        work.reset(new Work());
+        src = setup(ctx, *work, n, L, chunk, o, true, false);
+    }
+    if (src) return src;
+    Work& w = *work;
     r->storage = (uint32_t)w.storage;
     bool any_stop = false;
     if (int rc = build_image(ctx, c, w, lb, &any_stop, r)) return rc;
@@ -489,7 +505,7 @@ extern "C" int nsat_greedy_image(nsat_ctx* ctx, nsat_circuit* c, uint32_t partit
     const uint64_t L = 1ull << (n - pbits), chunk = 1ull << (n - lb);
     GCK(cudaSetDevice(ctx_device(ctx)));
     Work w;
-    if (int rc = setup(ctx, w, n, L, chunk, &o, false)) return rc;
+    if (int rc = setup(ctx, w, n, L, chunk, &o, false, true)) return rc;
     nsat_greedy_result r{};
     bool any = false;
     if (int rc = build_image(ctx, c, w, lb, &any, &r)) return rc;

@@ -85,6 +85,9 @@ const Circuit& circuit_of(const nsat_circuit* c);
 // For the tests only: leaves the static area of nsat_qsat_solve_noalloc as a
 // launch that was cut short might.
 extern "C" int nsat_test_fill_noalloc(nsat_ctx* ctx, int byte);
+// For the tests only: the k-th buffer taken from the pool from now on is
+// refused (0: none); returns what was left of an earlier call's k.
+extern "C" int nsat_test_fail_alloc(nsat_ctx* ctx, uint32_t k);
 // For the tests only: sets the polls after which grid_solve's barrier gives up;
 // returns how many times it has since the last call.
 extern "C" int nsat_test_grid_spins(nsat_ctx* ctx, uint32_t spins);

@@ -94,6 +94,7 @@ struct nsat_ctx {
     NsatJoinState* h_join = nullptr;
     NsatStopState* d_stop = nullptr;
     NsatGridState* d_grid = nullptr;  // put back to its first state by each solve
+    uint32_t fail_alloc = 0;          // tests: the buffer allocations until one fails (0: none)
     uint32_t grid_spins = NSAT_STOP_SPINS, grid_gave_up = 0;
     NsatStopState* h_stop = nullptr;
     void* h_read = nullptr;           // pinned, kReadStage bytes (nsat_table_read)
@@ -1159,6 +1160,7 @@ int nsat::qsat_solve_blocks(nsat_ctx* ctx, nsat_circuit* c, const uint8_t* quant
 int nsat::ctx_device(const nsat_ctx* ctx) { return ctx ? ctx->device : -1; }
 cudaStream_t nsat::ctx_stream(const nsat_ctx* ctx) { return ctx->stream; }
 cudaError_t nsat::ctx_alloc(nsat_ctx* ctx, void** p, size_t bytes) {
+    if (ctx->fail_alloc && --ctx->fail_alloc == 0) return cudaErrorMemoryAllocation;
     return cudaMallocFromPoolAsync(p, bytes, ctx->pool, ctx->stream);
 }
 void nsat::ctx_free(nsat_ctx* ctx, void* p) {
@@ -1172,6 +1174,11 @@ cudaEvent_t nsat::ctx_stop_event(nsat_ctx* ctx) { return ctx->evd; }
 NsatGridState* nsat::ctx_grid_state(nsat_ctx* ctx) { return ctx->d_grid; }
 uint32_t nsat::ctx_grid_spins(nsat_ctx* ctx) { return ctx->grid_spins; }
 void nsat::ctx_grid_gave_up(nsat_ctx* ctx) { ctx->grid_gave_up++; }
+int nsat_test_fail_alloc(nsat_ctx* ctx, uint32_t k) {
+    const int left = (int)ctx->fail_alloc;
+    ctx->fail_alloc = k;
+    return left;
+}
 int nsat_test_grid_spins(nsat_ctx* ctx, uint32_t spins) {
     const int gave_up = (int)ctx->grid_gave_up;
     ctx->grid_spins = spins;
