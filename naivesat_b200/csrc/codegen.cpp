@@ -289,6 +289,60 @@ Parts split(const KernelConfig& kc, const LutNet& net) {
     return best;
 }
 
+// The tree above the chunks of a QSAT launch (device_template.cuh): a block's
+// first node, the chunk bits below one of its nodes, the children that a node
+// has, and their quantifier.
+struct TreeBlock {
+    uint32_t first, shift, children;
+    bool all;
+};
+
+// The walks of a chunk up the blocks' nodes, as asm: nsat_nodes_above ORs the
+// nodes above chunk c; nsat_nodes_resolve enters the value v of chunk c and
+// returns whether it resolved the last block's node too.  As statements
+// unrolled over the blocks they took up to a sixth of a small formula's first
+// call (32-input adder with a key 108 ms, 89 so; 28 inputs, 80 gates, blocks of
+// up to five 98 and 78 ms); a loop over a table in constant memory compiles
+// as fast, but waits for each node's load (30 inputs, 1500 gates 183 -> 203 us).
+void emit_tree(std::ostringstream& s, const KernelConfig& kc) {
+    const uint32_t lc = 10 + kc.it + kc.wb, top = std::min(kc.m, kc.c);
+    std::vector<TreeBlock> blocks;
+    uint32_t nodes = 0;
+    const auto all = [&](uint32_t l) { return ((kc.allbits >> l) & 1u) != 0; };
+    for (uint32_t lo = lc, hi; lo < top; lo = hi) {
+        for (hi = lo + 1; hi < top && hi - lo < 8 && all(hi) == all(lo); hi++) {}
+        blocks.push_back(TreeBlock{nodes, hi - lc, 1u << (hi - lo), all(lo)});
+        nodes += 1u << (kc.c - hi);
+    }
+    s << "constexpr u32 NSAT_NODES = " << nodes << "u;\n";
+    s << "__device__ __forceinline__ u32 nsat_nodes_above(u32 c, const u32* nodes) {\n";
+    if (blocks.empty()) {
+        s << "    return 0u;\n}\n__device__ __forceinline__ bool nsat_nodes_resolve(u32 c, u32 v, u32* nodes) { return true; }\n";
+        return;
+    }
+    s << "    u32 seen;\n    asm volatile(\"{ .reg .b32 i; .reg .b64 a; .reg .b16 w<" << blocks.size() << ">;\\n\"\n";
+    for (size_t k = 0; k < blocks.size(); k++)      // every load before the first use
+        s << "\"shr.u32 i, %1, " << blocks[k].shift << "; add.u32 i, i, " << blocks[k].first
+          << "; mul.wide.u32 a, i, 2; add.u64 a, a, %2; ld.volatile.global.u16 w" << k << ", [a];\\n\"\n";
+    for (size_t k = 1; k < blocks.size(); k++) s << "\"or.b16 w0, w0, w" << k << ";\\n\"\n";
+    s << "\"cvt.u32.u16 %0, w0; }\" : \"=r\"(seen) : \"r\"(c), \"l\"(nodes));\n    return seen;\n}\n";
+    s << "__device__ __forceinline__ bool nsat_nodes_resolve(u32 c, u32 v, u32* nodes) {\n"
+      << "    u32 up = 0u;\n    asm volatile(\"{ .reg .pred p; .reg .b32 i, h, m, o; .reg .b64 a;\\n\"\n";
+    for (size_t k = 0; k < blocks.size(); k++) {
+        const TreeBlock& b = blocks[k];
+        // node i: half h of word a
+        s << "\"shr.u32 i, %1, " << b.shift << "; add.u32 i, i, " << b.first
+          << "; and.b32 h, i, 1; shl.b32 h, h, 4; shr.u32 i, i, 1; mul.wide.u32 a, i, 4; add.u64 a, a, %3;\\n\"\n"
+          // neither the deciding value nor the last child (or the node is resolved): done
+          << "\"setp.ne.u32 p, %2, " << (b.all ? 1 : 0) << "; @p bra R" << k
+          << "; mov.b32 m, 1; shl.b32 m, m, h; atom.global.add.u32 o, [a], m; shr.u32 o, o, h; and.b32 o, o, 0xffff; "
+          << "setp.ne.u32 p, o, " << b.children - 1 << "; @p bra D;\\n\"\n"
+          << "\"R" << k << ": mov.b32 m, 0x8000; shl.b32 m, m, h; atom.global.or.b32 o, [a], m; and.b32 o, o, m; "
+          << "setp.ne.u32 p, o, 0; @p bra D;\\n\"\n";
+    }
+    s << "\"mov.b32 %0, 1; D: }\" : \"+r\"(up) : \"r\"(c), \"r\"(v), \"l\"(nodes) : \"memory\");\n    return up != 0u;\n}\n";
+}
+
 }  // namespace
 
 std::string generate_source(const KernelConfig& kc, const LutNet& net) {
@@ -375,6 +429,7 @@ std::string generate_source(const KernelConfig& kc, const LutNet& net) {
         }
         s << "}\n";
     }
+    if (kc.mode == Mode::QSAT) emit_tree(s, kc);
     s << kDeviceTemplate;
     return s.str();
 }

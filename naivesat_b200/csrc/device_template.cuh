@@ -18,6 +18,8 @@
 //                                 32-lane word each
 //   nsat_eval_all(x, o)           all outputs (table mode)
 //   nsat_inputs_word(x, w)        inputs of word index w (table mode)
+//   nsat_nodes_above(c, nodes), nsat_nodes_resolve(c, v, nodes), NSAT_NODES
+//                                 the tree above the chunks (QSAT, below)
 //
 // Assignment enumeration inside one launch (bit p of the launch-relative
 // index selects circuit input IN_OF_BIT[p], baked into the functions above):
@@ -205,30 +207,9 @@ __device__ constexpr int low_run(u64 allbits) {
 // block above.  A chunk below a resolved node cannot change anything and is
 // not evaluated, nor is one whose units lie above a decisive unit.  A node is
 // 16 bits: 0x8000 once resolved, the count of its undecided children below.
-struct QBlocks {
-    int n;
-    int lo[64], hi[64];    // levels [lo, hi) of block k
-    u32 off[64];           // its nodes' first index
-    u32 nodes;
-};
+// The generator cuts the blocks and writes the two walks through them.
 constexpr int NSAT_LC = 10 + NSAT_IT + NSAT_WB;
 constexpr int NSAT_TOP = NSAT_M < NSAT_C ? NSAT_M : NSAT_C;
-__device__ constexpr QBlocks make_blocks() {
-    QBlocks b = {};
-    int l = NSAT_LC;
-    while (l < NSAT_TOP) {
-        int h = l + 1;
-        while (h < NSAT_TOP && h - l < 8 && (((NSAT_ALLBITS >> l) ^ (NSAT_ALLBITS >> h)) & 1ull) == 0ull) h++;
-        b.lo[b.n] = l;
-        b.hi[b.n] = h;
-        b.off[b.n] = b.nodes;
-        b.nodes += 1u << (NSAT_C - h);
-        b.n++;
-        l = h;
-    }
-    return b;
-}
-
 // Order of the chunks: 2^UB units side by side, the chunks of each in order.
 // One deciding child ends a node's other children, so the chunks in flight
 // are spread over units; within a unit depth first decides most per chunk.
@@ -252,14 +233,7 @@ __device__ __forceinline__ u32 chunk_of(u32 t) {
 
 // Whether chunk c has nothing left to decide.
 __device__ __forceinline__ bool chunk_decided(u32 c, const u32* nodes, const LaunchOut* out) {
-    constexpr QBlocks B = make_blocks();
-    bool done = false;
-#pragma unroll
-    for (int k = 0; k < B.n; k++) {
-        const u32 i = B.off[k] + (c >> (B.hi[k] - NSAT_LC));
-        const u32 w = *(volatile const u32*)(nodes + (i >> 1));
-        done |= ((w >> ((i & 1u) << 4)) & 0x8000u) != 0u;
-    }
+    bool done = (nsat_nodes_above(c, nodes) & 0x8000u) != 0u;
     if constexpr (NSAT_M < NSAT_C) {
         const u64 lowest = *(volatile const u64*)&out->min_idx;
         if constexpr (NSAT_M >= NSAT_LC) done |= lowest <= (u64)(c >> (NSAT_M - NSAT_LC));
@@ -270,20 +244,7 @@ __device__ __forceinline__ bool chunk_decided(u32 c, const u32* nodes, const Lau
 
 // One thread: chunk c has value v.
 __device__ __forceinline__ void chunk_value(u32 c, u32 v, u32* nodes, LaunchOut* out) {
-    constexpr QBlocks B = make_blocks();
-#pragma unroll
-    for (int k = 0; k < B.n; k++) {
-        const u32 i = B.off[k] + (c >> (B.hi[k] - NSAT_LC));
-        const u32 sh = (i & 1u) << 4;
-        u32* w = nodes + (i >> 1);
-        if (v != (u32)((NSAT_ALLBITS >> B.lo[k]) & 1ull)) {                    // the deciding value
-            if ((atomicOr(w, 0x8000u << sh) >> sh) & 0x8000u) return;
-        } else {
-            const u32 old = (atomicAdd(w, 1u << sh) >> sh) & 0xffffu;
-            if (old != (1u << (B.hi[k] - B.lo[k])) - 1u) return;               // not the last child, or resolved
-            if ((atomicOr(w, 0x8000u << sh) >> sh) & 0x8000u) return;
-        }
-    }
+    if (!nsat_nodes_resolve(c, v, nodes)) return;
     if constexpr (NSAT_M >= NSAT_C) out->tree = v;
     else if (v == (NSAT_Q0ALL ? 0u : 1u)) atomicMin(&out->min_idx, (u64)(c >> (NSAT_M - NSAT_LC)));
 }
@@ -448,26 +409,28 @@ nsat_qsat(u64 launch, LaunchOut* out, u64* host, u32 seq, u32* nodes, const u32*
         break;
 #else
         if (warp == 0) {
-            u32 base = s_base, mask = s_mask, step = s_step, c = ~0u;
+            u32 base = s_base, mask = s_mask, step = s_step, c;
             for (;;) {
                 const u32 t = base + lane;
                 c = chunk_of(t);
                 mask = __ballot_sync(0xffffffffu, ((mask >> lane) & 1u) && t < (1u << NSAT_CB) && !chunk_decided(c, nodes, out));
-                if (mask) {
-                    const int f = __ffs(mask) - 1;
-                    c = __shfl_sync(0xffffffffu, c, f);
-                    mask &= mask - 1u;
-                    step = 1u;
-                    break;
+                if (mask || base >= (1u << NSAT_CB)) break;
+                u32 take = 1u;
+                if (!claimed) {
+                    take = step;
+                    if (lane == 0) ahead = atomicAdd(&out->values, take);
                 }
-                c = ~0u;
-                if (base >= (1u << NSAT_CB)) break;
-                const u32 take = claimed ? 1u : step;
-                if (lane == 0) base = gridDim.x + (claimed ? ahead : atomicAdd(&out->values, take));
                 claimed = false;
-                base = __shfl_sync(0xffffffffu, base, 0);
-                mask = take >= 32u ? ~0u : (1u << take) - 1u;
+                base = gridDim.x + __shfl_sync(0xffffffffu, ahead, 0);
+                mask = (1u << take) - 1u;
                 step = step < 16u ? step * 2u : 16u;
+            }
+            if (mask) {
+                c = __shfl_sync(0xffffffffu, c, __ffs(mask) - 1);
+                mask &= mask - 1u;
+                step = 1u;
+            } else {
+                c = ~0u;
             }
             if (c != ~0u && mask == 0u && !claimed) {
                 if (lane == 0) ahead = atomicAdd(&out->values, 1u);
@@ -488,7 +451,7 @@ nsat_qsat(u64 launch, LaunchOut* out, u64* host, u32 seq, u32* nodes, const u32*
     __syncthreads();
     if (s_last) {
         __threadfence();
-        for (u32 i = threadIdx.x; i < (make_blocks().nodes + 1u) / 2u; i += NSAT_NT) nodes[i] = 0u;
+        for (u32 i = threadIdx.x; i < (NSAT_NODES + 1u) / 2u; i += NSAT_NT) nodes[i] = 0u;
         // the words release the host, and a launch of another stream may take
         // the nodes over then: every thread's zeros come before them
         __threadfence();
