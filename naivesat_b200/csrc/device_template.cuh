@@ -255,7 +255,7 @@ __device__ __forceinline__ void chunk_value(u32 c, u32 v, u32* nodes, LaunchOut*
 // launch has a CTA for every chunk (the claims' code would cost a small
 // circuit a third of its compile time).
 extern "C" __global__ void NSAT_BOUNDS
-nsat_qsat(u64 launch, LaunchOut* out, u64* host, u32 seq, u32* nodes, const u32* __restrict__ data) {
+nsat_qsat(u64 launch, LaunchOut* out, u64* host, u32 seq, u32* nodes, u32 shared, const u32* __restrict__ data) {
     nsat_begin(out);
     constexpr int M = NSAT_M;
     // Folding.  When levels 0..9 (the word and the warp tile) and the lowest
@@ -453,9 +453,12 @@ nsat_qsat(u64 launch, LaunchOut* out, u64* host, u32 seq, u32* nodes, const u32*
         __threadfence();
         for (u32 i = threadIdx.x; i < (NSAT_NODES + 1u) / 2u; i += NSAT_NT) nodes[i] = 0u;
         // the words release the host, and a launch of another stream may take
-        // the nodes over then: every thread's zeros come before them
-        __threadfence();
-        __syncthreads();
+        // shared nodes over then: every thread's zeros come before them (which
+        // takes 0.5-1 us; nodes of one stream need no more than its order)
+        if (shared) {
+            __threadfence();
+            __syncthreads();
+        }
         if (threadIdx.x == 0) {
             out->values = 0u;
             nsat_publish(out, host, seq);

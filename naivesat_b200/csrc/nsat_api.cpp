@@ -447,9 +447,9 @@ uint64_t reverse_bits(uint64_t v, uint32_t bits) {
 // for), so a solve of one launch that is estimated at less than 0.25 ms polls
 // its words in pinned memory, and the kernel times itself by the global timer:
 // there the events would be 4 % or more.  When the words are there, all that
-// the kernel writes in global memory is written (the QSAT nodes put back to
-// zero among it); its CTAs may still be returning.  Later work follows in
-// stream order, and a circuit waits before it lets its kernels go.
+// another stream may read or write is written (for the QSAT nodes that is the
+// shared area of noalloc solves); its CTAs may still be returning.  Later work
+// follows in stream order, and a circuit waits before it lets its kernels go.
 bool short_launch(uint32_t log2_assignments, uint32_t lop3) {
     return std::ldexp((double)lop3 + 32.0, (int)log2_assignments - 5) < 0.25e-3 * kCompiledLutWordsPerS;
 }
@@ -1057,6 +1057,7 @@ int qsat_common(nsat_ctx* ctx, nsat_circuit* c, const std::vector<uint8_t>& quan
     uint64_t nl = prefix_count > 1 ? prefix_count : (A == 64 ? ~0ull : (1ull << A));
     const unsigned grid = memo.grid, threads = kc.threads();
     unsigned char* scratch = fixed_scratch ? fixed_scratch : ctx->d_scratch;
+    uint32_t shared = fixed_scratch ? 1 : 0;
     const uint32_t* dd = ctx->d_data;
     double dev_ms = 0;
     uint32_t launches = 0;
@@ -1068,7 +1069,7 @@ int qsat_common(nsat_ctx* ctx, nsat_circuit* c, const std::vector<uint8_t>& quan
         [&](uint64_t k, int slot) {
             uint64_t index = L0 + k;
             Report to(ctx, slot);
-            void* params[] = {&index, &to.out, &to.host, &to.seq, &scratch, &dd};
+            void* params[] = {&index, &to.out, &to.host, &to.seq, &scratch, &shared, &dd};
             return launch(ctx, fn, grid, threads, params);
         },
         [&](uint64_t k, const HostOut& r) {

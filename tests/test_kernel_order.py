@@ -13,12 +13,13 @@ def source(name):
 
 def test_nodes_are_zero_before_the_host_is_released():
     """The last CTA's threads all put QSAT nodes back to zero; the words that
-    release the host (after which another context may use the nodes) follow a
+    release the host (after which another context may use shared nodes) follow a
     fence by each thread and a barrier."""
     text = source("device_template.cuh")
     tail = text[text.index("nodes[i] = 0u;"):]
     tail = tail[:tail.index("nsat_publish(")]
-    assert re.search(r"__threadfence\(\);\s*__syncthreads\(\);\s*if \(threadIdx\.x == 0\)", tail)
+    assert re.search(r"if \(shared\) \{\s*__threadfence\(\);\s*__syncthreads\(\);\s*\}\s*if \(threadIdx\.x == 0\)", tail)
+    assert "uint32_t shared = fixed_scratch ? 1 : 0;" in source("nsat_api.cpp")
 
 
 def test_overlapped_kernels_take_no_const_restrict():
