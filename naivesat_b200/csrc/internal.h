@@ -85,6 +85,8 @@ const Circuit& circuit_of(const nsat_circuit* c);
 // For the tests only: leaves the static area of nsat_qsat_solve_noalloc as a
 // launch that was cut short might.
 extern "C" int nsat_test_fill_noalloc(nsat_ctx* ctx, int byte);
+// For the tests only: the number of the context's next launch.
+extern "C" int nsat_test_launch_number(nsat_ctx* ctx, uint32_t next);
 // For the tests only: the k-th buffer taken from the pool from now on is
 // refused (0: none); returns what was left of an earlier call's k.
 extern "C" int nsat_test_fail_alloc(nsat_ctx* ctx, uint32_t k);

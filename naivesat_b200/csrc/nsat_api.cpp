@@ -1175,6 +1175,10 @@ cudaEvent_t nsat::ctx_stop_event(nsat_ctx* ctx) { return ctx->evd; }
 NsatGridState* nsat::ctx_grid_state(nsat_ctx* ctx) { return ctx->d_grid; }
 uint32_t nsat::ctx_grid_spins(nsat_ctx* ctx) { return ctx->grid_spins; }
 void nsat::ctx_grid_gave_up(nsat_ctx* ctx) { ctx->grid_gave_up++; }
+int nsat_test_launch_number(nsat_ctx* ctx, uint32_t next) {
+    ctx->seq = next - 1;
+    return NSAT_OK;
+}
 int nsat_test_fail_alloc(nsat_ctx* ctx, uint32_t k) {
     const int left = (int)ctx->fail_alloc;
     ctx->fail_alloc = k;
