@@ -267,7 +267,8 @@ typedef struct {
 } nsat_tune_opts;
 
 typedef struct {
-    uint32_t block_threads, min_blocks, cta_bits_max;   /* the chosen shape */
+    uint32_t block_threads, min_blocks, cta_bits_max;   /* the chosen shape (cta_bits_max 0, QSAT: by
+                                 the formula's size) */
     uint32_t candidates;      /* shapes timed (0 when taken from the cache) */
     uint32_t from_cache;
     uint32_t sync_every;      /* CTA barrier every this many LUTs in the evaluation (0 = none) */

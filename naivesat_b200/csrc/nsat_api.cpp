@@ -1707,7 +1707,8 @@ void precompile(nsat_ctx* ctx, nsat_circuit* c, uint32_t kind, const std::vector
 }
 
 std::string tune_key(nsat_ctx* ctx, nsat_circuit* c, uint32_t kind, const uint8_t* quants) {
-    std::string k = "tune2|" + std::to_string(kind) + "|" + std::to_string(c->circ.n) + "|";
+    // QSAT choices of version 2 say 12 CTA bits where the default was meant
+    std::string k = (kind == 1 ? "tune3|" : "tune2|") + std::to_string(kind) + "|" + std::to_string(c->circ.n) + "|";
     for (const Gate& g : c->circ.gates) k += std::to_string(g.func) + "," + std::to_string(g.i0) + "," + std::to_string(g.i1) + ";";
     k += "|";
     for (const Output& o : c->circ.outputs) k += std::to_string(o.wire) + (o.neg ? "n;" : ";");
@@ -1819,7 +1820,9 @@ extern "C" int nsat_autotune(nsat_ctx* ctx, nsat_circuit* c, const nsat_tune_opt
     }
     slot = best.sh;
     if (!slot.block_threads) slot.block_threads = 256;
-    if (!slot.cb_max) slot.cb_max = 12;
+    // the default cap; a QSAT formula without a cap of its own also cuts its
+    // launch into small chunks (choose_chunks), so there the choice stays open
+    if (!slot.cb_max && kind == 0) slot.cb_max = 12;
     res->block_threads = slot.block_threads;
     res->min_blocks = slot.min_blocks;
     res->cta_bits_max = slot.cb_max;
