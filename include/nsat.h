@@ -240,7 +240,8 @@ typedef struct {
     uint32_t rounds;       /* doubling rounds run */
     uint64_t start, end, steps;   /* steps only with want_steps */
     double build_ms, join_ms;     /* as device_ms of nsat_sat_result: by the global
-                                     timer up to 2^20 states (build), 2^14 (rounds) */
+                                     timer up to 2^20 states, while the rounds are
+                                     one launch */
 } nsat_stop_result;
 
 int nsat_stop_solve(nsat_ctx* ctx, nsat_table* t, const nsat_stop_opts* opts,

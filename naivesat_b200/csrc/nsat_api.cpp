@@ -618,8 +618,9 @@ int plan_qsat(uint32_t n, const std::vector<uint8_t>& quants_in, bool data, uint
     return NSAT_OK;
 }
 
-// chunked: the partitioned solver builds u64 entries chunk by chunk, so the
-// device-memory limit on n does not apply.
+// chunked: for the partitioned solver, which builds packed images chunk by
+// chunk from u64 entries, so the device-memory limit on n does not apply, and
+// device tables of n <= 31 at once (table_chunk picks the format).
 int plan_table(const Circuit& circ, bool steps, KernelConfig* kc, std::string* err, bool chunked = false) {
     const uint32_t n = circ.n;
     if (circ.outputs.size() != n + 1) { *err = "SATOSTOP circuit needs n+1 outputs"; return NSAT_EINVAL; }
@@ -783,8 +784,8 @@ extern "C" int nsat_circuit_new(nsat_ctx* ctx, const nsat_circuit_desc* desc, ns
 extern "C" void nsat_circuit_free(nsat_circuit* c) {
     if (!c) return;
     // The handle may hold the last reference to its kernels' modules: release
-    // them with their device current (solves return only after their launches
-    // finished, so none is queued), then give the caller back its device.
+    // them with their device current, then give the caller back its device.
+    // Only a polled launch may still be returning (the destructor waits for it).
     int prev = -1;
     const bool switched = cudaGetDevice(&prev) == cudaSuccess && c->device >= 0 && c->device != prev &&
                           cudaSetDevice(c->device) == cudaSuccess;
