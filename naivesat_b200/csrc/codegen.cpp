@@ -297,13 +297,15 @@ struct TreeBlock {
     bool all;
 };
 
-// The walks of a chunk up the blocks' nodes, as asm: nsat_nodes_above ORs the
-// nodes above chunk c; nsat_nodes_resolve enters the value v of chunk c and
-// returns whether it resolved the last block's node too.  As statements
-// unrolled over the blocks they took up to a sixth of a small formula's first
-// call (32-input adder with a key 108 ms, 89 so; 28 inputs, 80 gates, blocks of
-// up to five 98 and 78 ms); a loop over a table in constant memory compiles
-// as fast, but waits for each node's load (30 inputs, 1500 gates 183 -> 203 us).
+// The walks of a chunk up the blocks' nodes and the claims of chunks, as asm:
+// nsat_nodes_resolve enters the value v of chunk c and returns whether it
+// resolved the last block's node too; nsat_claim finds the next chunk that is
+// not decided.  As statements they took up to a fifth of a formula's first call,
+// which had become longer than with no tree at all (32-input adder with a key 88
+// -> 108 ms, 80 so; 28 inputs, 80 gates, blocks of up to five 89 -> 98,
+// 67 so).  A loop over a table in constant memory in place of the walks
+// compiles as fast, but waits for each node's load (30 inputs, 1500 gates 183 ->
+// 203 us).
 void emit_tree(std::ostringstream& s, const KernelConfig& kc) {
     const uint32_t lc = 10 + kc.it + kc.wb, top = std::min(kc.m, kc.c);
     std::vector<TreeBlock> blocks;
@@ -315,32 +317,70 @@ void emit_tree(std::ostringstream& s, const KernelConfig& kc) {
         nodes += 1u << (kc.c - hi);
     }
     s << "constexpr u32 NSAT_NODES = " << nodes << "u;\n";
-    s << "__device__ __forceinline__ u32 nsat_nodes_above(u32 c, const u32* nodes) {\n";
-    if (blocks.empty()) {
-        s << "    return 0u;\n}\n__device__ __forceinline__ bool nsat_nodes_resolve(u32 c, u32 v, u32* nodes) { return true; }\n";
-        return;
-    }
-    s << "    u32 seen;\n    asm volatile(\"{ .reg .b32 i; .reg .b64 a; .reg .b16 w<" << blocks.size() << ">;\\n\"\n";
-    for (size_t k = 0; k < blocks.size(); k++)      // every load before the first use
-        s << "\"shr.u32 i, %1, " << blocks[k].shift << "; add.u32 i, i, " << blocks[k].first
-          << "; mul.wide.u32 a, i, 2; add.u64 a, a, %2; ld.volatile.global.u16 w" << k << ", [a];\\n\"\n";
-    for (size_t k = 1; k < blocks.size(); k++) s << "\"or.b16 w0, w0, w" << k << ";\\n\"\n";
-    s << "\"cvt.u32.u16 %0, w0; }\" : \"=r\"(seen) : \"r\"(c), \"l\"(nodes));\n    return seen;\n}\n";
+    const auto line = [&s](const std::string& l) { s << "\"" << l << "\\n\"\n"; };
+    const auto num = [](uint64_t v) { return std::to_string(v); };
+
     s << "__device__ __forceinline__ bool nsat_nodes_resolve(u32 c, u32 v, u32* nodes) {\n"
-      << "    u32 up = 0u;\n    asm volatile(\"{ .reg .pred p; .reg .b32 i, h, m, o; .reg .b64 a;\\n\"\n";
+      << "    u32 up = 0u;\n    asm volatile(\n";
+    line("{ .reg .pred p; .reg .b32 i, h, m, o; .reg .b64 a;");
     for (size_t k = 0; k < blocks.size(); k++) {
         const TreeBlock& b = blocks[k];
         // node i: half h of word a
-        s << "\"shr.u32 i, %1, " << b.shift << "; add.u32 i, i, " << b.first
-          << "; and.b32 h, i, 1; shl.b32 h, h, 4; shr.u32 i, i, 1; mul.wide.u32 a, i, 4; add.u64 a, a, %3;\\n\"\n"
-          // neither the deciding value nor the last child (or the node is resolved): done
-          << "\"setp.ne.u32 p, %2, " << (b.all ? 1 : 0) << "; @p bra R" << k
-          << "; mov.b32 m, 1; shl.b32 m, m, h; atom.global.add.u32 o, [a], m; shr.u32 o, o, h; and.b32 o, o, 0xffff; "
-          << "setp.ne.u32 p, o, " << b.children - 1 << "; @p bra D;\\n\"\n"
-          << "\"R" << k << ": mov.b32 m, 0x8000; shl.b32 m, m, h; atom.global.or.b32 o, [a], m; and.b32 o, o, m; "
-          << "setp.ne.u32 p, o, 0; @p bra D;\\n\"\n";
+        line("shr.u32 i, %1, " + num(b.shift) + "; add.u32 i, i, " + num(b.first) +
+             "; and.b32 h, i, 1; shl.b32 h, h, 4; shr.u32 i, i, 1; mul.wide.u32 a, i, 4; add.u64 a, a, %3;");
+        // neither the deciding value nor the last child (or the node is resolved): done
+        line("setp.ne.u32 p, %2, " + num(b.all ? 1 : 0) + "; @p bra R" + num(k) +
+             "; mov.b32 m, 1; shl.b32 m, m, h; atom.global.add.u32 o, [a], m; shr.u32 o, o, h; and.b32 o, o, 0xffff;");
+        line("setp.ne.u32 p, o, " + num(b.children - 1) + "; @p bra D;");
+        line("R" + num(k) + ": mov.b32 m, 0x8000; shl.b32 m, m, h; atom.global.or.b32 o, [a], m; and.b32 o, o, m; "
+             "setp.ne.u32 p, o, 0; @p bra D;");
     }
-    s << "\"mov.b32 %0, 1; D: }\" : \"+r\"(up) : \"r\"(c), \"r\"(v), \"l\"(nodes) : \"memory\");\n    return up != 0u;\n}\n";
+    line("mov.b32 %0, 1; D: }");
+    s << ": \"+r\"(up) : \"r\"(c), \"r\"(v), \"l\"(nodes) : \"memory\");\n    return up != 0u;\n}\n";
+    if (kc.cb <= kResidentBits) return;
+
+    // One warp.  claim: first chunk index b, mask m of those not looked at yet,
+    // the chunk found (~0: none left).  k: how many the next claim takes, 0 when
+    // it has been made ahead.
+    const uint32_t units = kc.m >= lc && kc.m < kc.c ? kc.c - kc.m : 0, side = std::min(units, 7u);
+    const uint32_t in = kc.cb - units;
+    s << "__device__ __forceinline__ void nsat_claim(u32 lane, const u32* nodes, const u64* lowest, u32* counter, "
+      << "u32* claim, u32& ahead) {\n    asm volatile(\n";
+    line("{ .reg .pred p, q; .reg .b32 t, i, m, k, b, c; .reg .b64 a, l, x; .reg .b16 v, w<" + num(blocks.size() + 1) + ">;");
+    line("ld.shared.u32 b, [%5]; ld.shared.u32 m, [%5+4]; setp.ne.u32 p, m, 0; selp.b32 k, 1, 0, p;");
+    // the next claim, by lane 0
+    line("L: setp.ne.u32 p, m, 0; @p bra C;");
+    line("setp.ne.u32 p, k, 0; setp.eq.and.u32 q, %1, 0, p; @q atom.global.add.u32 %0, [%4], k; max.u32 k, k, 1;");
+    line("shfl.sync.idx.b32 b, %0, 0, 31, 0xffffffff; mov.u32 t, %%nctaid.x; add.u32 b, b, t;");
+    line("mov.b32 m, 1; shl.b32 m, m, k; sub.u32 m, m, 1; shl.b32 k, k, 1; min.u32 k, k, 16;");
+    // a lane each: p, chunk c is open
+    line("C: add.u32 t, b, %1; shr.u32 i, m, %1; and.b32 i, i, 1; setp.ne.u32 p, i, 0; setp.lt.and.u32 p, t, " +
+         num(1ull << kc.cb) + ", p;");
+    if (side == 0) line("mov.b32 c, t;");
+    else                                     // chunk_of
+        line("and.b32 i, t, " + num((1u << side) - 1) + "; shr.u32 c, t, " + num(side + in) + "; shl.b32 c, c, " + num(side) +
+             "; or.b32 c, c, i; shl.b32 c, c, " + num(in) + "; shr.u32 i, t, " + num(side) + "; and.b32 i, i, " +
+             num((1u << in) - 1) + "; or.b32 c, c, i;");
+    for (size_t k = 0; k < blocks.size(); k++)      // every load before the first use
+        line("mov.b16 w" + num(k) + ", 0; shr.u32 i, c, " + num(blocks[k].shift) + "; add.u32 i, i, " + num(blocks[k].first) +
+             "; mul.wide.u32 a, i, 2; add.u64 a, a, %2; @p ld.volatile.global.u16 w" + num(k) + ", [a];");
+    // no unit below chunk c's (or its own, where a unit has several chunks) is decisive
+    if (kc.m < kc.c) line("mov.b64 l, 0; @p ld.volatile.global.u64 l, [%3]; cvt.u64.u32 x, c;");
+    line("mov.b16 v, 0;");
+    for (size_t k = 0; k < blocks.size(); k++) line("or.b16 v, v, w" + num(k) + ";");
+    line("and.b16 v, v, 0x8000; setp.eq.and.u16 p, v, 0, p;");
+    if (kc.m < kc.c)
+        line(kc.m >= lc ? "shr.u64 x, x, " + num(kc.m - lc) + "; setp.gt.and.u64 p, l, x, p;"
+                        : "shl.b64 x, x, " + num(lc - kc.m) + "; setp.ge.and.u64 p, l, x, p;");
+    line("vote.sync.ballot.b32 m, p, 0xffffffff; setp.eq.u32 p, m, 0; setp.lt.and.u32 q, b, " + num(1ull << kc.cb) +
+         ", p; @q bra L;");
+    // the first open one; the next claim ahead when it is the last of this one
+    line("neg.s32 t, m; and.b32 t, t, m; bfind.u32 t, t; sub.u32 i, m, 1; and.b32 m, m, i;");
+    line("shfl.sync.idx.b32 c, c, t, 31, 0xffffffff; selp.b32 c, -1, c, p;");
+    line("setp.ne.u32 p, c, -1; setp.eq.and.u32 p, m, 0, p; setp.eq.and.u32 p, %1, 0, p; @p atom.global.add.u32 %0, [%4], 1;");
+    line("setp.eq.u32 q, %1, 0; @q st.shared.u32 [%5], b; @q st.shared.u32 [%5+4], m; @q st.shared.u32 [%5+8], c; }");
+    s << ": \"+r\"(ahead) : \"r\"(lane), \"l\"(nodes), \"l\"(lowest), \"l\"(counter), "
+      << "\"r\"((u32)__cvta_generic_to_shared(claim)) : \"memory\");\n}\n";
 }
 
 }  // namespace

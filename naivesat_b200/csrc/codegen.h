@@ -10,8 +10,11 @@ namespace nsat {
 
 enum class Mode { SAT = 1, QSAT = 2, TABLE = 3 };
 
-// A launch of up to 2^7 CTAs has them all resident (148 SMs).
-constexpr uint32_t kResidentBits = 7;
+// QSAT launches of up to 2^9 chunks (three CTAs on each of 148 SMs are 444)
+// have a CTA for each: about one wave, so there is hardly a chunk that could
+// turn out decided before it is evaluated, and a claim loop would only add to
+// the compile (24-input adder 79 -> 55 ms).
+constexpr uint32_t kResidentBits = 9;
 
 struct KernelConfig {
     Mode mode = Mode::SAT;

@@ -18,7 +18,7 @@
 //                                 32-lane word each
 //   nsat_eval_all(x, o)           all outputs (table mode)
 //   nsat_inputs_word(x, w)        inputs of word index w (table mode)
-//   nsat_nodes_above(c, nodes), nsat_nodes_resolve(c, v, nodes), NSAT_NODES
+//   nsat_nodes_resolve(c, v, nodes), nsat_claim(...), NSAT_NODES
 //                                 the tree above the chunks (QSAT, below)
 //
 // Assignment enumeration inside one launch (bit p of the launch-relative
@@ -207,7 +207,7 @@ __device__ constexpr int low_run(u64 allbits) {
 // block above.  A chunk below a resolved node cannot change anything and is
 // not evaluated, nor is one whose units lie above a decisive unit.  A node is
 // 16 bits: 0x8000 once resolved, the count of its undecided children below.
-// The generator cuts the blocks and writes the two walks through them.
+// The generator cuts the blocks and writes the walks through them.
 constexpr int NSAT_LC = 10 + NSAT_IT + NSAT_WB;
 constexpr int NSAT_TOP = NSAT_M < NSAT_C ? NSAT_M : NSAT_C;
 // Order of the chunks: 2^UB units side by side, the chunks of each in order.
@@ -231,17 +231,6 @@ __device__ __forceinline__ u32 chunk_of(u32 t) {
     }
 }
 
-// Whether chunk c has nothing left to decide.
-__device__ __forceinline__ bool chunk_decided(u32 c, const u32* nodes, const LaunchOut* out) {
-    bool done = (nsat_nodes_above(c, nodes) & 0x8000u) != 0u;
-    if constexpr (NSAT_M < NSAT_C) {
-        const u64 lowest = *(volatile const u64*)&out->min_idx;
-        if constexpr (NSAT_M >= NSAT_LC) done |= lowest <= (u64)(c >> (NSAT_M - NSAT_LC));
-        else done |= lowest < ((u64)c << (NSAT_LC - NSAT_M));
-    }
-    return done;
-}
-
 // One thread: chunk c has value v.
 __device__ __forceinline__ void chunk_value(u32 c, u32 v, u32* nodes, LaunchOut* out) {
     if (!nsat_nodes_resolve(c, v, nodes)) return;
@@ -251,9 +240,8 @@ __device__ __forceinline__ void chunk_value(u32 c, u32 v, u32* nodes, LaunchOut*
 
 // Resident CTAs take chunks until none is left: chunk blockIdx.x first, then
 // from the launch's counter (out->values), one at a time while they need
-// evaluation, up to 16 at once while they turn out decided.  NSAT_ONE: the
-// launch has a CTA for every chunk (the claims' code would cost a small
-// circuit a third of its compile time).
+// evaluation, up to 16 at once while they turn out decided (nsat_claim).
+// NSAT_ONE: the launch has a CTA for every chunk.
 extern "C" __global__ void NSAT_BOUNDS
 nsat_qsat(u64 launch, LaunchOut* out, u64* host, u32 seq, u32* nodes, u32 shared, const u32* __restrict__ data) {
     nsat_begin(out);
@@ -279,11 +267,13 @@ nsat_qsat(u64 launch, LaunchOut* out, u64* host, u32 seq, u32* nodes, u32 shared
     __shared__ u32 s_last, s_res[32];
     u32 cta = chunk_of(blockIdx.x);             // not checked: nothing is decided yet
 #if !NSAT_ONE
-    __shared__ u32 s_cta, s_base, s_mask, s_step;      // warp 0's claim: chunks s_base + the bits of s_mask
-    if (threadIdx.x == 0) { s_base = blockIdx.x; s_mask = 0u; s_step = 1u; }
-    u32 ahead = 0u;        // warp 0, lane 0: the next claim, made while this chunk is evaluated
-    bool claimed = warp == 0;
-    if (threadIdx.x == 0) ahead = atomicAdd(&out->values, 1u);
+    __shared__ u32 s_claim[3];     // warp 0's claim: chunks [0] + the bits of [1]; the chunk to evaluate
+    u32 ahead = 0u;        // warp 0, lane 0: the next claim, made while the last chunk of one is evaluated
+    if (threadIdx.x == 0) {
+        s_claim[0] = blockIdx.x;
+        s_claim[1] = 0u;
+        ahead = atomicAdd(&out->values, 1u);
+    }
 #endif
     for (;;) {
         // index within the chunk (at most 25 bits) of this warp's first item
@@ -404,42 +394,13 @@ nsat_qsat(u64 launch, LaunchOut* out, u64* host, u32 seq, u32* nodes, u32 shared
                 }
             }
         }
-        __syncthreads();       // s_cta and s_res are written again
+        __syncthreads();       // s_claim and s_res are written again
 #if NSAT_ONE
         break;
 #else
-        if (warp == 0) {
-            u32 base = s_base, mask = s_mask, step = s_step, c;
-            for (;;) {
-                const u32 t = base + lane;
-                c = chunk_of(t);
-                mask = __ballot_sync(0xffffffffu, ((mask >> lane) & 1u) && t < (1u << NSAT_CB) && !chunk_decided(c, nodes, out));
-                if (mask || base >= (1u << NSAT_CB)) break;
-                u32 take = 1u;
-                if (!claimed) {
-                    take = step;
-                    if (lane == 0) ahead = atomicAdd(&out->values, take);
-                }
-                claimed = false;
-                base = gridDim.x + __shfl_sync(0xffffffffu, ahead, 0);
-                mask = (1u << take) - 1u;
-                step = step < 16u ? step * 2u : 16u;
-            }
-            if (mask) {
-                c = __shfl_sync(0xffffffffu, c, __ffs(mask) - 1);
-                mask &= mask - 1u;
-                step = 1u;
-            } else {
-                c = ~0u;
-            }
-            if (c != ~0u && mask == 0u && !claimed) {
-                if (lane == 0) ahead = atomicAdd(&out->values, 1u);
-                claimed = true;
-            }
-            if (lane == 0) { s_base = base; s_mask = mask; s_step = step; s_cta = c; }
-        }
+        if (warp == 0) nsat_claim(lane, nodes, &out->min_idx, &out->values, s_claim, ahead);
         __syncthreads();
-        cta = s_cta;
+        cta = s_claim[2];
         if (cta == ~0u) break;
 #endif
     }
