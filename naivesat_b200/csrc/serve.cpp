@@ -558,7 +558,28 @@ int run_joins(nsat_server* s, Job* j) {
     x.a = (uint32_t*)(s->arena.base + j->table_off);
     x.b = (uint32_t*)(s->arena.base + j->table2_off);
     x.dist = x.b + (1ull << j->n);
-    if (int rc = stop_run(s->ctx, &x)) return rc;
+    // scratch is the first area's other half, then what the arena has left: the
+    // server's memory stays what its caller gave it (where the arena is full, a
+    // solve runs its plain rounds)
+    char* spare = (char*)(x.a + (1ull << j->n));
+    size_t spare_left = (size_t)4 << j->n;
+    std::vector<std::pair<size_t, size_t>> lent;
+    x.scratch = [&](size_t bytes) -> void* {
+        if (bytes <= spare_left) {
+            char* p = spare;
+            const size_t take = std::min((bytes + 255) & ~(size_t)255, spare_left);
+            spare += take;
+            spare_left -= take;
+            return p;
+        }
+        size_t off = 0;
+        if (!s->arena.alloc(bytes, &off)) return nullptr;
+        lent.emplace_back(off, bytes);
+        return s->arena.base + off;
+    };
+    const int rc = stop_run(s->ctx, &x);
+    for (const auto& l : lent) s->arena.release(l.first, l.second);
+    if (rc) return rc;
     s->launches += x.launches;
     s->h2d_bytes += sizeof(NsatStopState);
     s->d2h_bytes += sizeof(NsatStopState) + 8;

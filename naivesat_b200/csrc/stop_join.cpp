@@ -48,12 +48,18 @@ struct Level {
 
 struct Scratch {
     nsat_ctx* ctx;
+    const std::function<void*(size_t)>& own;
     std::vector<void*> p;
-    explicit Scratch(nsat_ctx* c) : ctx(c) {}
+    Scratch(nsat_ctx* c, const std::function<void*(size_t)>& o) : ctx(c), own(o) {}
     ~Scratch() { for (void* q : p) ctx_free(ctx, q); }
     template <typename T>
     bool get(T** out, uint64_t count) {
         void* q = nullptr;
+        if (own) {
+            q = own(count * sizeof(T));
+            *out = static_cast<T*>(q);
+            return q != nullptr;
+        }
         if (ctx_alloc(ctx, &q, count * sizeof(T)) != cudaSuccess) {
             cudaGetLastError();
             return false;
@@ -110,7 +116,7 @@ int stop_run(nsat_ctx* ctx, StopRun* x) {
         x->table = x->b;
         return NSAT_OK;
     }
-    Scratch mem(ctx);
+    Scratch mem(ctx, x->scratch);
     uint32_t* dist = x->steps ? x->dist : nullptr;
     if (x->steps && !dist && !mem.get(&dist, N)) return NSAT_ENOMEM;
     uint32_t* keep = nullptr;

@@ -2,6 +2,8 @@
 #pragma once
 #include <stdint.h>
 
+#include <functional>
+
 #include "internal.h"
 #include "stop_kernels.h"
 
@@ -17,6 +19,9 @@ struct StopRun {
     cudaEvent_t begin = nullptr;   // recorded before the first kernel (null: not wanted)
     cudaEvent_t done = nullptr;    // and behind the last
     uint64_t* out64 = nullptr;     // steps: the 64-bit table after the last round (null: not wanted)
+    // where scratch buffers come from, null when there is no room; the caller
+    // has them back after the call (not set: the context's pool)
+    std::function<void*(size_t)> scratch;
     // out
     uint32_t rounds = 0;
     bool found = false;
