@@ -192,7 +192,7 @@ int nsat_qsat_solve(nsat_ctx* ctx, nsat_circuit* c, const uint8_t* quants,
  * until exit, and every solve clears the part that it uses (on the context's
  * stream, before its first launch), so what an earlier call left there does not
  * matter.  A solve whose launches need more scratch (2 << CB bytes, CB =
- * log2 CTAs per launch, so launches of up to 2^15 CTAs fit) fails with
+ * log2 chunks per launch, so launches of up to 2^15 chunks fit) fails with
  * NSAT_EUNSUPPORTED before any kernel is compiled; lower chunk_bits then.
  * The first call on a device looks the array up (cudaGetSymbolAddress) and the
  * first call for a circuit/quantifier string compiles and loads its kernel;

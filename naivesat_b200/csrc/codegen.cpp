@@ -160,8 +160,9 @@ void emit_luts(std::ostringstream& s, const LutNet& net, bool blocks, uint32_t s
 // iteration's lowest inner bits, beside one of the rest (shared).  In copy c
 // those bits are the constants of c, which are folded here: the compiler does
 // not fold every lop3 (36 inputs, 3018 gates, planted block: 83 or 163 ms by
-// the circuit, 7.1 ms folded here, first call 314 -> 99 ms).  A copy that folds to a constant costs nothing, as half of the copies
-// do for each bit that a conjunction tests.
+// the circuit, 8.9-11.1 ms for six circuits folded here).  A copy that folds to
+// a constant costs nothing, as half of the copies do for each bit that a
+// conjunction tests.
 struct Parts {
     uint32_t inner = 0;
     LutNet shared;                       // used_inputs: of the copies too
@@ -273,8 +274,9 @@ Parts fold(const KernelConfig& kc, const LutNet& net, uint32_t inner) {
 // call in ms, left to the compiler and so: SAT 81 LUTs, 32 inputs 395, 76 and
 // 116, 70; 201 LUTs, 33 inputs 2993, 102 and 1384, 73; 652 LUTs, 30 inputs
 // 1190, 198 and 1147, 108.  QSAT 14 LUTs, 30 inputs 61, 90 and 33, 100; 339
-// LUTs, 26 inputs 41, 121 and 34, 122.  With 400 for QSAT a 38-LUT adder takes
-// 68 instead of 60 us and compiles no faster.
+// LUTs, 26 inputs 41, 121 and 34, 122, both with the chunk tree's code as
+// statements (emit_tree), which was 20-45 ms of these first calls.  With 400 for
+// QSAT a 38-LUT adder takes 68 instead of 60 us and compiles no faster.
 constexpr uint32_t kMostInner = 4;
 Parts split(const KernelConfig& kc, const LutNet& net) {
     const bool sat = kc.mode == Mode::SAT;
